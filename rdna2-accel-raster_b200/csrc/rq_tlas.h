@@ -23,7 +23,7 @@ struct rq_tlas {
     rq_ctx* ctx = nullptr;
     int device = 0;
     uint32_t num_instances = 0;
-    TlasInst* d_inst = nullptr;   // num_instances records
+    TlasInst* d_inst = nullptr;   // num_instances records; the block also holds the next two
     float* d_fwd = nullptr;       // 12 floats per instance: object -> world
     float* d_tri9 = nullptr;      // the instances' world boxes as degenerate triangles
     rq_bvh* top = nullptr;        // BVH over the instance boxes, one instance per leaf
