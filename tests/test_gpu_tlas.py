@@ -91,3 +91,29 @@ def test_tlas_rejects_bad_instances(ctx):
     with pytest.raises(rq.RqError):
         rq.Tlas(ctx, [])
     b.destroy()
+
+
+@pytest.mark.parametrize("flags", [0, rq.RQ_TRACE_ANY])
+def test_tlas_ray_counts(ctx, flags):
+    """Shares of a launch at their edges: fewer rays than a block has lanes, one more, one wave's share per block and
+    a ray more, several waves.  A ray's result does not depend on the launch it is in."""
+    blas, _, insts = scene(ctx)
+    t = rq.Tlas(ctx, [(x, i, m, blas[b]) for x, i, m, b in insts])
+    rays = torch.from_numpy(rays_in_box(400001, 6).view(np.float32).reshape(-1, 8)).cuda()
+    want = t.trace(rays, flags=flags)
+    for n in (1, 31, 127, 128, 129, 18944, 151553):
+        assert torch.equal(t.trace(rays[:n].contiguous(), flags=flags), want[:n]), n
+    ctx.sync_check()
+    t.destroy()
+
+
+def test_tlas_instance_forms(ctx):
+    """Arrays of either float type, nested lists and numbers that are not plain ints describe the same scene."""
+    blas, _, insts = scene(ctx)
+    rays = torch.from_numpy(rays_in_box(20000, 8).view(np.float32).reshape(-1, 8)).cuda()
+    forms = [lambda x: x, lambda x: x.astype(np.float64), lambda x: x.reshape(12), lambda x: x.tolist()]
+    got = [rq.Tlas(ctx, [(f(x), i, m, blas[b]) for x, i, m, b in insts]).trace(rays) for f in forms]
+    got.append(rq.Tlas(ctx, [(forms[k % 4](x), i, m, blas[b]) for k, (x, i, m, b) in enumerate(insts)]).trace(rays))
+    for g in got[1:]:
+        assert torch.equal(g, got[0])
+    assert int(got[0][:, 0].sum()) > 0
