@@ -1583,15 +1583,14 @@ inline uint32_t grid_for(uint32_t n, int sms) {
 size_t rq_build_scratch_carve(void* base, uint32_t n, BuildScratch& s, bool sah) {
     Carve c{reinterpret_cast<uintptr_t>(base), 0};
     const size_t N = n ? n : 1;
-    const uint32_t tiles = rq_sort_tiles(uint32_t(N)), stiles = rq_scan_tiles(uint32_t(N));
+    const uint32_t stiles = rq_scan_tiles(uint32_t(N));
     s.cent = c.take<float4>(N);
     s.bounds = c.take<uint32_t>(8);
     s.keys[0] = c.take<uint32_t>(N);
     s.vals[0] = c.take<uint32_t>(N);
     s.keys[1] = c.take<uint32_t>(N);
     s.vals[1] = c.take<uint32_t>(N);
-    s.hist = c.take<uint32_t>(4 * 256);
-    s.sort_status = c.take<uint32_t>(4ull * tiles * 256);
+    s.sort_words = c.take<uint32_t>(rq_sort_words(uint32_t(N), 1));
     s.tile_ctr = c.take<uint32_t>(16);
     s.kl = c.take<int32_t>(N);
     s.kr = c.take<int32_t>(N);
@@ -1771,7 +1770,7 @@ int rq_launch_build(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t stride_
     k_centroids<<<grid_for(n, sms), kT, 0, st>>>(pos, sf, idx, n, s.cent, s.bounds);
     k_morton<<<grid_for(n, sms), kT, 0, st>>>(s.cent, n, s.bounds, s.keys[0], s.vals[0]);
     int rb = 0;
-    rc = rq_launch_sort(ctx, s, n, 30, st, &rb);
+    rc = rq_launch_sort(ctx, SortIO{{s.keys[0], s.keys[1]}, {s.vals[0], s.vals[1]}, 0, s.sort_words}, n, 30, 1, st, &rb);
     if (rc) return rc;
     const uint32_t* skeys = s.keys[rb];
     const uint32_t* sids = s.vals[rb];

@@ -319,7 +319,8 @@ int rq_launch_build_median(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t 
         k_med_keys<<<g, kT, 0, st>>>(s.cent, n, a, s.keys[0], s.vals[0]);
         cudaMemsetAsync(s.tile_ctr, 0, 16 * sizeof(uint32_t), st);
         int rb = 0;
-        rc = rq_launch_sort(ctx, s, n, 32, st, &rb);
+        rc = rq_launch_sort(ctx, SortIO{{s.keys[0], s.keys[1]}, {s.vals[0], s.vals[1]}, 0, s.sort_words}, n, 32, 1, st,
+                            &rb);
         if (rc) return rc;
         e = cudaMemcpyAsync(m.order[a], s.vals[rb], sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st);
     }

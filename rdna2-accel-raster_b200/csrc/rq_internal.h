@@ -90,9 +90,8 @@ struct BuildScratch {
     uint32_t* bounds;      // 6 ordered-uint: min xyz, max xyz
     uint32_t* keys[2];     // N each
     uint32_t* vals[2];     // N each
-    uint32_t* hist;        // 4 x 256
-    uint32_t* sort_status; // 4 passes x tiles x 256
-    uint32_t* tile_ctr;    // 8 counters
+    uint32_t* sort_words;  // rq_sort_words(N, 1)
+    uint32_t* tile_ctr;    // 16 counters
     int32_t* kl;           // N-1 Karras left child (bit 31: leaf)
     int32_t* kr;           // N-1 right child
     uint32_t* klo;         // N-1 range start
@@ -147,10 +146,20 @@ int rq_launch_refit(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t stride_
                     cudaStream_t s);
 
 // ---------------------------------------------------------------- k_sort
-uint32_t rq_sort_tiles(uint32_t n);
-// Stable LSD radix sort of (keys, vals) on `bits` low key bits; result ends
-// in buffer index returned (0 or 1).
-int rq_launch_sort(rq_ctx* ctx, BuildScratch& s, uint32_t n, uint32_t bits, cudaStream_t st, int* result_buf);
+// Buffers of a batch of sorts of n keys each: sort y's keys and values start
+// y * stride words into the two buffers of each (stride a multiple of 4, the
+// buffers 16-byte aligned).
+struct SortIO {
+    uint32_t* keys[2];
+    uint32_t* vals[2];
+    size_t stride;
+    uint32_t* words;  // rq_sort_words(n, batch) words of scratch
+};
+size_t rq_sort_words(uint32_t n, uint32_t batch);
+// Stable LSD radix sorts of (keys, vals) on `bits` low key bits; the results
+// end in buffer index returned (0 or 1).
+int rq_launch_sort(rq_ctx* ctx, const SortIO& io, uint32_t n, uint32_t bits, uint32_t batch, cudaStream_t st,
+                   int* result_buf);
 uint32_t rq_scan_tiles(uint32_t n);
 // Exclusive scan of in[0..n) (of in[order[i]] when order is given).
 void rq_launch_scan(rq_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* status,

@@ -64,6 +64,12 @@ def test_duplicate_codes_parity(ctx):
     assert_same_as_oracle(ctx, v, None)
 
 
+@pytest.mark.parametrize("n", [1023, 1024, 1025, 606207, 606208, 606209, 610304, 610305])
+def test_sort_forms_parity(ctx, n):
+    """The sort's tile edges in both its forms and on both sides of the length where one takes over from the other."""
+    assert_same_as_oracle(ctx, soup(n, 200 + n % 97), None)
+
+
 def test_large_soup_parity(ctx):
     assert_same_as_oracle(ctx, soup(300000, 11), None)
 
