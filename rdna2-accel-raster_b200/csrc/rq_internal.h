@@ -139,7 +139,7 @@ size_t rq_build_scratch_carve(void* base, uint32_t n, BuildScratch& s, bool sah 
 // such subtree rebuilt by binned SAH (RQ_BUILD_SAH); 0: the plain LBVH.
 int rq_launch_build(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t stride_bytes, const uint32_t* idx,
                     uint32_t n, uint32_t max_leaf, bool collapse, cudaStream_t s, uint32_t sah_max = 0);
-// The reference's median-split topology (k_median.cu); synchronises once per tree level.
+// The reference's median-split topology (k_median.cu).
 int rq_launch_build_median(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t stride_bytes, const uint32_t* idx,
                            uint32_t n, uint32_t max_leaf, bool collapse, cudaStream_t s);
 int rq_launch_refit(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t stride_bytes, const uint32_t* idx,
@@ -161,9 +161,9 @@ size_t rq_sort_words(uint32_t n, uint32_t batch);
 int rq_launch_sort(rq_ctx* ctx, const SortIO& io, uint32_t n, uint32_t bits, uint32_t batch, cudaStream_t st,
                    int* result_buf);
 uint32_t rq_scan_tiles(uint32_t n);
-// Exclusive scan of in[0..n) (of in[order[i]] when order is given).
+// Exclusive scan of in[0..n).
 void rq_launch_scan(rq_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* status,
-                    uint32_t* tile_ctr, cudaStream_t st, const uint32_t* order = nullptr);
+                    uint32_t* tile_ctr, cudaStream_t st);
 
 // ---------------------------------------------------------------- k_collapse
 int rq_launch_collapse(rq_ctx* ctx, rq_bvh* bvh, BuildScratch& s, cudaStream_t st);

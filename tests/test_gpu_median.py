@@ -126,3 +126,53 @@ def test_median_build_replayed_from_a_graph(ctx):
     del g
     bm.destroy()
     bl.destroy()
+
+
+def median_statement(pos, max_leaf):
+    """The median build's rules over a soup, one range at a time: binary nodes in pre-order and the permutation."""
+    v = pos.reshape(-1, 3, 3).astype(np.float32)
+    cent = ((v[:, 0] + v[:, 1]) + v[:, 2]) / np.float32(3.0)
+    nodes, perm = [], np.empty(len(v), np.uint32)
+    work = [(0, [np.argsort(cent[:, a], kind="stable") for a in range(3)], -1)]
+    while work:
+        s, orders, right_of = work.pop()
+        c, me = len(orders[0]), len(nodes)
+        if right_of >= 0:
+            nodes[right_of][3] = me
+        ids = orders[0]
+        nodes.append([v[ids].min((0, 1)), v[ids].max((0, 1)), ~s, c])
+        ext = np.array([cent[o[-1], a] - cent[o[0], a] for a, o in enumerate(orders)], np.float32)
+        if c <= max_leaf or ext.max() < np.float32(1e-6):
+            perm[s:s + c] = ids
+            continue
+        nodes[me][2] = me + 1
+        left = np.zeros(len(v), bool)
+        left[orders[int(ext.argmax())][:c // 2]] = True
+        work.append((s + c // 2, [o[~left[o]] for o in orders], me))
+        work.append((s, [o[left[o]] for o in orders], -1))
+    out = np.zeros(len(nodes), rq.BVH2_NODE)
+    for k, (lo, hi, lc, rc) in enumerate(nodes):
+        out[k] = (lo, lc, hi, rc)
+    return out, perm
+
+
+def tie_soup(n, same):
+    """A soup with repeated centroid values on every axis, `same` of its triangles identical."""
+    rng = np.random.default_rng(n)
+    c = np.round(rng.uniform(-4, 4, (n, 1, 3)) * 16) / 16
+    p = (c + np.array([[0, 0, 0], [0.25, 0, 0], [0, 0.25, 0.125]])).astype(np.float32)
+    p[rng.permutation(n)[:same]] = p[0]
+    return p.reshape(-1, 3)
+
+
+@pytest.mark.parametrize("n,same,max_leaf", [(1, 0, 4), (5, 0, 4), (17, 5, 1), (1023, 0, 4), (1024, 0, 1), (1025, 0, 1),
+                                             (1025, 1025, 4), (2047, 0, 16), (2049, 600, 4), (4099, 0, 2),
+                                             (9000, 7000, 4), (9001, 9001, 4), (20000, 0, 4)])
+def test_median_matches_its_statement(ctx, n, same, max_leaf):
+    """Ranges at the edges of a block's and a tile's size, ties on every axis, leaves by extent above and below them."""
+    pos = tie_soup(n, same)
+    n2g, trg, _, perm = gpu_median(ctx, pos, max_leaf)
+    n2, want = median_statement(pos, max_leaf)
+    assert np.array_equal(perm, want)
+    assert n2g.tobytes() == n2.tobytes()
+    assert np.array_equal(trg["v1"][:, :3], pos.reshape(-1, 3, 3)[want, 1])
