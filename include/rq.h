@@ -68,15 +68,13 @@ typedef struct rq_trace_tuning {
     uint32_t chunk;    /* ray ids a warp takes per refill: 32 or 64 (default 32) */
     uint32_t reg_cap;  /* registers per thread the launch bounds allow: 0 (no bound), 64, 72 (threads
                           64 or 128 only) or 80 (default) */
-    uint32_t top_levels; /* 0, or 4: each block stages the tree's top 4 levels (<= 85 nodes) in shared memory */
-    uint32_t speculative; /* 1: lanes holding a leaf keep taking inner nodes while the warp searches
-                             (the frame only reports hit or miss, so the order does not show) */
+    uint32_t top_levels; /* 0 or 4: accepted, without effect (staging the top levels in shared memory
+                            was never faster) */
+    uint32_t speculative; /* 0 or 1: accepted, without effect (the plain schedule is as fast) */
     uint32_t refill_min;  /* a warp hands new rays to its idle lanes only once at least this many of
                              its 32 lanes are idle (or all are): 1..32; 0 means 1 */
-    uint32_t leaf_batch;  /* 0: rays finish and lanes refill between rounds only.  1..32: a lane whose
-                             ray runs out of nodes reports at once and idle lanes refill inside the
-                             node loop, which hands over to the leaf tests once this many lanes hold a
-                             leaf (speculative shapes only) */
+    uint32_t leaf_batch;  /* 0..32 (speculative shapes only): accepted, without effect (rays finish and
+                             lanes refill between rounds) */
 } rq_trace_tuning;
 int rq_ctx_trace_tuning_get(const rq_ctx* ctx, rq_trace_tuning* out);
 /* RQ_ERR_INVALID_ARG for a shape that has no kernel. */
@@ -86,10 +84,9 @@ int rq_ctx_trace_tuning_set(rq_ctx* ctx, const rq_trace_tuning* t);
  * do not depend on it. */
 typedef struct rq_camera_tuning {
     uint32_t engine;      /* 0: one ray per thread, 8x4-pixel tiles per warp (default); 1: the
-                             persistent refilling engine with in-loop refill (128-thread blocks,
-                             64 registers) */
+                             persistent refilling engine (128-thread blocks, 64 registers) */
     uint32_t refill_min;  /* engine: idle lanes before a refill, 1..32 (0 means 1) */
-    uint32_t leaf_batch;  /* engine: parked leaves that end the node loop, 1..32 (0 means 32) */
+    uint32_t leaf_batch;  /* 1..32 (0 means 32): accepted, without effect */
 } rq_camera_tuning;
 int rq_ctx_camera_tuning_get(const rq_ctx* ctx, rq_camera_tuning* out);
 int rq_ctx_camera_tuning_set(rq_ctx* ctx, const rq_camera_tuning* t);
@@ -339,7 +336,7 @@ typedef struct rq_batch_tuning {
     uint32_t trace_reg_cap;       /* registers per thread the launch bounds allow: 0 (none), 64, 72
                                      (threads 64 or 128 only) or 80 */
     uint32_t trace_blocks_per_sm; /* 0: as many as fit */
-    uint32_t stack_entries;       /* stack entries per lane; 0 or anything below
+    uint32_t stack_entries;       /* stack room per lane as 3 entries per level; 0 or anything below
                                      3 * (depth + 2) + 1 means that bound */
     uint32_t max_build_blocks;    /* read only: build scratch slices the batch holds */
     float build_ms;               /* rq_batch_autotune: measured time of this shape */

@@ -27,6 +27,8 @@
 //               cosine-hemisphere any-hit rays; k_ao_depth_finish turns the
 //               per-pixel result bits into the AO fraction.
 // No ray buffer touches HBM.
+#include <type_traits>
+
 #include "rq_device.cuh"
 #include "rq_internal.h"
 #include "trace_core.cuh"
@@ -35,6 +37,10 @@
 namespace {
 
 constexpr int kT = 128;
+// Idle lanes of a warp that call for new rays in the AO-from-depth and
+// reflection passes (1080p, a million triangles, 2 AO samples; us for AO /
+// reflections: 1: 1,873 / 850, 8: 1,841 / 848, 16: 1,770 / 826, 24: 1,950 / 889).
+constexpr int kScatterRefill = 16;
 constexpr uint32_t kTileW = 8, kTileH = 4;
 
 struct CamArgs {
@@ -188,13 +194,13 @@ struct ShadeSrc {
 };
 
 // One camera ray per thread, 16x8 pixels per block: primary rays are
-// coherent, so lanes stay together without refilling.  `stack` rows of
-// shared memory per thread (the tree's bound, at most STACK).
-template <bool MT, int STACK>
+// coherent, so lanes stay together without refilling.  `rows` stack entries
+// per thread.
+template <bool MT, bool WIDE>
 __global__ void __launch_bounds__(kT) k_gbuffer_seq(const rq_bvh4_node* __restrict__ nodes,
                                                     const rq_triangle* __restrict__ tris,
-                                                    const __grid_constant__ GbufSrc src, uint32_t* err, int stack) {
-    extern __shared__ int32_t s_stack[];
+                                                    const __grid_constant__ GbufSrc src, uint32_t* err, int rows) {
+    extern __shared__ __align__(16) char s_stack[];
     // each warp takes an 8x4 pixel tile of the block's 16x8 (the most compact
     // footprint, so its rays stay close)
     const uint32_t w = threadIdx.x >> 5, l = threadIdx.x & 31u;
@@ -206,48 +212,43 @@ __global__ void __launch_bounds__(kT) k_gbuffer_seq(const rq_bvh4_node* __restri
     GbufSrc::Meta m;
     src.make(id, r, m);
     rq::TraceResult res;
-    rq::trace_ray<false, MT, false, STACK, kT>(nodes, tris, s_stack + threadIdx.x, r.o, r.d, r.tmin, r.tmax, res,
-                                               err, stack);
+    using Entry = typename rq::OpenNode<false, WIDE>::Entry;
+    rq::trace_ray<MT, kT, WIDE>(nodes, tris, reinterpret_cast<Entry*>(s_stack) + threadIdx.x, rows, r.o, r.d, r.tmin,
+                                r.tmax, res, err);
     rq::Hit h;
     h.hit = res.idx != rq::kNoHit;
     h.t = res.t;
     h.idx = res.idx;
     h.u = res.u;
     h.v = res.v;
-    h.boxes = res.boxes;
-    h.tris = res.tris;
     src.finish(id, m, r, h);
 }
 
-// Camera rays on the refilling engine with in-loop refill (closest hit):
-// rays that need few nodes hand their lane to the next pixel instead of
-// waiting for the warp's longest ray.
-template <bool MT, int TT, int REGS>
+// Camera rays on the refilling engine (closest hit): rays that need few nodes
+// hand their lane to the next pixel instead of waiting for the warp's longest
+// ray.
+template <bool MT, int TT, int REGS, bool WIDE>
 __global__ void __launch_bounds__(TT, 65536 / (TT * REGS))
     k_gbuffer_eng(const rq_bvh4_node* __restrict__ nodes, const rq_triangle* __restrict__ tris,
-                  const __grid_constant__ GbufSrc src0, uint32_t* ctr, uint32_t* err, int stack, int refill_min,
-                  int leaf_batch) {
-    extern __shared__ __align__(16) int32_t s_stack[];
+                  const __grid_constant__ GbufSrc src0, uint32_t* ctr, uint32_t* err, int rows, int refill_min) {
+    extern __shared__ __align__(16) char s_stack[];
     GbufSrc src = src0;
-    rq::trace_persistent<0, MT, false, 128, TT, GbufSrc, 32, 0, false, true>(
-        nodes, tris, src, ctr, s_stack + threadIdx.x, err, stack, nullptr, refill_min, leaf_batch);
+    using Entry = typename rq::OpenNode<false, WIDE>::Entry;
+    rq::trace_persistent<0, MT, false, TT, GbufSrc, 32, WIDE>(
+        nodes, tris, src, ctr, reinterpret_cast<Entry*>(s_stack) + threadIdx.x, rows, err, refill_min);
 }
 
 // TT threads per block, CHUNK ray ids per refill, REGS: launch bounds that
-// hold registers to REGS (0: none) — the tuned shapes; `stack` rows per lane;
-// idle lanes are refilled once `refill_min` of a warp's lanes are idle.
-// INLOOP: rays finish and lanes refill inside the node loop (leaf_batch
-// parked leaves end it).
-template <bool MT, bool STATS, int TT, int CHUNK, int REGS, int TOP, bool SPEC, bool INLOOP = false>
+// hold registers to REGS (0: none) — the tuned shapes; `rows` stack entries
+// per lane; idle lanes are refilled once `refill_min` of a warp's lanes are
+// idle.
+template <bool MT, bool STATS, int TT, int CHUNK, int REGS>
 __global__ void __launch_bounds__(TT, 65536 / (TT * (REGS ? REGS : 65536 / TT)))
     k_shadow_ao(const rq_bvh4_node* __restrict__ nodes, const rq_triangle* __restrict__ tris,
                 const rq_gbuffer_px* __restrict__ gbuf, const __grid_constant__ ShadeArgs sa,
-                unsigned long long* words, unsigned long long* counters, uint32_t* ctr, uint32_t* err, int stack,
-                int refill_min, int leaf_batch) {
-    extern __shared__ __align__(16) int32_t s_stack[];
-    // shared memory: the stack (stack rows x TT), then the staged top levels
-    float4* s_top = reinterpret_cast<float4*>(s_stack + stack * TT);
-    if (TOP > 0) rq::stage_top<TOP>(nodes, s_top);
+                unsigned long long* words, unsigned long long* counters, uint32_t* ctr, uint32_t* err, int rows,
+                int refill_min) {
+    extern __shared__ __align__(16) uint32_t s_entries[];
     ShadeSrc<STATS> src;
     src.kinds = sa.nl + sa.spp;
     src.tiles_x = (sa.w + kTileW - 1) / kTileW;
@@ -255,8 +256,8 @@ __global__ void __launch_bounds__(TT, 65536 / (TT * (REGS ? REGS : 65536 / TT)))
     src.s = &sa;
     src.gbuf = gbuf;
     src.words = words;
-    rq::trace_persistent<1, MT, STATS, 128, TT, ShadeSrc<STATS>, CHUNK, TOP, SPEC, INLOOP>(
-        nodes, tris, src, ctr, s_stack + threadIdx.x, err, stack, s_top, refill_min, leaf_batch);
+    rq::trace_persistent<1, MT, STATS, TT, ShadeSrc<STATS>, CHUNK>(nodes, tris, src, ctr, s_entries + threadIdx.x, rows,
+                                                                   err, refill_min);
     if (counters) {
         const uint32_t r = __reduce_add_sync(rq::kFull, src.rays);
         if ((threadIdx.x & 31u) == 0 && r) atomicAdd(counters, (unsigned long long)r);
@@ -324,13 +325,15 @@ struct ReflSrc {
     }
 };
 
-template <bool MT, int TT, int REGS>
+template <bool MT, int TT, int REGS, bool WIDE>
 __global__ void __launch_bounds__(TT, 65536 / (TT * REGS))
     k_reflect(const rq_bvh4_node* __restrict__ nodes, const rq_triangle* __restrict__ tris,
-              const __grid_constant__ ReflSrc src0, uint32_t* ctr, uint32_t* err, int stack) {
-    extern __shared__ __align__(16) int32_t s_stack[];
+              const __grid_constant__ ReflSrc src0, uint32_t* ctr, uint32_t* err, int rows) {
+    extern __shared__ __align__(16) char s_stack[];
     ReflSrc src = src0;
-    rq::trace_persistent<0, MT, false, 128, TT, ReflSrc>(nodes, tris, src, ctr, s_stack + threadIdx.x, err, stack);
+    using Entry = typename rq::OpenNode<false, WIDE>::Entry;
+    rq::trace_persistent<0, MT, false, TT, ReflSrc, 32, WIDE>(
+        nodes, tris, src, ctr, reinterpret_cast<Entry*>(s_stack) + threadIdx.x, rows, err, kScatterRefill);
 }
 
 // ------------------------------------------------------------ AO from depth
@@ -407,15 +410,15 @@ template <bool MT, int TT, int REGS>
 __global__ void __launch_bounds__(TT, 65536 / (TT * REGS))
     k_ao_depth(const rq_bvh4_node* __restrict__ nodes, const rq_triangle* __restrict__ tris,
                const float* __restrict__ depth, const __grid_constant__ AoDepthArgs a, uint32_t* words,
-               unsigned long long* counters, uint32_t* ctr, uint32_t* err, int stack) {
-    extern __shared__ __align__(16) int32_t s_stack[];
+               unsigned long long* counters, uint32_t* ctr, uint32_t* err, int rows) {
+    extern __shared__ __align__(16) uint32_t s_entries[];
     AoDepthSrc src;
     src.tiles_x = (a.w + kTileW - 1) / kTileW;
     src.total = src.tiles_x * ((a.h + kTileH - 1) / kTileH) * a.spp * 32u;
     src.a = &a;
     src.depth = depth;
     src.words = words;
-    rq::trace_persistent<1, MT, false, 128, TT, AoDepthSrc>(nodes, tris, src, ctr, s_stack + threadIdx.x, err, stack);
+    rq::trace_persistent<1, MT, false, TT, AoDepthSrc>(nodes, tris, src, ctr, s_entries + threadIdx.x, rows, err, kScatterRefill);
     if (counters) {
         const uint32_t r = __reduce_add_sync(rq::kFull, src.rays);
         if ((threadIdx.x & 31u) == 0 && r) atomicAdd(counters, (unsigned long long)r);
@@ -440,61 +443,49 @@ cudaError_t persistent_grid(rq_ctx* ctx, const void* k, int threads, size_t smem
     return e;
 }
 
-template <class F>
-cudaError_t with_stack(uint32_t bound, F&& f) {
-    if (bound <= 32) return f(std::integral_constant<int, 32>{});
-    if (bound <= 64) return f(std::integral_constant<int, 64>{});
-    return f(std::integral_constant<int, 128>{});
-}
+// Stack rows per lane: an entry per open node of a path, for the depth the
+// host knows and what an in-place rebuild may add before it is read back.
+int stack_rows(const rq_bvh* bvh) { return int(bvh->h_counts[2]) + 4; }
 
-// Shadow/AO kernel of a launch shape (only the default shape has the
-// counting and reference-arithmetic variants).
+// Shadow/AO kernel of a launch shape (only the default shape has the counting
+// and reference-arithmetic variants).
 template <bool MT, bool STATS>
-const void* shade_kernel(const rq_trace_tuning& t) {
-#define RQ_SHAPE(T, C, R, L, S)                                                                             \
-    if (t.threads == T && t.chunk == C && t.reg_cap == R && t.top_levels == L && (t.speculative != 0) == S) \
-        return reinterpret_cast<const void*>(k_shadow_ao<MT, STATS, T, C, R, L, S>);
-#define RQ_SHAPES(T, C)                                                                              \
-    RQ_SHAPE(T, C, 0, 0, false) RQ_SHAPE(T, C, 64, 0, false) RQ_SHAPE(T, C, 80, 0, false) RQ_SHAPE(T, C, 80, 4, false) \
-    RQ_SHAPE(T, C, 80, 0, true)
+const void* shade_kernel(uint32_t threads, uint32_t chunk, uint32_t reg_cap) {
+#define RQ_SHAPE(T, C, R) \
+    if (threads == T && chunk == C && reg_cap == R) return reinterpret_cast<const void*>(k_shadow_ao<MT, STATS, T, C, R>);
+#define RQ_SHAPES(T, C) RQ_SHAPE(T, C, 0) RQ_SHAPE(T, C, 64) RQ_SHAPE(T, C, 72) RQ_SHAPE(T, C, 80)
     if constexpr (!MT && !STATS) {
         RQ_SHAPES(64, 32) RQ_SHAPES(64, 64) RQ_SHAPES(128, 64) RQ_SHAPES(256, 32) RQ_SHAPES(256, 64)
-        RQ_SHAPE(128, 32, 64, 0, false) RQ_SHAPE(128, 32, 80, 0, false) RQ_SHAPE(128, 32, 80, 4, false)
-        RQ_SHAPE(128, 32, 80, 0, true)
-        // a budget of 72 registers: 7 blocks of 128 (14 of 64) threads per SM
-        RQ_SHAPE(64, 32, 72, 0, false) RQ_SHAPE(64, 32, 72, 0, true) RQ_SHAPE(64, 64, 72, 0, false)
-        RQ_SHAPE(64, 64, 72, 0, true) RQ_SHAPE(128, 32, 72, 0, false) RQ_SHAPE(128, 32, 72, 0, true)
-        RQ_SHAPE(128, 64, 72, 0, false) RQ_SHAPE(128, 64, 72, 0, true)
-        RQ_SHAPE(64, 64, 64, 0, true) RQ_SHAPE(128, 64, 64, 0, true) RQ_SHAPE(256, 64, 64, 0, true)
+        RQ_SHAPE(128, 32, 64) RQ_SHAPE(128, 32, 72) RQ_SHAPE(128, 32, 80)
     }
-    RQ_SHAPE(128, 32, 0, 0, false)
+    RQ_SHAPE(128, 32, 0)
 #undef RQ_SHAPES
 #undef RQ_SHAPE
     return nullptr;
 }
 
-// Shapes with in-loop refill (speculative, leaf_batch > 0).
-template <bool MT, bool STATS>
-const void* shade_kernel_inloop(const rq_trace_tuning& t) {
-#define RQ_SHAPE(T, C, R)                                                                      \
-    if (t.threads == T && t.chunk == C && t.reg_cap == R && t.top_levels == 0 && t.speculative) \
-        return reinterpret_cast<const void*>(k_shadow_ao<MT, STATS, T, C, R, 0, true, true>);
-    if constexpr (!MT && !STATS) {
-        RQ_SHAPE(64, 32, 64) RQ_SHAPE(64, 64, 64) RQ_SHAPE(128, 32, 64) RQ_SHAPE(128, 64, 64) RQ_SHAPE(256, 32, 64)
-        RQ_SHAPE(256, 64, 64) RQ_SHAPE(128, 64, 72) RQ_SHAPE(256, 64, 72)
-    }
-#undef RQ_SHAPE
-    return nullptr;
-}
-
-template <bool MT, bool STATS>
-const void* shade_kernel_any(const rq_trace_tuning& t) {
-    return t.leaf_batch ? shade_kernel_inloop<MT, STATS>(t) : shade_kernel<MT, STATS>(t);
-}
-
 }  // namespace
 
-bool rq_shade_shape_ok(const rq_trace_tuning& t) { return shade_kernel_any<false, false>(t) != nullptr; }
+// The shapes a context accepts.  Staged top levels, speculative traversal and
+// in-loop refill (leaf_batch) no longer have kernels of their own: each
+// measured slower than or equal to the plain schedule, and with one stack
+// entry per open node there is nothing left for them to save.  Shapes that
+// name them run the plain schedule, with the same results.
+bool rq_shade_shape_ok(const rq_trace_tuning& t) {
+    const bool threads = t.threads == 64 || t.threads == 128 || t.threads == 256;
+    if (!threads || (t.chunk != 32 && t.chunk != 64)) return false;
+    const bool spec = t.speculative != 0;
+    if (t.leaf_batch)
+        return !t.top_levels && spec &&
+               (t.reg_cap == 64 || (t.reg_cap == 72 && t.chunk == 64 && t.threads != 64));
+    switch (t.reg_cap) {
+        case 0: return !t.top_levels && !spec;
+        case 64: return !t.top_levels && (!spec || t.chunk == 64);
+        case 72: return !t.top_levels && t.threads != 256;
+        case 80: return t.top_levels == 0 || (t.top_levels == 4 && !spec);
+    }
+    return false;
+}
 
 int rq_launch_gbuffer(rq_ctx* ctx, const rq_bvh* bvh, const rq_camera& cam, rq_gbuffer_px* gbuf, cudaStream_t st) {
     GbufSrc src;
@@ -514,14 +505,16 @@ int rq_launch_gbuffer(rq_ctx* ctx, const rq_bvh* bvh, const rq_camera& cam, rq_g
     src.tris = bvh->tris;
     src.perm = bvh->perm;
     src.gbuf = gbuf;
-    const uint32_t bound = 3u * (bvh->h_counts[2] + 2u) + 1u;
-    const bool mt = cam.flags & RQ_TRI_MT;
+    const bool mt = cam.flags & RQ_TRI_MT, wide = bvh->cap_nodes4 > RQ_NARROW_NODES;
+    int rows = stack_rows(bvh);
+    const size_t entry = wide ? 8 : 4;
     if (ctx->camera.engine) {
         constexpr int kET = 128, kER = 64;
-        const int stack = int((bound + 3u) & ~3u);
-        const void* k = mt ? reinterpret_cast<const void*>(k_gbuffer_eng<true, kET, kER>)
-                           : reinterpret_cast<const void*>(k_gbuffer_eng<false, kET, kER>);
-        const size_t smem = size_t(stack) * kET * sizeof(int32_t);
+        const void* k = wide ? (mt ? reinterpret_cast<const void*>(k_gbuffer_eng<true, kET, kER, true>)
+                                   : reinterpret_cast<const void*>(k_gbuffer_eng<false, kET, kER, true>))
+                             : (mt ? reinterpret_cast<const void*>(k_gbuffer_eng<true, kET, kER, false>)
+                                   : reinterpret_cast<const void*>(k_gbuffer_eng<false, kET, kER, false>));
+        const size_t smem = size_t(rows) * kET * entry;
         uint32_t blocks = 0;
         cudaError_t e = cudaMemsetAsync(ctx->d_ctr, 0, sizeof(uint32_t), st);
         if (e == cudaSuccess) e = persistent_grid(ctx, k, kET, smem, blocks);
@@ -530,25 +523,17 @@ int rq_launch_gbuffer(rq_ctx* ctx, const rq_bvh* bvh, const rq_camera& cam, rq_g
             const rq_triangle* tris = bvh->tris;
             uint32_t* ctr = ctx->d_ctr;
             uint32_t* err = ctx->d_err;
-            int stk = stack, rm = int(ctx->camera.refill_min), lb = int(ctx->camera.leaf_batch);
-            void* args[] = {&nodes, &tris, &src, &ctr, &err, &stk, &rm, &lb};
+            int rm = int(ctx->camera.refill_min);
+            void* args[] = {&nodes, &tris, &src, &ctr, &err, &rows, &rm};
             e = cudaLaunchKernel(k, dim3(blocks), dim3(kET), args, smem, st);
         }
         return rq_cuda_status(ctx, e, "gbuffer launch");
     }
     dim3 grid((cam.width + 15) / 16, (cam.height + 7) / 8);
-    cudaError_t e = with_stack(bound, [&](auto S) {
-        constexpr int STACK = decltype(S)::value;
-        auto k = mt ? k_gbuffer_seq<true, STACK> : k_gbuffer_seq<false, STACK>;
-        const size_t smem = size_t(bound) * kT * 4;  // bound <= STACK
-        if (smem > 48 * 1024) {
-            cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            if (r != cudaSuccess) return r;
-        }
-        k<<<grid, kT, smem, st>>>(bvh->nodes4, bvh->tris, src, ctx->d_err, int(bound));
-        return cudaGetLastError();
-    });
-    return rq_cuda_status(ctx, e, "gbuffer launch");
+    auto k = wide ? (mt ? k_gbuffer_seq<true, true> : k_gbuffer_seq<false, true>)
+                  : (mt ? k_gbuffer_seq<true, false> : k_gbuffer_seq<false, false>);
+    k<<<grid, kT, size_t(rows) * kT * entry, st>>>(bvh->nodes4, bvh->tris, src, ctx->d_err, rows);
+    return rq_cuda_status(ctx, cudaGetLastError(), "gbuffer launch");
 }
 
 int rq_launch_shadow_ao(rq_ctx* ctx, const rq_bvh* bvh, const rq_gbuffer_px* gbuf, const rq_shade_params& p,
@@ -574,7 +559,6 @@ int rq_launch_shadow_ao(rq_ctx* ctx, const rq_bvh* bvh, const rq_gbuffer_px* gbu
     int rc = rq_ensure_scratch(ctx, sizeof(unsigned long long) * size_t(npix) + 256, st);
     if (rc) return rc;
     unsigned long long* words = static_cast<unsigned long long*>(ctx->scratch);
-    const uint32_t bound = 3u * (bvh->h_counts[2] + 2u) + 1u;
     const bool mt = p.flags & RQ_TRI_MT;
     const bool stats = (p.flags & RQ_SHADE_COUNT_TESTS) && counter;
     uint32_t* ctr = ctx->d_ctr;
@@ -583,14 +567,13 @@ int rq_launch_shadow_ao(rq_ctx* ctx, const rq_bvh* bvh, const rq_gbuffer_px* gbu
     if (e == cudaSuccess && p.num_lights + p.ao_spp > 0) {
         // the counting and reference-arithmetic variants run in the default shape
         const rq_trace_tuning shape = (mt || stats) ? rq_trace_tuning{128, 32, 0, 0, 0, 1, 0} : ctx->shade_shape;
-        const size_t top_bytes = shape.top_levels == 4 ? rq::TopLevels<4>::kBytes : 0;
-        const void* k = mt ? (stats ? shade_kernel_any<true, true>(shape) : shade_kernel_any<true, false>(shape))
-                           : (stats ? shade_kernel_any<false, true>(shape) : shade_kernel_any<false, false>(shape));
+        auto kernel = [&](auto M, auto S) { return shade_kernel<M.value, S.value>(shape.threads, shape.chunk, shape.reg_cap); };
+        const std::true_type yes;
+        const std::false_type no;
+        const void* k = mt ? (stats ? kernel(yes, yes) : kernel(yes, no)) : (stats ? kernel(no, yes) : kernel(no, no));
         if (!k) return rq_set_error(ctx, RQ_ERR_INVALID_ARG, "no traversal kernel for this shape");
-        // stack rows: the bound for the tree's depth, rounded up to 4
-        const int stack = int((bound + 3u) & ~3u);
-        const size_t smem = size_t(stack) * shape.threads * sizeof(int32_t) + top_bytes;
-        if (smem > 48 * 1024) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        int rows = stack_rows(bvh);
+        const size_t smem = size_t(rows) * shape.threads * sizeof(uint32_t);
         int per_sm = 0;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, int(shape.threads), smem);
         if (e == cudaSuccess) {
@@ -599,9 +582,7 @@ int rq_launch_shadow_ao(rq_ctx* ctx, const rq_bvh* bvh, const rq_gbuffer_px* gbu
             const rq_triangle* tris = bvh->tris;
             uint32_t* err = ctx->d_err;
             int refill_min = int(shape.refill_min ? shape.refill_min : 1u);
-            int leaf_batch = int(shape.leaf_batch ? shape.leaf_batch : 32u);
-            void* args[] = {&nodes, &tris, &gbuf, &s, &words, &counter, &ctr, &err, const_cast<int*>(&stack),
-                            &refill_min, &leaf_batch};
+            void* args[] = {&nodes, &tris, &gbuf, &s, &words, &counter, &ctr, &err, &rows, &refill_min};
             e = cudaLaunchKernel(k, dim3(blocks), dim3(shape.threads), args, smem, st);
         }
     }
@@ -633,12 +614,13 @@ int rq_launch_reflect(rq_ctx* ctx, const rq_bvh* bvh, const rq_gbuffer_px* gbuf,
     src.gbuf = gbuf;
     src.perm = bvh->perm;
     src.hits = hits;
-    const uint32_t bound = 3u * (bvh->h_counts[2] + 2u) + 1u;
-    const int stack = int((bound + 3u) & ~3u);
-    const bool mt = p.flags & RQ_TRI_MT;
-    const void* k = mt ? reinterpret_cast<const void*>(k_reflect<true, kReflThreads, kReflRegs>)
-                       : reinterpret_cast<const void*>(k_reflect<false, kReflThreads, kReflRegs>);
-    const size_t smem = size_t(stack) * kReflThreads * sizeof(int32_t);
+    const bool mt = p.flags & RQ_TRI_MT, wide = bvh->cap_nodes4 > RQ_NARROW_NODES;
+    int rows = stack_rows(bvh);
+    const void* k = wide ? (mt ? reinterpret_cast<const void*>(k_reflect<true, kReflThreads, kReflRegs, true>)
+                               : reinterpret_cast<const void*>(k_reflect<false, kReflThreads, kReflRegs, true>))
+                         : (mt ? reinterpret_cast<const void*>(k_reflect<true, kReflThreads, kReflRegs, false>)
+                               : reinterpret_cast<const void*>(k_reflect<false, kReflThreads, kReflRegs, false>));
+    const size_t smem = size_t(rows) * kReflThreads * (wide ? 8 : 4);
     uint32_t blocks = 0;
     cudaError_t e = cudaMemsetAsync(ctx->d_ctr, 0, sizeof(uint32_t), st);
     if (e == cudaSuccess) e = persistent_grid(ctx, k, kReflThreads, smem, blocks);
@@ -647,8 +629,7 @@ int rq_launch_reflect(rq_ctx* ctx, const rq_bvh* bvh, const rq_gbuffer_px* gbuf,
         const rq_triangle* tris = bvh->tris;
         uint32_t* ctr = ctx->d_ctr;
         uint32_t* err = ctx->d_err;
-        int stk = stack;
-        void* args[] = {&nodes, &tris, &src, &ctr, &err, &stk};
+        void* args[] = {&nodes, &tris, &src, &ctr, &err, &rows};
         e = cudaLaunchKernel(k, dim3(blocks), dim3(kReflThreads), args, smem, st);
     }
     return rq_cuda_status(ctx, e, "reflection launch");
@@ -671,12 +652,11 @@ int rq_launch_ao_depth(rq_ctx* ctx, const rq_bvh* bvh, const float* depth, const
     int rc = rq_ensure_scratch(ctx, sizeof(uint32_t) * size_t(npix) + 256, st);
     if (rc) return rc;
     uint32_t* words = static_cast<uint32_t*>(ctx->scratch);
-    const uint32_t bound = 3u * (bvh->h_counts[2] + 2u) + 1u;
-    const int stack = int((bound + 3u) & ~3u);
+    int rows = stack_rows(bvh);
     const bool mt = p.flags & RQ_TRI_MT;
     const void* k = mt ? reinterpret_cast<const void*>(k_ao_depth<true, kAoThreads, kAoRegs>)
                        : reinterpret_cast<const void*>(k_ao_depth<false, kAoThreads, kAoRegs>);
-    const size_t smem = size_t(stack) * kAoThreads * sizeof(int32_t);
+    const size_t smem = size_t(rows) * kAoThreads * sizeof(uint32_t);
     uint32_t blocks = 0;
     cudaError_t e = cudaMemsetAsync(words, 0, sizeof(uint32_t) * size_t(npix), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_ctr, 0, sizeof(uint32_t), st);
@@ -686,8 +666,7 @@ int rq_launch_ao_depth(rq_ctx* ctx, const rq_bvh* bvh, const float* depth, const
         const rq_triangle* tris = bvh->tris;
         uint32_t* ctr = ctx->d_ctr;
         uint32_t* err = ctx->d_err;
-        int stk = stack;
-        void* args[] = {&nodes, &tris, &depth, &a, &words, &counters, &ctr, &err, &stk};
+        void* args[] = {&nodes, &tris, &depth, &a, &words, &counters, &ctr, &err, &rows};
         e = cudaLaunchKernel(k, dim3(blocks), dim3(kAoThreads), args, smem, st);
     }
     if (e == cudaSuccess) {

@@ -168,17 +168,19 @@ struct ServeSrc {
 };
 
 // At most 72 registers per thread (7 blocks of 128 threads per SM), the
-// budget that measured fastest for the frame's any-hit traversal.  `stack`
-// rows of shared memory per thread (the deepest tree's bound, at most STACK).
-template <bool MT, int STACK>
-__global__ void __launch_bounds__(kST, 7) k_serve(const ServeJob* __restrict__ jobs, const uint32_t* __restrict__ begins,
+// budget that measured fastest for the frame's any-hit traversal.  `rows`
+// stack entries per lane (for the deepest tree); WIDE: a mesh has room for
+// more nodes than a 32-bit entry can name.
+template <bool MT, bool WIDE>
+__global__ void __launch_bounds__(kST, 8) k_serve(const ServeJob* __restrict__ jobs, const uint32_t* __restrict__ begins,
                                                uint32_t njobs, uint32_t total, uint32_t seq, uint32_t* done,
-                                               uint32_t* ctr, uint32_t* err, int stack) {
-    extern __shared__ int32_t smem[];
+                                               uint32_t* ctr, uint32_t* err, int rows) {
+    extern __shared__ __align__(16) int32_t smem[];
     uint32_t* s_begin = reinterpret_cast<uint32_t*>(smem);
     for (uint32_t k = threadIdx.x; k <= njobs; k += kST) s_begin[k] = __ldg(begins + k);
     __syncthreads();
-    int32_t* stk = smem + ((njobs + 1 + 3) & ~3u);
+    using Entry = typename rq::OpenNode<false, WIDE>::Entry;
+    Entry* stk = reinterpret_cast<Entry*>(smem + ((njobs + 1 + 3) & ~3u));
     ServeSrc src;
     src.total = total;
     src.njobs = njobs;
@@ -186,8 +188,8 @@ __global__ void __launch_bounds__(kST, 7) k_serve(const ServeJob* __restrict__ j
     src.jobs = jobs;
     src.s_begin = s_begin;
     src.done = done;
-    rq::trace_persistent<rq::kAnyPerRay, MT, false, STACK, kST>(nullptr, nullptr, src, ctr, stk + threadIdx.x, err,
-                                                                 stack, nullptr, kServeRefill);
+    rq::trace_persistent<rq::kAnyPerRay, MT, false, kST, ServeSrc, 32, WIDE>(nullptr, nullptr, src, ctr,
+                                                                             stk + threadIdx.x, rows, err, kServeRefill);
 }
 
 __global__ void __launch_bounds__(256) k_gen_mesh_rays(const float* __restrict__ pos,
@@ -205,36 +207,29 @@ __global__ void __launch_bounds__(256) k_gen_mesh_rays(const float* __restrict__
     if (any_flags) any_flags[i] = any ? RQ_TRACE_ANY : RQ_TRACE_CLOSEST;
 }
 
-template <class F>
-cudaError_t with_stack(uint32_t bound, F&& f) {
-    if (bound <= 32) return f(std::integral_constant<int, 32>{});
-    if (bound <= 64) return f(std::integral_constant<int, 64>{});
-    return f(std::integral_constant<int, 128>{});
-}
-
 }  // namespace
 
 int rq_launch_serve(rq_ctx* ctx, const ServeJob* jobs, const uint32_t* begins, uint32_t njobs, uint32_t total,
-                    uint32_t max_depth4, uint32_t trace_flags, uint32_t seq, uint32_t* done, uint32_t* ctr,
+                    uint32_t max_depth4, bool wide, uint32_t trace_flags, uint32_t seq, uint32_t* done, uint32_t* ctr,
                     cudaStream_t st) {
     if (njobs == 0 || njobs > RQ_SERVE_MAX_JOBS) return rq_set_error(ctx, RQ_ERR_INVALID_ARG, "bad job count");
     const uint32_t bound = 3u * (max_depth4 + 2u) + 1u;
     if (bound > 128u) return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "4-wide tree deeper than 40 levels");
     const bool mt = trace_flags & RQ_TRI_MT;
-    cudaError_t e = with_stack(bound, [&](auto S) {
-        constexpr int STACK = decltype(S)::value;
-        auto kern = mt ? k_serve<true, STACK> : k_serve<false, STACK>;
-        const size_t smem = size_t((njobs + 1 + 3) & ~3u) * 4u + size_t(bound) * kST * 4u;  // bound <= STACK
-        const size_t smem_max = size_t((RQ_SERVE_MAX_JOBS + 1 + 3) & ~3u) * 4u + size_t(STACK) * kST * 4u;
-        cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_max));
-        int per_sm = 0;
-        if (r == cudaSuccess) r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kST, smem);
-        if (r != cudaSuccess) return r;
+    auto kern = wide ? (mt ? k_serve<true, true> : k_serve<false, true>) : (mt ? k_serve<true, false> : k_serve<false, false>);
+    const int rows = int(max_depth4) + 4;
+    const size_t entry = wide ? 8 : 4;
+    const size_t smem = size_t((njobs + 1 + 3) & ~3u) * 4u + size_t(rows) * kST * entry;
+    cudaError_t e = cudaSuccess;
+    if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    int per_sm = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kST, smem);
+    if (e == cudaSuccess) {
         uint32_t blocks = uint32_t(ctx->num_sms) * uint32_t(per_sm > 0 ? per_sm : 1);
         blocks = std::min(blocks, (total + kST - 1) / kST);
-        kern<<<blocks, kST, smem, st>>>(jobs, begins, njobs, total, seq, done, ctr, ctx->d_err, int(bound));
-        return cudaGetLastError();
-    });
+        kern<<<blocks, kST, smem, st>>>(jobs, begins, njobs, total, seq, done, ctr, ctx->d_err, rows);
+        e = cudaGetLastError();
+    }
     return rq_cuda_status(ctx, e, "serve launch");
 }
 

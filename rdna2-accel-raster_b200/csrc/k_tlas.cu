@@ -28,6 +28,7 @@
 #include "rq_device.cuh"
 #include "rq_internal.h"
 #include "rq_tlas.h"
+#include "trace_engine.cuh"
 
 namespace {
 
@@ -45,8 +46,7 @@ constexpr int kTlasRefill = 8;   // idle lanes of a warp that call for new rays 
 // loop, 605 us at 512 rays per block; 128 (a ray per lane, no refill) 913 us,
 // 1,024 (fewer blocks than fit) 899 us.
 constexpr uint32_t kTlasMaxRays = 2048;
-constexpr uint32_t kFullMask = 0xffffffffu;
-constexpr int32_t kMarker = 0x40000000;  // "leave the instance" (inner entries are < 2^27)
+constexpr int32_t kMarker = 0x40000000;  // pending: leave the instance
 
 __global__ void __launch_bounds__(128) k_instance_boxes(const TlasInst* __restrict__ inst,
                                                         const float* __restrict__ fwd, uint32_t n,
@@ -103,17 +103,20 @@ __device__ __forceinline__ SlabRay slab_setup(F3 o, F3 d) {
 
 // A lane's pending work outside the node loop: a triangle leaf or an instance
 // (entries with bit 31) or the marker that ends an instance.
-template <bool ANY, bool MT>
+template <bool ANY, bool MT, bool WIDE>
 __global__ void __launch_bounds__(kTT, kTlasBlocks)
     k_trace_tlas(const rq_bvh4_node* __restrict__ top_nodes, const uint32_t* __restrict__ top_perm,
                  const TlasInst* __restrict__ inst, const rq_ray* __restrict__ rays, uint32_t n, uint32_t cull,
-                 uint32_t per_block, rq_hit* __restrict__ hits, int stack_cap, uint32_t* err) {
-    extern __shared__ int32_t s_stack[];
+                 uint32_t per_block, rq_hit* __restrict__ hits, int rows, uint32_t* err) {
+    extern __shared__ __align__(16) char s_stack[];
+    using Open = OpenNode<ANY, WIDE>;
+    using Entry = typename Open::Entry;
+    constexpr Entry kLeave = ~Entry(0);  // "leave the instance": no node's entry (a mask of 15 would need node 2^28 - 1)
     __shared__ uint32_t s_next;  // the block's next ray
     if (threadIdx.x == 0) s_next = blockIdx.x * per_block;
     __syncthreads();
     const uint32_t last = min(n, (blockIdx.x + 1u) * per_block);
-    int32_t* stk = s_stack + threadIdx.x;
+    Entry* stk = reinterpret_cast<Entry*>(s_stack) + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
     uint32_t next = 0, end = 0;  // the warp's chunk of ray ids
     bool exhausted = false;
@@ -128,17 +131,17 @@ __global__ void __launch_bounds__(kTT, kTlasBlocks)
     bool hit = false;
     uint32_t hit_inst = 0, hit_prim = 0;
     int sp = 0;
-    int32_t top = 0;  // the stack's top entry
-    bool has_top = false;
+    Open top;  // the deepest open node
+    top.left = 0;
     for (;;) {
         // ---- new rays for idle lanes, once enough are idle
-        uint32_t idle = __ballot_sync(kFullMask, !active);
-        const bool go = __popc(idle) >= kTlasRefill || idle == kFullMask;
+        uint32_t idle = __ballot_sync(kFull, !active);
+        const bool go = __popc(idle) >= kTlasRefill || idle == kFull;
         while (go && idle && !exhausted) {
             if (next == end) {
                 uint32_t base = 0;
                 if (lane == 0) base = atomicAdd(&s_next, 32u);
-                base = __shfl_sync(kFullMask, base, 0);
+                base = __shfl_sync(kFull, base, 0);
                 if (base >= last) {
                     exhausted = true;
                     break;
@@ -158,45 +161,53 @@ __global__ void __launch_bounds__(kTT, kTlasBlocks)
                 nodes = top_nodes;
                 in = nullptr;
                 hit = false;
-                top = 0;
-                has_top = true;
+                top.root();
                 sp = 0;
                 active = true;
             }
             next += take;
-            idle = __ballot_sync(kFullMask, !active);
+            idle = __ballot_sync(kFull, !active);
         }
-        if (!__any_sync(kFullMask, active)) {
+        if (!__any_sync(kFull, active)) {
             if (exhausted) break;
             continue;
         }
         // ---- node phase, until every lane holds other work or is done
-        int32_t pend = 0;  // leaf entries have bit 31 set, the marker is not 0
+        int32_t pend = 0;  // a leaf (bit 31 set) or kMarker
         for (;;) {
-            const bool want = active && pend == 0 && (has_top || sp > 0);
-            if (!__any_sync(kFullMask, want)) break;
+            const bool want = active && pend == 0 && (top.left != 0u || sp > 0);
+            const uint32_t wm = __ballot_sync(kFull, want);
+            if (!wm) break;
+            if (__popc(wm) <= kFewSearch && __popc(__ballot_sync(kFull, pend != 0)) >= kLeafWait) break;
             if (!want) continue;
-            int32_t e;
-            if (has_top) {
-                e = top;
-                has_top = false;
-            } else {
-                e = stk[(--sp) * kTT];
+            if (top.left == 0u) {
+                const Entry e = stk[(--sp) * kTT];
+                if (e == kLeave) {
+                    pend = kMarker;
+                    continue;
+                }
+                top.unpack(e);
             }
-            if (e < 0 || e == kMarker) {
-                pend = e;
+            const uint32_t slot = top.take();
+            int32_t ci, cc;
+            child_of(nodes, top.node, slot, ci, cc);
+            if (cc >= 0) {
+                if (cc > 0) pend = int32_t(0x80000000u | (uint32_t(cc - 1) << 27) | uint32_t(~ci));
                 continue;
             }
-            const float4* np = reinterpret_cast<const float4*>(nodes + e);
             float tk[4];
-            const uint32_t hitm = box4_nf<false>(GlobalRows{np}, sr, tmin, best, tk);
-            const int4 cix = ldg4i(reinterpret_cast<const int4*>(np + 6));
-            const int4 cnt = ldg4i(reinterpret_cast<const int4*>(np + 7));
-            const int32_t aci[4] = {cix.x, cix.y, cix.z, cix.w}, acc[4] = {cnt.x, cnt.y, cnt.z, cnt.w};
-            if (ANY)
-                push_children_any<kTT>(hitm, aci, acc, stk, sp, stack_cap, top, has_top, err, RQ_DERR_STACK);
-            else
-                push_children<kTT>(hitm, aci, acc, tk, true, stk, sp, stack_cap, top, has_top, err, RQ_DERR_STACK);
+            const uint32_t hitm =
+                box4_hits<false>(GlobalRows{reinterpret_cast<const float4*>(nodes + ci)}, sr, tmin, best, tk);
+            if (hitm) {
+                if (top.left) {
+                    if (sp < rows)
+                        stk[(sp++) * kTT] = top.pack();
+                    else
+                        set_err(err, RQ_DERR_STACK);
+                }
+                top.node = ci;
+                top.left = ANY ? hitm : child_sequence(hitm, tk, true);
+            }
         }
         // ---- the lanes' other work
         bool done = false;
@@ -211,7 +222,7 @@ __global__ void __launch_bounds__(kTT, kTlasBlocks)
             } else if (!in) {  // an instance (one per top-level leaf)
                 const TlasInst* cand = inst + __ldg(top_perm + first);
                 if ((__ldg(&cand->mask) & cull) != 0u) {
-                    if (sp + 2 > stack_cap) {
+                    if (sp + 2 > rows) {
                         set_err(err, RQ_DERR_STACK);
                         done = true;
                     } else {
@@ -227,10 +238,9 @@ __global__ void __launch_bounds__(kTT, kTlasBlocks)
                         if (!MT) w = wt_setup(od);
                         nodes = cand->nodes;
                         in = cand;
-                        // what was on top stays above nothing of this instance's
-                        stk[(sp++) * kTT] = kMarker;
-                        top = 0;
-                        has_top = true;
+                        if (top.left) stk[(sp++) * kTT] = top.pack();
+                        stk[(sp++) * kTT] = kLeave;
+                        top.root();
                     }
                 }
             } else {
@@ -257,7 +267,7 @@ __global__ void __launch_bounds__(kTT, kTlasBlocks)
             }
         }
         // ---- report finished rays
-        if (active && (done || (sp == 0 && !has_top))) {
+        if (active && (done || (sp == 0 && top.left == 0u))) {
             uint4 out = make_uint4(0u, __float_as_uint(-1.0f), 0xffffffffu, 0xffffffffu);
             if (hit) out = make_uint4(1u, __float_as_uint(best), hit_inst, hit_prim);
             reinterpret_cast<uint4*>(hits)[id] = out;
@@ -278,10 +288,10 @@ int rq_launch_trace_tlas(rq_ctx* ctx, const rq_tlas* t, const rq_ray* rays, uint
                          uint32_t cull_mask, rq_hit* hits, cudaStream_t st) {
     if (n == 0) return RQ_OK;
     const bool any = flags & RQ_TRACE_ANY, mt = flags & RQ_TRI_MT;
-    const int stack = int((t->stack_bound + 3u) & ~3u);
-    const size_t smem = size_t(stack) * kTT * sizeof(int32_t);
-    auto k = any ? (mt ? k_trace_tlas<true, true> : k_trace_tlas<true, false>)
-                 : (mt ? k_trace_tlas<false, true> : k_trace_tlas<false, false>);
+    const size_t smem = size_t(t->rows) * kTT * (t->wide && !any ? 8 : 4);
+    auto k = any       ? (mt ? k_trace_tlas<true, true, false> : k_trace_tlas<true, false, false>)
+             : t->wide ? (mt ? k_trace_tlas<false, true, true> : k_trace_tlas<false, false, true>)
+                       : (mt ? k_trace_tlas<false, true, false> : k_trace_tlas<false, false, false>);
     cudaError_t e = cudaSuccess;
     if (smem > 48 * 1024) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     int per_sm = 0;
@@ -291,7 +301,7 @@ int rq_launch_trace_tlas(rq_ctx* ctx, const rq_tlas* t, const rq_ray* rays, uint
         const uint32_t share = ((n + fill - 1) / fill + 31u) & ~31u;
         const uint32_t per_block = std::max(uint32_t(kTT), std::min(share, kTlasMaxRays));
         k<<<(n + per_block - 1) / per_block, kTT, smem, st>>>(t->top->nodes4, t->top->perm, t->d_inst, rays, n,
-                                                               cull_mask, per_block, hits, stack, ctx->d_err);
+                                                               cull_mask, per_block, hits, t->rows, ctx->d_err);
         e = cudaGetLastError();
     }
     return rq_cuda_status(ctx, e, "tlas trace launch");

@@ -1,18 +1,13 @@
 // k_trace.cu — ray traversal kernels.
 //
-//  k_trace4   the engine's 4-wide traversal (rq_trace): per-thread stack in
-//             shared memory sized from the tree's depth (3*depth+1 entries
-//             always suffice: each node visit pops one entry and pushes at
-//             most four), 128-B nodes read as eight 16-B vector loads, inner
-//             nodes and leaf children both pushed as entries.  Closest hit:
-//             hit children sorted near-to-far (ties by slot) and pushed
-//             far-first; any hit: pushed slot 3..0 and stop at the first
-//             accepted triangle.  Watertight or Moller-Trumbore triangles.
-//  k_trace_radv  the same rules over a RADV image (Box32 + triangle nodes).
+//  k_trace4   the engine's 4-wide traversal (rq_trace, trace_engine.cuh) over
+//             a ray buffer.  Closest hit: nearest child first (ties by slot);
+//             any hit: by slot, to the first accepted triangle.  Watertight
+//             or Moller-Trumbore triangles.
+//  k_trace_radv  the same order over a RADV image (Box32 + triangle nodes).
 //  k_ref4     software_bvh_bvh4.comp:96-195 as published (24-entry stack that
 //             drops overflow, leaves tested inline far-to-near, RayStats).
 //  k_ref2     software_bvh_lds.comp:86-175 as published (hitFound flag).
-#include <atomic>
 #include "rq_device.cuh"
 #include "rq_internal.h"
 #include "trace_engine.cuh"
@@ -66,18 +61,20 @@ struct BufSrc {
     }
 };
 
-template <bool ANY, bool MT, bool STATS, bool BARY, int STACK>
+// `max_depth`: levels the stack's `rows` entries cover.
+template <bool ANY, bool MT, bool STATS, bool BARY, bool WIDE>
 __global__ void __launch_bounds__(kT, kTraceBlocksPerSm) k_trace4(const rq_bvh4_node* __restrict__ nodes,
                                                const rq_triangle* __restrict__ tris,
                                                const __grid_constant__ BufSrc<STATS, BARY> src,
-                                               const uint32_t* __restrict__ counts, uint32_t* ctr, uint32_t* err) {
-    extern __shared__ int32_t s_stack[];
-    // the stack variant was picked from the host's copy of the depth; the
-    // live depth (after an in-place rebuild) must still fit
-    if (blockIdx.x == 0 && threadIdx.x == 0 && 3u * __ldg(counts + 2) + 1u > uint32_t(STACK))
-        rq::set_err(err, RQ_DERR_STACK);
-    rq::trace_persistent<ANY, MT, STATS, STACK, kT>(nodes, tris, src, ctr, s_stack + threadIdx.x, err, STACK, nullptr,
-                                                    kTraceRefill);
+                                               const uint32_t* __restrict__ counts, uint32_t* ctr, uint32_t* err,
+                                               int rows, uint32_t max_depth) {
+    extern __shared__ __align__(16) char s_stack[];
+    // the rows were picked from the host's copy of the depth; the live depth
+    // (after an in-place rebuild) must still fit
+    if (blockIdx.x == 0 && threadIdx.x == 0 && __ldg(counts + 2) > max_depth) rq::set_err(err, RQ_DERR_STACK);
+    using Entry = typename rq::OpenNode<ANY, WIDE>::Entry;
+    rq::trace_persistent<ANY, MT, STATS, kT, const BufSrc<STATS, BARY>, 32, WIDE>(
+        nodes, tris, src, ctr, reinterpret_cast<Entry*>(s_stack) + threadIdx.x, rows, err, kTraceRefill);
 }
 
 template <bool ANY, bool MT, bool BARY>
@@ -321,55 +318,41 @@ __global__ void __launch_bounds__(kT) k_ref2(const rq_bvh2_node* __restrict__ no
     flags[idx] = hitFound;
 }
 
-template <bool ANY, bool MT, bool STATS, bool BARY, int STACK>
+template <bool ANY, bool MT, bool EX>
 cudaError_t launch4(rq_ctx* ctx, const rq_bvh* b, const rq_ray* rays, uint32_t n, rq_hit* hits, float* bary,
                     rq_ray_stats* stats, cudaStream_t st) {
-    auto kern = k_trace4<ANY, MT, STATS, BARY, STACK>;
-    const size_t smem = size_t(STACK) * kT * sizeof(int32_t);
-    // blocks per SM of this variant, found on its first launch on each device
-    // (the shared-memory attribute is per device; the host calls cost more
-    // than a small launch's kernel)
-    static std::atomic<int> s_per_sm[64];
-    const int dev = ctx->device;
-    int per_sm = (dev >= 0 && dev < 64) ? s_per_sm[dev].load(std::memory_order_relaxed) : 0;
-    cudaError_t e = cudaSuccess;
-    if (per_sm == 0) {
-        if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kT, smem);
-        if (e != cudaSuccess) return e;
-        if (per_sm < 1) per_sm = 1;
-        if (dev >= 0 && dev < 64) s_per_sm[dev].store(per_sm, std::memory_order_relaxed);
-    }
+    // Stack rows (an entry per open node of a path) by the depth the host
+    // knows, with room for the levels an in-place rebuild may add.  At most
+    // 44 rows of 4 or 8 bytes: kTraceBlocksPerSm blocks always fit an SM
+    // (64 registers, 45 KB at most with the 8-byte entries of 4 blocks).
+    const uint32_t d = b->h_counts[2];
+    const uint32_t max_depth = d <= 8u ? 10u : (d <= 19u ? 21u : 42u);
+    const bool wide = !ANY && b->cap_nodes4 > RQ_NARROW_NODES;
+    auto kern = wide ? k_trace4<ANY, MT, EX, EX, !ANY> : k_trace4<ANY, MT, EX, EX, false>;
+    const int rows = int(max_depth) + 2;
+    const size_t smem = size_t(rows) * kT * (wide ? 8 : 4);
     // persistent grid: every SM filled, never more blocks than 32-ray chunks
-    uint32_t blocks = uint32_t(ctx->num_sms) * uint32_t(per_sm > 0 ? per_sm : 1);
+    uint32_t blocks = uint32_t(ctx->num_sms) * uint32_t(wide && rows > 24 ? 4 : kTraceBlocksPerSm);
     const uint32_t need = (n + kT - 1) / kT;
     if (blocks > need) blocks = need;
-    BufSrc<STATS, BARY> src;
+    BufSrc<EX, EX> src;
     src.total = n;
     src.rays = rays;
     src.perm = b->perm;
     src.hits = hits;
     src.bary = bary;
     src.stats = stats;
-    e = cudaMemsetAsync(ctx->d_ctr, 0, sizeof(uint32_t), st);
+    cudaError_t e = cudaMemsetAsync(ctx->d_ctr, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    kern<<<blocks, kT, smem, st>>>(b->nodes4, b->tris, src, b->d_counts, ctx->d_ctr, ctx->d_err);
+    kern<<<blocks, kT, smem, st>>>(b->nodes4, b->tris, src, b->d_counts, ctx->d_ctr, ctx->d_err, rows, max_depth);
     return cudaGetLastError();
 }
 
-template <bool ANY, bool MT, bool STATS, bool BARY>
-cudaError_t launch4_stack(uint32_t bound, rq_ctx* ctx, const rq_bvh* b, const rq_ray* rays, uint32_t n,
-                          rq_hit* hits, float* bary, rq_ray_stats* stats, cudaStream_t st) {
-    if (bound <= 32) return launch4<ANY, MT, STATS, BARY, 32>(ctx, b, rays, n, hits, bary, stats, st);
-    if (bound <= 64) return launch4<ANY, MT, STATS, BARY, 64>(ctx, b, rays, n, hits, bary, stats, st);
-    return launch4<ANY, MT, STATS, BARY, 128>(ctx, b, rays, n, hits, bary, stats, st);
-}
-
 template <bool ANY, bool MT>
-cudaError_t launch4_opts(uint32_t bound, bool ex, rq_ctx* ctx, const rq_bvh* b, const rq_ray* rays, uint32_t n,
-                         rq_hit* hits, float* bary, rq_ray_stats* stats, cudaStream_t st) {
-    if (ex) return launch4_stack<ANY, MT, true, true>(bound, ctx, b, rays, n, hits, bary, stats, st);
-    return launch4_stack<ANY, MT, false, false>(bound, ctx, b, rays, n, hits, bary, stats, st);
+cudaError_t launch4_opts(bool ex, rq_ctx* ctx, const rq_bvh* b, const rq_ray* rays, uint32_t n, rq_hit* hits,
+                         float* bary, rq_ray_stats* stats, cudaStream_t st) {
+    if (ex) return launch4<ANY, MT, true>(ctx, b, rays, n, hits, bary, stats, st);
+    return launch4<ANY, MT, false>(ctx, b, rays, n, hits, bary, stats, st);
 }
 
 }  // namespace
@@ -377,9 +360,6 @@ cudaError_t launch4_opts(uint32_t bound, bool ex, rq_ctx* ctx, const rq_bvh* b, 
 int rq_launch_trace(rq_ctx* ctx, const rq_bvh* bvh, const rq_ray* rays, uint32_t n, uint32_t flags, rq_hit* hits,
                     float* bary, rq_ray_stats* stats, cudaStream_t st) {
     if (n == 0) return RQ_OK;
-    // stack entries: 3 per level below the root plus one, with two levels of
-    // headroom for in-place rebuilds whose depth the host has not seen yet
-    uint32_t bound = 3u * (bvh->h_counts[2] + 2u) + 1u;
     if (3u * bvh->h_counts[2] + 1u > 128u)
         return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "4-wide tree deeper than 42 levels");
     // With stats or barycentrics requested, the kernel variant that records
@@ -397,13 +377,13 @@ int rq_launch_trace(rq_ctx* ctx, const rq_bvh* bvh, const rq_ray* rays, uint32_t
     const bool ex = stats || bary;
     cudaError_t e;
     if (any && mt)
-        e = launch4_opts<true, true>(bound, ex, ctx, bvh, rays, n, hits, ba_out, st_out, st);
+        e = launch4_opts<true, true>(ex, ctx, bvh, rays, n, hits, ba_out, st_out, st);
     else if (any)
-        e = launch4_opts<true, false>(bound, ex, ctx, bvh, rays, n, hits, ba_out, st_out, st);
+        e = launch4_opts<true, false>(ex, ctx, bvh, rays, n, hits, ba_out, st_out, st);
     else if (mt)
-        e = launch4_opts<false, true>(bound, ex, ctx, bvh, rays, n, hits, ba_out, st_out, st);
+        e = launch4_opts<false, true>(ex, ctx, bvh, rays, n, hits, ba_out, st_out, st);
     else
-        e = launch4_opts<false, false>(bound, ex, ctx, bvh, rays, n, hits, ba_out, st_out, st);
+        e = launch4_opts<false, false>(ex, ctx, bvh, rays, n, hits, ba_out, st_out, st);
     return rq_cuda_status(ctx, e, "trace launch");
 }
 

@@ -27,6 +27,10 @@
 // Largest triangle count a leaf stack entry can address (27-bit first prim).
 #define RQ_MAX_TRIANGLES (1u << 27)
 
+// 4-wide nodes a closest-hit traversal's 32-bit stack entry can name (23 bits
+// beside 9 of child order); trees with room for more use 64-bit entries.
+#define RQ_NARROW_NODES (1u << 23)
+
 struct rq_ctx {
     int device = 0;
     int num_sms = 0;

@@ -32,7 +32,7 @@ static_assert(sizeof(ServeJob) == 96, "ServeJob layout");
 // device `begins` of njobs + 1 entries, the last = total ids).  `done`
 // holds njobs zeroed counters; `ctr` one zeroed work counter.
 int rq_launch_serve(rq_ctx* ctx, const ServeJob* jobs, const uint32_t* begins, uint32_t njobs, uint32_t total,
-                    uint32_t max_depth4, uint32_t trace_flags, uint32_t seq, uint32_t* done, uint32_t* ctr,
+                    uint32_t max_depth4, bool wide, uint32_t trace_flags, uint32_t seq, uint32_t* done, uint32_t* ctr,
                     cudaStream_t st);
 int rq_launch_gen_mesh_rays(rq_ctx* ctx, const float* pos, const uint32_t* idx, uint32_t ntri, uint32_t kind,
                             uint32_t seed, uint32_t n, rq_ray* rays, uint32_t* any_flags, cudaStream_t st);

@@ -27,7 +27,8 @@ struct rq_tlas {
     float* d_fwd = nullptr;       // 12 floats per instance: object -> world
     float* d_tri9 = nullptr;      // the instances' world boxes as degenerate triangles
     rq_bvh* top = nullptr;        // BVH over the instance boxes, one instance per leaf
-    uint32_t stack_bound = 0;     // entries per ray: top + marker + deepest BLAS
+    int rows = 0;                 // stack entries per ray: top level, marker, deepest BLAS
+    bool wide = false;            // a tree has room for more nodes than a 32-bit entry can name
     cudaStream_t last_stream = nullptr;
 };
 

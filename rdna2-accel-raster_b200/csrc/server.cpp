@@ -340,6 +340,7 @@ struct rq_server {
         uint32_t* hb = reinterpret_cast<uint32_t*>(static_cast<char*>(sl->h_buf) + kBeginsOff);
         const uint32_t seqno = ++seq;
         uint32_t begin = 0, depth = 0;
+        bool wide = false;
         for (size_t j = 0; j < sel.size(); ++j) {
             const rq_request& r = sel[j].p.req;
             MeshRec* m = mesh(r.mesh);
@@ -362,6 +363,7 @@ struct rq_server {
             hb[j] = begin;
             begin += (r.num_rays + 31u) & ~31u;
             depth = std::max(depth, m->depth4);
+            wide |= m->bvh->cap_nodes4 > RQ_NARROW_NODES;
         }
         const uint32_t nj = uint32_t(sel.size());
         hb[nj] = begin;
@@ -382,7 +384,7 @@ struct rq_server {
         }
         if (rc == RQ_OK)
             rc = rq_launch_serve(ctx, reinterpret_cast<const ServeJob*>(d), reinterpret_cast<const uint32_t*>(d + kBeginsOff),
-                                 nj, begin, depth, cfg.trace_flags, seqno, reinterpret_cast<uint32_t*>(d + kDoneOff),
+                                 nj, begin, depth, wide, cfg.trace_flags, seqno, reinterpret_cast<uint32_t*>(d + kDoneOff),
                                  reinterpret_cast<uint32_t*>(d + kCtrOff), sl->st);
         if (rc == RQ_OK) rc = rq_cuda_status(ctx, cudaEventRecord(sl->ev, sl->st), "serve event");
         const double t = now();

@@ -58,7 +58,7 @@ int build(rq_ctx* ctx, const rq_instance* instances, uint32_t n, rq_tlas** out, 
     std::vector<char> table(inst_bytes + fwd_bytes);
     TlasInst* inst = reinterpret_cast<TlasInst*>(table.data());
     float* fwd = reinterpret_cast<float*>(table.data() + inst_bytes);
-    uint32_t blas_bound = 0;
+    uint32_t blas_bound = 0, blas_depth = 0, most_nodes = n;
     // The live depth of each BLAS costs a stream synchronisation and a copy,
     // so it is read once per handle, not once per instance: 256 instances of
     // 8 meshes took 5.0 ms on the host, most of it in 256 such reads.
@@ -86,6 +86,8 @@ int build(rq_ctx* ctx, const rq_instance* instances, uint32_t n, rq_tlas** out, 
         inst[i].instance_id = s.instance_id;
         inst[i].mask = s.mask;
         blas_bound = std::max(blas_bound, 3u * (seen->second + 2u) + 1u);
+        blas_depth = std::max(blas_depth, seen->second);
+        most_nodes = std::max(most_nodes, s.blas->cap_nodes4);
     }
     rq_tlas* t = new (std::nothrow) rq_tlas();
     if (!t) return RQ_ERR_OOM;
@@ -104,8 +106,10 @@ int build(rq_ctx* ctx, const rq_instance* instances, uint32_t n, rq_tlas** out, 
     if (rc == RQ_OK) rc = rq_build(ctx, t->d_tri9, 12, 3 * n, nullptr, n, 1, RQ_BUILD_BVH4, &t->top, stream);
     if (rc == RQ_OK) {
         // (a first build has read its node counts back)
-        t->stack_bound = 3u * (t->top->h_counts[2] + 2u) + 1u + 1u + blas_bound;
-        if (t->stack_bound > 256u) rc = rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "scene too deep for the stack");
+        const uint32_t top_depth = t->top->h_counts[2];
+        t->rows = int(top_depth + blas_depth) + 8;
+        t->wide = most_nodes > RQ_NARROW_NODES;
+        if (3u * (top_depth + 2u) + 1u + 1u + blas_bound > 256u) rc = rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "scene too deep for the stack");
     }
     if (rc) {
         free_tlas(t);

@@ -1,26 +1,40 @@
 // trace_engine.cuh — persistent traversal with per-lane ray refill.
 //
 // Every lane of a warp owns one ray at a time.  Ray ids come from a global
-// counter in chunks of 32 (one atomic per chunk); whenever lanes are idle,
+// counter in chunks (one atomic per chunk); whenever enough lanes are idle,
 // a ballot and a rank within the idle mask hand them the next ids, so a warp
-// keeps 32 rays in flight until the ids run out.  Each round:
-//   1. inner phase — lanes without a pending leaf pop stack entries; an inner
-//      node is box-tested and its hit children pushed (closest hit: sorted
-//      near-to-far and pushed far-first; any hit: slot 3..0), a leaf entry is
-//      parked as the lane's pending leaf; the phase ends when no lane wants
-//      another inner node (every lane parked a leaf or ran out of entries);
+// keeps its rays in flight until the ids run out.  Each round:
+//   1. node phase — lanes without a parked leaf take the next child of the
+//      deepest open node: an inner child is opened (its four boxes tested, the
+//      hit ones noted with their order), a leaf is parked; the phase ends when
+//      no lane searches, or few do while others wait with leaves;
 //   2. leaf phase — lanes test their parked leaf's triangles in order;
-//   3. lanes whose stack is empty, or whose any-hit ray found a hit, report
-//      the result to the ray source and become idle.
-// With INLOOP, lanes whose stack runs out during the inner phase report at
-// once and idle lanes are refilled inside the inner phase too, which then
-// ends only when no lane searches or `leaf_batch` lanes hold a parked leaf:
-// rays that need few nodes no longer wait for the warp's longest one.
-// Per ray this visits stack entries in exactly the order of a sequential
-// pop-process-push traversal, so results do not depend on which lane or
-// round a ray runs in and match the oracle's traversal bit for bit.  The
-// stack's top entry is held in a register (the first child to visit after a
-// node never goes through shared memory).
+//   3. lanes that have nothing left to visit, or whose any-hit ray found a
+//      hit, report the result to the ray source and become idle.
+// Per ray the children are visited in exactly the order of a sequential
+// depth-first traversal (closest hit: nearest child first, ties by slot; any
+// hit: by slot), so results do not depend on which lane or round a ray runs
+// in and match the oracle's traversal bit for bit.
+//
+// The open nodes of a ray are a path, so the stack holds one entry per open
+// node with children left — its index and their order — rather than one per
+// child: depth + 1 rows where 3 * depth + 1 were needed (15 for 43 on the
+// 2.5M-triangle frame's tree; the shared memory goes to the L1).  Where a
+// child leads (child_index, child_count) is read when its turn comes, not for
+// all four when the node is opened: the box test needs six of the node's
+// eight rows, an unvisited child costs nothing, and an any-hit node's entry
+// is its hit mask as it stands.  Measured against an entry per child with its
+// target resolved when its node is opened: 2^20 incoherent rays on 999,698
+// triangles (closest hit) 511 -> 412 us; the 1080p frame's 27.1M shadow and AO
+// rays 6.17 -> 5.59 ms; 2.07M camera rays on 8.3M triangles 1.94 -> 1.64 ms.
+// What bounds it now is the L1 (LSU wavefronts at 72 % of their peak on the
+// shadow rays, 83 % on the incoherent ones: lanes of a warp read different
+// nodes) together with instruction issue (69 % and 52 %).
+// Tried here and no faster: 32-byte loads of two rows with the planes picked
+// by selects (shadow 5.75 ms, incoherent 393 us), packed two-wide plane
+// distances (spills), 56 or 48 registers for 36 or 40 warps per SM (shadow
+// 5.73 / 5.76 ms), speculative traversal, refilling inside the node loop,
+// staging the top levels in shared memory.
 //
 // A ray source provides:
 //   uint32_t total;                                 number of ray ids
@@ -29,12 +43,14 @@
 //   optional: kRoundEnd = true and void round_end(bool finished, const Meta& m).
 #pragma once
 
+#include <type_traits>
+
 #include "rq_device.cuh"
 #include "rq_internal.h"
 
 namespace rq {
 
-constexpr int32_t kNoLeaf = 0;  // leaf entries always have bit 31 set
+constexpr int32_t kNoLeaf = 0;  // a parked leaf always has bit 31 set
 constexpr uint32_t kFull = 0xffffffffu;
 constexpr uint32_t kChunk = 32;  // default ray ids per refill atomic
 
@@ -79,105 +95,87 @@ struct Hit {
     uint32_t boxes, tris;
 };
 
-// ----------------------------------------------------------- top levels
-// The top TOP levels of a 4-wide tree (at most (4^TOP - 1) / 3 nodes, the
-// root first, breadth-first) staged in shared memory by every block.  A
-// staged node occupies kTopStride float4 (144 B: node k starts 4 banks
-// after node k-1, so 16-B reads of different nodes by one quarter-warp do
-// not collide); its inner children that are staged too have child index
-// kStaged | slot.  Stack entries with kStaged name a shared-memory slot.
-constexpr int32_t kStaged = 0x40000000;
-constexpr int kTopStride = 9;
+// ---------------------------------------------------------------- open nodes
+// The deepest open node of a ray: its index (kRootRef: the root itself is the
+// next child) and the children left to visit.  MASK (any-hit kernels): `left`
+// is a mask of slots, visited from the lowest.  Otherwise a sequence of 3-bit
+// fields 4 | slot, the next one lowest; at most four, and at most three once
+// the first has been taken, which is when the node can go to the stack.
+// Stack entries are node << 4 | mask or node << 9 | sequence in 32 bits: the
+// sequence form holds node indices below 2^23 (RQ_NARROW_NODES), so trees with
+// more room than that run with 64-bit entries (WIDE).
+constexpr int32_t kRootRef = -1;
 
-template <int TOP>
-struct TopLevels {
-    static constexpr int kMax = TOP <= 0 ? 0 : ((1 << (2 * TOP)) - 1) / 3;
-    // shared memory: the nodes, slot -> global index, slot x child -> slot, count
-    static constexpr size_t kBytes = TOP <= 0 ? 0 : size_t(kMax) * kTopStride * 16 + size_t(kMax) * 5 * 4 + 16;
+template <bool MASK, bool WIDE>
+struct OpenNode {
+    using Entry = typename std::conditional<WIDE, unsigned long long, uint32_t>::type;
+    static constexpr int kBits = MASK ? 4 : 9;
+    int32_t node;
+    uint32_t left;
+
+    __device__ __forceinline__ void root() {
+        node = kRootRef;
+        left = 4u;  // (one child, whichever the form)
+    }
+    __device__ __forceinline__ Entry pack() const { return (Entry(uint32_t(node)) << kBits) | left; }
+    __device__ __forceinline__ void unpack(Entry e) {
+        node = int32_t(e >> kBits);
+        left = uint32_t(e) & ((1u << kBits) - 1u);
+    }
+    __device__ __forceinline__ uint32_t take() {
+        if (MASK) {
+            const uint32_t k = uint32_t(__ffs(left)) - 1u;
+            left &= left - 1u;
+            return k;
+        }
+        const uint32_t k = left & 3u;
+        left >>= 3;
+        return k;
+    }
 };
 
-// Stage the top levels (call with the whole block, before any traversal).
-// `s_top` points at TopLevels<TOP>::kBytes of 16-B aligned shared memory.
-template <int TOP>
-__device__ __forceinline__ void stage_top(const rq_bvh4_node* __restrict__ nodes, float4* s_top) {
-    constexpr int kMax = TopLevels<TOP>::kMax;
-    int32_t* s_g = reinterpret_cast<int32_t*>(s_top + kMax * kTopStride);
-    int32_t* s_c = s_g + kMax;
-    uint32_t* s_n = reinterpret_cast<uint32_t*>(s_c + 4 * kMax);
-    if (threadIdx.x < 32) {
-        const uint32_t lane = threadIdx.x;
-        for (int i = lane; i < 4 * kMax; i += 32) s_c[i] = -1;
-        if (lane == 0) s_g[0] = 0;
-        __syncwarp();
-        uint32_t n = 1, lo = 0, hi = 1;
-        for (int lvl = 1; lvl < TOP; ++lvl) {
-            for (uint32_t b = lo; b < hi; b += 32) {
-                const uint32_t s = b + lane;
-                int4 ci = make_int4(0, 0, 0, 0), cc = make_int4(0, 0, 0, 0);
-                if (s < hi) {
-                    const int4* np = reinterpret_cast<const int4*>(nodes + s_g[s]);
-                    ci = __ldg(np + 6);
-                    cc = __ldg(np + 7);
-                }
-                const int32_t x[4] = {ci.x, ci.y, ci.z, ci.w}, c[4] = {cc.x, cc.y, cc.z, cc.w};
+// The order of a node's hit children as a sequence: near to far with ties by
+// slot (sorted), or by slot.
+__device__ __forceinline__ uint32_t child_sequence(uint32_t hitm, const float (&tk)[4], bool sorted) {
+    float t[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const bool inner = s < hi && c[k] < 0;
-                    const uint32_t m = __ballot_sync(kFull, inner);
-                    if (inner) {
-                        const uint32_t slot = n + __popc(m & ((1u << lane) - 1u));
-                        s_g[slot] = x[k];
-                        s_c[4 * s + k] = int32_t(slot);
-                    }
-                    n += __popc(m);
-                }
-                __syncwarp();
-            }
-            lo = hi;
-            hi = n;
-        }
-        if (lane == 0) *s_n = n;
-    }
-    __syncthreads();
-    const uint32_t n = *s_n;
-    for (uint32_t i = threadIdx.x; i < n * 8u; i += blockDim.x) {
-        const uint32_t s = i >> 3, j = i & 7u;
-        float4 v = __ldg(reinterpret_cast<const float4*>(nodes + s_g[s]) + j);
-        if (j == 6) {
-            int32_t ci[4] = {__float_as_int(v.x), __float_as_int(v.y), __float_as_int(v.z), __float_as_int(v.w)};
+    for (int k = 0; k < 4; ++k) t[k] = ((hitm >> k) & 1u) ? (sorted ? tk[k] : 0.0f) : INFINITY;
+    const uint32_t p01 = t[0] <= t[1], p02 = t[0] <= t[2], p03 = t[0] <= t[3], p12 = t[1] <= t[2], p13 = t[1] <= t[3],
+                   p23 = t[2] <= t[3];
+    const uint32_t r[4] = {3u - (p01 + p02 + p03), p01 + 2u - (p12 + p13), p02 + p12 + 1u - p23, p03 + p13 + p23};
+    uint32_t s = 0;
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (s_c[4 * s + k] >= 0) ci[k] = kStaged | s_c[4 * s + k];
-            v = make_float4(__int_as_float(ci[0]), __int_as_float(ci[1]), __int_as_float(ci[2]), __int_as_float(ci[3]));
-        }
-        s_top[s * kTopStride + j] = v;
-    }
-    __syncthreads();
+    for (uint32_t k = 0; k < 4; ++k) s |= ((hitm >> k) & 1u) ? (4u | k) << (3u * r[k]) : 0u;
+    return s;
 }
 
-// STACK bounds the entries per lane (stk has STACK rows of STRIDE words);
-// stack_cap, if smaller, is the bound actually allocated.  CHUNK: ray ids
-// taken per atomic.  refill_min: idle lanes get new rays only once at least
-// this many lanes of the warp are idle (or all are), so that lanes join in
-// groups and a warp's rays stay closer in position and direction.  TOP > 0:
-// the top levels were staged in s_top by stage_top<TOP> (single-BVH sources
-// only).  SPEC: speculative traversal
-// (Aila and Laine 2009) — it changes the order in which a ray meets its
-// nodes, so it is only for any-hit rays whose result is hit or miss alone
-// (which triangle was found first is not reported by such sources).
-// INLOOP: finish and refill inside the inner phase (above); leaf_batch: the
-// parked leaves that end an INLOOP inner phase (1..32).  Neither changes a
-// ray's order of nodes.
-template <int ANY, bool MT, bool STATS, int STACK, int STRIDE, class Src, int CHUNK = int(kChunk), int TOP = 0,
-          bool SPEC = false, bool INLOOP = false>
+// Where child `slot` of `node` leads: child_index, child_count.
+__device__ __forceinline__ void child_of(const rq_bvh4_node* __restrict__ nodes, int32_t node, uint32_t slot,
+                                         int32_t& ci, int32_t& cc) {
+    ci = 0;
+    cc = -1;  // (the root)
+    if (node >= 0) {
+        const int32_t* q = reinterpret_cast<const int32_t*>(nodes + node) + 24 + slot;
+        ci = __ldg(q);
+        cc = __ldg(q + 4);
+    }
+}
+
+// Leaves of the node phase: it ends once at most kFewSearch lanes search while
+// kLeafWait hold a leaf (measured on B200: 8 and 8; without it the 1080p
+// frame's shadow pass was 3 %, the depth-AO pass 13 % slower, 16 and 8 were
+// 3 % and 4 % slower than 8 and 8).
+constexpr int kFewSearch = 8, kLeafWait = 8;
+
+// stk: this lane's column of `rows` stack entries, STRIDE apart.  CHUNK: ray
+// ids taken per atomic.  refill_min: idle lanes get new rays only once at
+// least this many lanes of the warp are idle (or all are), so that lanes join
+// in groups and a warp's rays stay closer in position and direction.
+template <int ANY, bool MT, bool STATS, int STRIDE, class Src, int CHUNK = int(kChunk), bool WIDE = false>
 __device__ __forceinline__ void trace_persistent(const rq_bvh4_node* __restrict__ nodes,
                                                  const rq_triangle* __restrict__ tris, Src& src, uint32_t* ctr,
-                                                 int32_t* stk, uint32_t* err, int stack_cap = STACK,
-                                                 const float4* s_top = nullptr, int refill_min = 1,
-                                                 int leaf_batch = 32) {
-    static_assert(TOP == 0 || !IsMulti<Src>::value, "top-level staging needs one BVH per launch");
-    static_assert(!SPEC || ANY == 1, "speculative traversal changes which hit an any-hit ray finds first");
-    static_assert(!INLOOP || !HasRoundEnd<Src>::value, "in-loop refill reports rays outside the round hooks");
+                                                 typename OpenNode<ANY == 1, WIDE>::Entry* stk, int rows,
+                                                 uint32_t* err, int refill_min = 1) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
     // warp-uniform chunk of ray ids
@@ -191,9 +189,9 @@ __device__ __forceinline__ void trace_persistent(const rq_bvh4_node* __restrict_
     SlabRay sr;
     WtRay w;
     float best = 0.0f;
-    int sp = 0;            // entries in the shared-memory stack
-    int32_t top = 0;       // the stack's top entry, kept in a register
-    bool has_top = false;
+    OpenNode<ANY == 1, WIDE> top;  // the deepest open node
+    top.left = 0;
+    int sp = 0;  // entries on the stack
     Hit h;
     h.hit = false;
     h.t = 0.0f;
@@ -201,12 +199,8 @@ __device__ __forceinline__ void trace_persistent(const rq_bvh4_node* __restrict_
     h.u = h.v = 0.0f;
     h.boxes = h.tris = 0;
 
-    int32_t leaf = kNoLeaf;  // the lane's parked leaf entry
-    bool stalled = false;    // SPEC: a second leaf waits in `top`
-
-    // hand the next ray ids to idle lanes once refill_min of them are idle
-    // (called by all 32 lanes together)
-    auto refill = [&]() {
+    for (;;) {
+        // ---- new rays for idle lanes, once refill_min of them are idle
         uint32_t idle = __ballot_sync(kFull, !active);
         const bool go = __popc(idle) >= refill_min || idle == kFull;
         while (go && idle && !exhausted) {
@@ -240,11 +234,8 @@ __device__ __forceinline__ void trace_persistent(const rq_bvh4_node* __restrict_
                     h.idx = kNoHit;
                     h.u = h.v = 0.0f;
                     h.boxes = h.tris = 0;
-                    top = TOP > 0 ? kStaged : 0;  // the root (slot 0 when staged)
-                    has_top = true;
+                    top.root();
                     sp = 0;
-                    leaf = kNoLeaf;
-                    stalled = false;
                 }
             }
             next += take;
@@ -252,82 +243,42 @@ __device__ __forceinline__ void trace_persistent(const rq_bvh4_node* __restrict_
             // empty pixel) take the next id at once
             idle = __ballot_sync(kFull, !active);
         }
-    };
-
-    for (;;) {
-        // ---- refill idle lanes
-        refill();
         if (!__any_sync(kFull, active)) {
             if (exhausted) break;
             continue;
         }
 
-        // ---- inner phase (SPEC: lanes holding a leaf keep taking inner
-        // nodes while other lanes still search; a second leaf stays on the
-        // stack and stalls the lane until the leaf phase)
-        leaf = kNoLeaf;
-        stalled = false;
+        // ---- node phase
+        int32_t leaf = kNoLeaf;
         for (;;) {
-            if constexpr (INLOOP) {
-                // a ray whose stack ran out with no leaf pending is done
-                if (active && !(has_top || sp > 0) && leaf == kNoLeaf) {
-                    h.t = best;
-                    src.finish(rid, meta, ray, h);
-                    active = false;
-                }
-                refill();
-            }
-            const bool left = has_top || sp > 0;
-            const bool searching = active && left && leaf == kNoLeaf;
-            if (!__any_sync(kFull, searching)) break;
-            if constexpr (INLOOP) {
-                if (__popc(__ballot_sync(kFull, active && leaf != kNoLeaf)) >= leaf_batch) break;
-            }
-            const bool want = SPEC ? (active && left && !stalled) : searching;
-            if (!want) continue;
-            int32_t e;
-            if (has_top) {
-                e = top;
-                has_top = false;
-            } else {
-                e = stk[(--sp) * STRIDE];
-            }
-            if (e < 0) {
-                if (!SPEC || leaf == kNoLeaf) {
-                    leaf = e;
-                } else {
-                    top = e;
-                    has_top = true;
-                    stalled = true;
-                }
+            const bool search = active && leaf == kNoLeaf && (top.left != 0u || sp > 0);
+            const uint32_t sm = __ballot_sync(kFull, search);
+            if (!sm) break;
+            if (__popc(sm) <= kFewSearch && __popc(__ballot_sync(kFull, leaf != kNoLeaf)) >= kLeafWait) break;
+            if (!search) continue;
+            if (top.left == 0u) top.unpack(stk[(--sp) * STRIDE]);
+            const uint32_t slot = top.take();
+            const rq_bvh4_node* nb = IsMulti<Src>::value ? ray.nodes : nodes;
+            int32_t ci, cc;
+            child_of(nb, top.node, slot, ci, cc);
+            if (cc >= 0) {  // a leaf (or an empty slot whose point box the ray met)
+                if (cc > 0) leaf = int32_t(0x80000000u | (uint32_t(cc - 1) << 27) | uint32_t(~ci));
                 continue;
             }
-            // box tests, each axis's near and far plane rows chosen by the
-            // ray's signs
             float tk[4];
-            uint32_t hitm;
-            int4 cix, cnt;
-            if (TOP > 0 && (e & kStaged)) {
-                const float4* sp4 = s_top + (e & ~kStaged) * kTopStride;
-                hitm = box4_nf<false>([&](int i) { return sp4[i]; }, sr, ray.tmin, best, tk);
-                const float4 a = sp4[6], b = sp4[7];
-                cix = make_int4(__float_as_int(a.x), __float_as_int(a.y), __float_as_int(a.z), __float_as_int(a.w));
-                cnt = make_int4(__float_as_int(b.x), __float_as_int(b.y), __float_as_int(b.z), __float_as_int(b.w));
-            } else {
-                const rq_bvh4_node* nb = IsMulti<Src>::value ? ray.nodes : nodes;
-                const float4* np = reinterpret_cast<const float4*>(nb + e);
-                hitm = box4_nf<false>([&](int i) { return ldg4(np + i); }, sr, ray.tmin, best, tk);
-                cix = ldg4i(reinterpret_cast<const int4*>(np + 6));
-                cnt = ldg4i(reinterpret_cast<const int4*>(np + 7));
-            }
+            const uint32_t hitm = box4_hits<false>(GlobalRows{reinterpret_cast<const float4*>(nb + ci)}, sr, ray.tmin,
+                                                   best, tk);
             if (STATS) h.boxes += 4;
-            const int32_t aci[4] = {cix.x, cix.y, cix.z, cix.w}, acc[4] = {cnt.x, cnt.y, cnt.z, cnt.w};
-            // closest hit: near to far; any hit: slot order.  The first child
-            // to visit stays in the register.
-            if (ANY == 1 || (ANY == kAnyPerRay && ray.any))
-                push_children_any<STRIDE>(hitm, aci, acc, stk, sp, stack_cap, top, has_top, err, RQ_DERR_STACK);
-            else
-                push_children<STRIDE>(hitm, aci, acc, tk, true, stk, sp, stack_cap, top, has_top, err, RQ_DERR_STACK);
+            if (hitm) {
+                if (top.left) {
+                    if (sp < rows)
+                        stk[(sp++) * STRIDE] = top.pack();
+                    else
+                        set_err(err, RQ_DERR_STACK);  // deeper than the host knew
+                }
+                top.node = ci;
+                top.left = ANY == 1 ? hitm : child_sequence(hitm, tk, ANY == 0 || !ray.any);
+            }
         }
 
         // ---- leaf phase
@@ -359,7 +310,7 @@ __device__ __forceinline__ void trace_persistent(const rq_bvh4_node* __restrict_
 
         // ---- report finished rays
         bool fin = false;
-        if (active && (done || (sp == 0 && !has_top))) {
+        if (active && (done || (sp == 0 && top.left == 0u))) {
             h.t = best;
             src.finish(rid, meta, ray, h);
             active = false;

@@ -2,10 +2,8 @@
 
 `python -m rq.tune --out FILE` times, on the device:
   - the 1080p shadows + AO frame's traversal (rq_render_shadow_ao) in every
-    block size x refill chunk x register budget, with and without staged top
-    levels and speculative traversal, then the refill threshold, then the
-    in-loop refill shapes x refill threshold x leaf batch (median of 5 runs
-    each);
+    block size x refill chunk x register budget, then the refill threshold
+    (median of 5 runs each);
   - the batched workload (512 deforming grids, 4,096 any-hit + 4,096
     closest-hit rays per mesh) through rq_batch_autotune: every build block
     size x blocks per SM, every traversal block size x chunk x register budget;
@@ -42,22 +40,20 @@ def lookup(key, path=TABLE):
     return e["shape"] if e else None
 
 
-# (threads, refill chunk, register budget, staged top levels, speculative)
+# (threads, refill chunk, register budget, top levels, speculative); the last
+# two have no effect any more, the shapes that name them are still accepted
 SHADE_SHAPES = ([(t, c, r, 0, 0) for t in (64, 128, 256) for c in (32, 64) for r in (0, 64, 80)]
                 + [(t, c, 80, 4, 0) for t in (64, 128, 256) for c in (32, 64)]
                 + [(t, c, 80, 0, 1) for t in (64, 128, 256) for c in (32, 64)]
                 + [(t, c, 72, 0, s) for t in (64, 128) for c in (32, 64) for s in (0, 1)]
                 + [(t, 64, 64, 0, 1) for t in (64, 128, 256)])
-# second stage: the refill threshold (idle lanes out of 32), with and without
-# speculation, for the fastest block size / chunk / register budgets
+# second stage: the refill threshold (idle lanes out of 32) for the fastest
+# block size / chunk / register budgets
 REFILL_MINS = (4, 8, 12, 16, 20, 24)
 REFILL_TOP = 4
-# third stage: in-loop refill (speculative shapes): (threads, chunk, register
-# budget) x refill threshold x leaf batch
+# accepted with a leaf batch (speculative shapes), which has no effect any more
 INLOOP_SHAPES = [(64, 32, 64), (64, 64, 64), (128, 32, 64), (128, 64, 64), (256, 32, 64), (256, 64, 64),
                  (128, 64, 72), (256, 64, 72)]
-INLOOP_REFILL = (4, 8, 12, 16)
-INLOOP_LEAF_BATCH = (4, 8, 12, 16, 24)
 SHAPE_KEYS = ("threads", "chunk", "reg_cap", "top_levels", "speculative", "refill_min", "leaf_batch")
 
 
@@ -94,34 +90,22 @@ def tune_shadow(ctx, bvh, gbuf, params, reps=5):
                        "refill_min": refill, "leaf_batch": leaf_batch, "ms": statistics.median(ms)})
 
     for t, c, r, top, spec in SHADE_SHAPES:
-        timed(t, c, r, top, spec, 1)
-    bases = []
-    for s in sorted(trials, key=lambda x: x["ms"]):
-        b = (s["threads"], s["chunk"], s["reg_cap"], s["top_levels"])
-        if b not in bases:
-            bases.append(b)
-    for t, c, r, top in bases[:REFILL_TOP]:
-        for spec in (0, 1):
-            if (t, c, r, top, spec) not in SHADE_SHAPES:
-                continue
-            for refill in REFILL_MINS:
-                timed(t, c, r, top, spec, refill)
-    for t, c, r in INLOOP_SHAPES:
-        for refill in INLOOP_REFILL:
-            for lb in INLOOP_LEAF_BATCH:
-                timed(t, c, r, 0, 1, refill, lb)
+        if not top and not spec:
+            timed(t, c, r, 0, 0, 1)
+    for s in sorted(trials, key=lambda x: x["ms"])[:REFILL_TOP]:
+        for refill in REFILL_MINS:
+            timed(s["threads"], s["chunk"], s["reg_cap"], 0, 0, refill)
     best = min(trials, key=lambda x: x["ms"])
     ctx.set_trace_tuning(**{k: best.get(k, 0) for k in SHAPE_KEYS})
     return {k: best.get(k, 0) for k in SHAPE_KEYS}, trials
 
 
 CAMERA_REFILL = (1, 4, 8, 16)
-CAMERA_LEAF_BATCH = (4, 8, 16, 32)
 
 
 def tune_camera(ctx, bvh, cam, reps=5):
     """Time rq_render_gbuffer on one ray per thread and on the refilling
-    engine (refill threshold x leaf batch); keep the fastest.  Returns
+    engine (refill thresholds); keep the fastest.  Returns
     (schedule, trials)."""
     import statistics
     import torch
@@ -145,8 +129,7 @@ def tune_camera(ctx, bvh, cam, reps=5):
 
     timed(0, 1, 32)
     for refill in CAMERA_REFILL:
-        for lb in CAMERA_LEAF_BATCH:
-            timed(1, refill, lb)
+        timed(1, refill, 32)
     best = min(trials, key=lambda x: x["ms"])
     keys = ("engine", "refill_min", "leaf_batch")
     ctx.set_camera_tuning(**{k: best[k] for k in keys})

@@ -187,3 +187,41 @@ def test_empty_and_degenerate_rays(ctx):
     z = torch.empty((0, 8), dtype=torch.float32, device="cuda")
     rq.trace(ctx, b, z)
     b.destroy()
+
+
+def test_handle_with_room_for_many_nodes(ctx):
+    """A handle whose arrays could hold more nodes than a 32-bit stack entry can name is traced with 64-bit entries:
+    the same mesh in such a handle and in one of its own size gives the same rays."""
+    import rq.workloads as W
+    n = (1 << 23) + 1
+    big = torch.zeros((n, 3, 3), device="cuda")
+    big[:, 1, 0] = 0.01
+    big[:, 2, 1] = 0.01
+    big += torch.rand((n, 1, 3), device="cuda")
+    roomy = rq.Bvh.build(ctx, big.reshape(-1, 3))
+    del big
+    pos, idx = rq.scene_grid(96, 64, seed=21)
+    p, i = torch.from_numpy(pos).cuda(), torch.from_numpy(idx.view(np.int32)).cuda()
+    rq.Bvh.build(ctx, p, i, into=roomy)
+    roomy.info()
+    own = rq.Bvh.build(ctx, p, i)
+    rays = torch.from_numpy(rq.scene_rays_down(40000, seed=9)).cuda()
+    for flags in (0, rq.RQ_TRI_MT, rq.RQ_TRACE_ANY):
+        a, b = rq.trace(ctx, roomy, rays, flags, bary=True, stats=True), rq.trace(ctx, own, rays, flags, bary=True, stats=True)
+        assert all(torch.equal(x, y) for x, y in zip(a, b))
+        assert torch.equal(rq.trace(ctx, roomy, rays, flags)[0], b[0])
+    for flags in (0, rq.RQ_TRI_MT):
+        cam = W.shadow_camera(160, 90, flags=flags)
+        ga, gb = (rq.render_gbuffer(ctx, h, cam) for h in (roomy, own))
+        ctx.set_camera_tuning(1, 8)
+        gc = rq.render_gbuffer(ctx, roomy, cam)
+        ctx.set_camera_tuning()
+        assert torch.equal(ga, gb) and torch.equal(gc, gb)
+        refl = rq.reflect_params(cam, flags=flags)
+        assert torch.equal(rq.render_reflect(ctx, roomy, ga, refl), rq.render_reflect(ctx, own, gb, refl))
+    eye = np.hstack([np.eye(3), np.zeros((3, 1))]).astype(np.float32)
+    ta, tb = (rq.Tlas(ctx, [(eye, 3, 0xFF, h)]) for h in (roomy, own))
+    assert torch.equal(ta.trace(rays), tb.trace(rays))
+    ctx.sync_check()
+    for h in (ta, tb, roomy, own):
+        h.destroy()
