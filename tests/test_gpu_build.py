@@ -227,3 +227,38 @@ def test_bad_arguments_fail_loudly(ctx):
     assert e.value.status == rq.RQ_ERR_INVALID_ARG
     with pytest.raises(rq.RqError):
         rq.Bvh.build(ctx, p, None, max_leaf=17)
+
+
+@pytest.mark.parametrize("n,max_leaf,mode", [(1, 4, {}), (2, 1, {}), (512, 1, {}), (513, 1, {}), (1100, 4, {}),
+                                             (6000, 2, {}), (6000, 4, {"sah": True}), (6000, 1, {"median": True}),
+                                             (20000, 16, {"sah": True})])
+def test_refit_boxes(ctx, n, max_leaf, mode):
+    """Every box of a refitted tree is the union below it, at the edges of the refit's runs of 1,024 nodes."""
+    p = torch.from_numpy(soup(n, 300 + n)).cuda()
+    b = rq.Bvh.build(ctx, p, None, max_leaf=max_leaf, **mode)
+    before = b.download()
+    moved = (p * torch.tensor([1.5, -0.5, 2.0], device="cuda") + torch.sin(7.0 * p)).contiguous()
+    b.refit(moved)
+    ctx.sync_check()
+    n2, tr, n4, perm = b.download()
+    v = moved.cpu().numpy().reshape(-1, 3, 3)[perm]
+    assert np.array_equal(perm, before[3]) and np.array_equal(tr["v0"][:, :3], v[:, 0])
+    for f in ("left_child", "right_child"):
+        assert np.array_equal(n2[f], before[0][f])
+    lo, hi = np.empty((len(n2), 3), np.float32), np.empty((len(n2), 3), np.float32)
+    for k in range(len(n2) - 1, -1, -1):
+        l, r = int(n2["left_child"][k]), int(n2["right_child"][k])
+        if l < 0:
+            lo[k], hi[k] = v[~l:~l + r].min((0, 1)), v[~l:~l + r].max((0, 1))
+        else:
+            lo[k], hi[k] = np.minimum(lo[l], lo[r]), np.maximum(hi[l], hi[r])
+    assert np.array_equal(n2["aabb_min"], lo) and np.array_equal(n2["aabb_max"], hi)
+    used = n4["child_count"] != 0
+    for k, ax in enumerate("xyz"):
+        assert n4["min_" + ax][0][used[0]].min() == lo[0, k] and n4["max_" + ax][0][used[0]].max() == hi[0, k]
+        # a leaf slot's box is its triangles'
+        for node, slot in zip(*np.nonzero(n4["child_count"] > 0)):
+            f, c = ~int(n4["child_index"][node, slot]), int(n4["child_count"][node, slot])
+            assert n4["min_" + ax][node, slot] == v[f:f + c, :, k].min()
+            assert n4["max_" + ax][node, slot] == v[f:f + c, :, k].max()
+    b.destroy()
