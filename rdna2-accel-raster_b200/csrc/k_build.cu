@@ -1843,6 +1843,8 @@ int rq_launch_build(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t stride_
     const size_t need = rq_build_scratch_carve(nullptr, n, s, sah);
     int rc = rq_ensure_scratch(ctx, need, st);
     if (rc) return rc;
+    if (!sah && rq_small_build(n))
+        return rq_launch_build_small(ctx, bvh, pos, stride_bytes, idx, n, max_leaf, collapse, st);
     rq_build_scratch_carve(ctx->scratch, n, s, sah);
     const uint32_t sf = stride_bytes / 4;
     const int sms = ctx->num_sms;

@@ -143,6 +143,10 @@ size_t rq_build_scratch_carve(void* base, uint32_t n, BuildScratch& s, bool sah 
 // such subtree rebuilt by binned SAH (RQ_BUILD_SAH); 0: the plain LBVH.
 int rq_launch_build(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t stride_bytes, const uint32_t* idx,
                     uint32_t n, uint32_t max_leaf, bool collapse, cudaStream_t s, uint32_t sah_max = 0);
+// The plain LBVH of a small mesh, in one block (k_small.cu).
+bool rq_small_build(uint32_t n);
+int rq_launch_build_small(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t stride_bytes, const uint32_t* idx,
+                          uint32_t n, uint32_t max_leaf, bool collapse, cudaStream_t s);
 // The reference's median-split topology (k_median.cu).
 int rq_launch_build_median(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t stride_bytes, const uint32_t* idx,
                            uint32_t n, uint32_t max_leaf, bool collapse, cudaStream_t s);

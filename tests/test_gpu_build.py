@@ -64,6 +64,13 @@ def test_duplicate_codes_parity(ctx):
     assert_same_as_oracle(ctx, v, None)
 
 
+@pytest.mark.parametrize("n,max_leaf", [(1, 1), (2, 1), (31, 1), (128, 16), (129, 1), (1025, 2), (2048, 1), (2049, 1),
+                                        (4095, 3), (4096, 1), (4096, 4), (4096, 16), (4097, 1)])
+def test_small_build_parity(ctx, n, max_leaf):
+    """Both sides of the one-block build's limits: primitives, and nodes that fit its shared memory."""
+    assert_same_as_oracle(ctx, soup(n, 400 + n), None, max_leaf)
+
+
 @pytest.mark.parametrize("n", [1023, 1024, 1025, 606207, 606208, 606209, 610304, 610305])
 def test_sort_forms_parity(ctx, n):
     """The sort's tile edges in both its forms and on both sides of the length where one takes over from the other."""
