@@ -6,10 +6,12 @@
 // triangles, five dependent loads per node and level).  Here one block of
 // 1,024 threads takes the mesh through the same steps with everything but the
 // vertices and the outputs in shared memory: centroids and Morton codes, a
-// stable radix sort, Karras nodes, the pre-order positions, the boxes (of the
+// stable radix sort, the radix tree, the pre-order positions, the boxes (of the
 // emitted nodes only, at their pre-order places), the 4-wide collapse.
 // The rules are those of build_core.cuh, so the bytes equal k_build.cu's.
-// 4,096 triangles: <figures>.
+// 4,096 triangles 143 -> 75 us, 256 triangles 88 -> 28 us (the sort 15 and 8 us
+// of them, the vertex gathers 14 us, the collapse 10 us).  Above 4,096 the
+// shared memory is full, and one SM gathering the vertices would be the bound.
 // Trees of more than kNodes binary nodes (possible above kNodes / 2 triangles)
 // keep their node arrays in the context's scratch instead.
 #include <atomic>
@@ -57,10 +59,10 @@ struct Shared {
             uint16_t cnt[kWarps][256];
         } s;
     } a;
-    // Karras nodes, then the 4-wide nodes
+    // the radix tree by split, then the 4-wide nodes
     union {
         struct {
-            uint16_t kl[kSmallMax], kr[kSmallMax], klo[kSmallMax], khi[kSmallMax];  // bit 15 of kl, kr: a leaf
+            uint16_t kr[kSmallMax], klo[kSmallMax], khi[kSmallMax];                 // bit 15 of kr: a leaf
             uint16_t par_in[kSmallMax], par_lf[kSmallMax];                          // (parent << 1) | is_right
         } k;
         struct {
@@ -78,6 +80,8 @@ struct Shared {
     uint8_t leaf[kNodes];
     uint32_t seen[2 * kSmallMax / 32];  // arrivals of the refit
     uint32_t warp[kWarps];
+    uint32_t part[4][256];
+    uint8_t adj[kSmallMax];  // common prefix of a sorted key and the next
     float red[6][kWarps];
     uint32_t lvl[kLevels + 2];
     uint32_t tail;
@@ -111,10 +115,10 @@ __device__ __forceinline__ uint32_t scan1024(uint32_t v, uint32_t* s_warp, uint3
     return r;
 }
 
-__device__ __forceinline__ int delta(const uint32_t* k, int n, int i, int j) {
-    if (j < 0 || j > n - 1) return -1;
-    const uint32_t x = k[i] ^ k[j];
-    return x ? __clz(x) : 32 + __clz(uint32_t(i) ^ uint32_t(j));
+// Common prefix of sorted keys i and i + 1, by index where they are equal.
+__device__ __forceinline__ int delta(const uint32_t* k, uint32_t i) {
+    const uint32_t x = k[i] ^ k[i + 1];
+    return x ? __clz(x) : 32 + __clz(i ^ (i + 1));
 }
 
 // Left-child links above the node whose parent link is `par`.
@@ -143,6 +147,23 @@ struct SmallArgs {
     TreeArrays far;  // the node arrays of a tree that does not fit
     uint32_t* err;
 };
+
+// f(position, triangle, vertices) for this thread's sorted positions, two
+// triangles' loads in flight together.
+template <class F>
+__device__ __forceinline__ void each_triangle(const SmallArgs& A, const Shared& S, F f) {
+#pragma unroll
+    for (uint32_t r = 0; r < kItems; r += 2) {
+        const uint32_t k0 = r * kT + threadIdx.x, k1 = k0 + kT;
+        if (k0 >= A.n) break;
+        const uint32_t i0 = S.ids[k0], i1 = k1 < A.n ? S.ids[k1] : i0;
+        F3 a0, b0, c0, a1, b1, c1;
+        load_tri(A.pos, A.sf, A.idx, i0, a0, b0, c0);
+        load_tri(A.pos, A.sf, A.idx, i1, a1, b1, c1);
+        f(k0, i0, a0, b0, c0);
+        if (k1 < A.n) f(k1, i1, a1, b1, c1);
+    }
+}
 
 __global__ void __launch_bounds__(kT, 1) k_build_small(const __grid_constant__ SmallArgs A) {
     extern __shared__ __align__(16) char s_raw[];
@@ -240,19 +261,39 @@ __global__ void __launch_bounds__(kT, 1) k_build_small(const __grid_constant__ S
             __syncwarp();
         }
         __syncthreads();
-        // digit d's counts: 4 threads of 8 warps each
-        const uint32_t d = threadIdx.x >> 2, w0 = (threadIdx.x & 3u) * 8u;
+        // digit d's counts: 4 threads of 8 warps each, then the digits' bases
+        const uint32_t d = threadIdx.x & 255u, quarter = threadIdx.x >> 8;
         uint32_t c8[8], own = 0;
 #pragma unroll
         for (int w = 0; w < 8; ++w) {
-            c8[w] = S.a.s.cnt[w0 + w][d];
+            c8[w] = S.a.s.cnt[quarter * 8 + w][d];
             own += c8[w];
         }
-        uint32_t tot;
-        uint32_t run = scan1024(own, S.warp, &tot);
+        S.part[quarter][d] = own;
+        __syncthreads();
+        uint32_t run = 0, tot = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            const uint32_t v = S.part[q][d];
+            if (q < quarter) run += v;
+            tot += v;
+        }
+        {
+            // (every 8 warps hold the 256 digits in order)
+            uint32_t x = tot;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (int(lane) >= o) x += y;
+            }
+            if (lane == 31) S.warp[warp] = x;
+            __syncthreads();
+            run += x - tot;
+            for (uint32_t w = warp & ~7u; w < warp; ++w) run += S.warp[w];
+        }
 #pragma unroll
         for (int w = 0; w < 8; ++w) {
-            S.a.s.cnt[w0 + w][d] = uint16_t(run);
+            S.a.s.cnt[quarter * 8 + w][d] = uint16_t(run);
             run += c8[w];
         }
         __syncthreads();
@@ -269,36 +310,43 @@ __global__ void __launch_bounds__(kT, 1) k_build_small(const __grid_constant__ S
     }
     const uint32_t* keys = S.k.keys;
 
-    // ---- Karras nodes (karras_node of build_core.cuh)
-    for (int i = int(threadIdx.x); i < int(n) - 1; i += kT) {
-        const int d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
-        const int dmin = delta(keys, n, i, i - d);
-        int lmax = 2;
-        while (delta(keys, n, i, i + lmax * d) > dmin) lmax <<= 1;
-        int l = 0;
-        for (int t = lmax >> 1; t >= 1; t >>= 1)
-            if (delta(keys, n, i, i + (l + t) * d) > dmin) l += t;
-        const int j = i + l * d;
-        const int dnode = delta(keys, n, i, j);
-        int s = 0, t = l;
-        do {
-            t = (t + 1) >> 1;
-            if (delta(keys, n, i, i + (s + t) * d) > dnode) s += t;
-        } while (t > 1);
-        const int gamma = i + s * d + min(d, 0), lo = min(i, j), hi = max(i, j);
-        const bool lleaf = lo == gamma, rleaf = hi == gamma + 1;
-        S.b.k.kl[i] = uint16_t(lleaf ? 0x8000 | gamma : gamma);
-        S.b.k.kr[i] = uint16_t(rleaf ? 0x8000 | (gamma + 1) : gamma + 1);
-        S.b.k.klo[i] = uint16_t(lo);
-        S.b.k.khi[i] = uint16_t(hi);
-        (lleaf ? S.b.k.par_lf : S.b.k.par_in)[gamma] = uint16_t(i << 1);
-        (rleaf ? S.b.k.par_lf : S.b.k.par_in)[gamma + 1] = uint16_t((i << 1) | 1);
-        if (i == 0) S.b.k.par_in[0] = kNone16;
-    }
-    if (n == 1 && threadIdx.x == 0) S.b.k.par_lf[0] = kNone16;
+    // ---- the binary radix tree of the sorted codes (Karras's; built from the
+    // leaves up as Apetrei 2014: a range's parent splits it off at whichever
+    // end shares the longer prefix with its neighbour).  A node is named by
+    // its split: the last primitive of its left child.
+    for (uint32_t i = threadIdx.x; i < n; i += kT) S.adj[i] = i + 1 < n ? uint8_t(delta(keys, i) + 1) : uint8_t(0);
     __syncthreads();
+    // (a thread takes neighbours: all but its last climb end early)
+    for (uint32_t k = threadIdx.x * kItems; k < min(n, (threadIdx.x + 1) * kItems); ++k) {
+        uint32_t lo = k, hi = k, ref = 0x8000u | k;
+        for (;;) {
+            const uint32_t dl = lo ? S.adj[lo - 1] : 0u, dr = S.adj[hi];
+            uint16_t* mine = ref & 0x8000u ? S.b.k.par_lf + (ref & 0x7fffu) : S.b.k.par_in + ref;
+            if (!(dl | dr)) {  // the root
+                *mine = kNone16;
+                break;
+            }
+            const bool left = dr > dl;
+            const uint32_t p = left ? hi : lo - 1u;
+            *mine = uint16_t((p << 1) | (left ? 0u : 1u));
+            if (left) {
+                S.b.k.klo[p] = uint16_t(lo);
+            } else {
+                S.b.k.kr[p] = uint16_t(ref);
+                S.b.k.khi[p] = uint16_t(hi);
+            }
+            __threadfence_block();  // this range before the arrival
+            if (!((atomicOr(&S.seen[p >> 5], 1u << (p & 31u)) >> (p & 31u)) & 1u)) break;
+            __threadfence_block();
+            lo = S.b.k.klo[p];
+            hi = S.b.k.khi[p];
+            ref = p;
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < 2 * kSmallMax / 32; i += kT) S.seen[i] = 0u;
 
-    // ---- leaf order outputs; emission counts (leaf_step)
+    // ---- emission counts (leaf_step)
     uint32_t sum = 0;
     uint32_t cw[kItems];
 #pragma unroll
@@ -327,18 +375,7 @@ __global__ void __launch_bounds__(kT, 1) k_build_small(const __grid_constant__ S
             run += cw[r];
         }
     }
-    for (uint32_t k = threadIdx.x; k < n; k += kT) {
-        const uint32_t id = S.ids[k];
-        F3 p0, p1, p2;
-        load_tri(A.pos, A.sf, A.idx, id, p0, p1, p2);
-        float4* tp = reinterpret_cast<float4*>(A.tris + k);
-        tp[0] = make_float4(p0.x, p0.y, p0.z, 0.0f);
-        tp[1] = make_float4(p1.x, p1.y, p1.z, 0.0f);
-        tp[2] = make_float4(p2.x, p2.y, p2.z, 0.0f);
-        A.perm[k] = id;
-        A.skeys[k] = keys[k];
-    }
-    __syncthreads();  // (the keys' place becomes the areas')
+    __syncthreads();
 
     // ---- the emitted tree's links, by pre-order position (emit_step)
     const bool near = total <= kNodes;
@@ -377,38 +414,66 @@ __global__ void __launch_bounds__(kT, 1) k_build_small(const __grid_constant__ S
     }
     __syncthreads();
 
-    // ---- boxes: each leaf's, then upward (the second child to arrive goes on)
+    // ---- the leaf order's outputs; boxes: the primitives' by position, then
+    // each leaf's at its node (one SM gathers 4,096 triangles' vertices in 9 us,
+    // so they are read once here and once for the centroids)
     auto box = [&](int k, uint32_t v) -> float& { return T.box[k * T.cap + v]; };
-    for (uint32_t p = threadIdx.x; p < n; p += kT) {
+    each_triangle(A, S, [&](uint32_t k, uint32_t id, F3 a, F3 b, F3 c) {
+        float4* tp = reinterpret_cast<float4*>(A.tris + k);
+        tp[0] = make_float4(a.x, a.y, a.z, 0.0f);
+        tp[1] = make_float4(b.x, b.y, b.z, 0.0f);
+        tp[2] = make_float4(c.x, c.y, c.z, 0.0f);
+        A.perm[k] = id;
+        A.skeys[k] = keys[k];
+        box(0, k) = fminf(a.x, fminf(b.x, c.x));
+        box(1, k) = fminf(a.y, fminf(b.y, c.y));
+        box(2, k) = fminf(a.z, fminf(b.z, c.z));
+        box(3, k) = fmaxf(a.x, fmaxf(b.x, c.x));
+        box(4, k) = fmaxf(a.y, fmaxf(b.y, c.y));
+        box(5, k) = fmaxf(a.z, fmaxf(b.z, c.z));
+    });
+    __syncthreads();
+    {
+        float lf[kItems][6];
+#pragma unroll
+        for (uint32_t r = 0; r < kItems; ++r) {
+            const uint32_t p = r * kT + threadIdx.x;
+            if (p >= n || !S.c[p]) continue;
+            const uint32_t last = p + T.leaf[S.A[p] + S.c[p] - 1u];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) lf[r][k] = box(k, p);
+            for (uint32_t q = p + 1; q < last; ++q)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    lf[r][k] = fminf(lf[r][k], box(k, q));
+                    lf[r][3 + k] = fmaxf(lf[r][3 + k], box(3 + k, q));
+                }
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t r = 0; r < kItems; ++r) {
+            const uint32_t p = r * kT + threadIdx.x;
+            if (p >= n || !S.c[p]) continue;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) box(k, S.A[p] + S.c[p] - 1u) = lf[r][k];
+        }
+    }
+    __syncthreads();
+    // ---- and upward: the second child to arrive goes on
+    for (uint32_t p = threadIdx.x * kItems; p < min(n, (threadIdx.x + 1) * kItems); ++p) {
         if (!S.c[p]) continue;
         uint32_t v = S.A[p] + S.c[p] - 1u;
-        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-        for (uint32_t q = p; q < p + T.leaf[v]; ++q) {
-            const float4* tp = reinterpret_cast<const float4*>(A.tris + q);
-            const float4 a = tp[0], b = tp[1], c = tp[2];
-            lo[0] = fminf(lo[0], fminf(a.x, fminf(b.x, c.x)));
-            lo[1] = fminf(lo[1], fminf(a.y, fminf(b.y, c.y)));
-            lo[2] = fminf(lo[2], fminf(a.z, fminf(b.z, c.z)));
-            hi[0] = fmaxf(hi[0], fmaxf(a.x, fmaxf(b.x, c.x)));
-            hi[1] = fmaxf(hi[1], fmaxf(a.y, fmaxf(b.y, c.y)));
-            hi[2] = fmaxf(hi[2], fmaxf(a.z, fmaxf(b.z, c.z)));
-        }
         for (;;) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                box(k, v) = lo[k];
-                box(3 + k, v) = hi[k];
-            }
             const uint32_t up = T.par[v];
             if (up == kNone16) break;
-            __threadfence_block();  // this box before the arrival
+            __threadfence_block();  // v's box before the arrival
             if (!((atomicOr(&S.seen[up >> 5], 1u << (up & 31u)) >> (up & 31u)) & 1u)) break;
             __threadfence_block();
             const uint32_t l = up + 1u, r = T.link[up];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                lo[k] = fminf(box(k, l), box(k, r));
-                hi[k] = fmaxf(box(3 + k, l), box(3 + k, r));
+                box(k, up) = fminf(box(k, l), box(k, r));
+                box(3 + k, up) = fmaxf(box(3 + k, l), box(3 + k, r));
             }
             v = up;
         }
