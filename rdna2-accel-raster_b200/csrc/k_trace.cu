@@ -77,15 +77,27 @@ __global__ void __launch_bounds__(kT, kTraceBlocksPerSm) k_trace4(const rq_bvh4_
         nodes, tris, src, ctr, reinterpret_cast<Entry*>(s_stack) + threadIdx.x, rows, err, kTraceRefill);
 }
 
+// One ray per thread over a RADV image.  Open nodes as in trace_engine.cuh: one
+// stack entry per open box node, its id and the order of the children left; the
+// nearest child's id is at hand when its node has been opened, the others' are
+// read when their turn comes.  Few rays make a launch of one partial wave (the
+// fast builder's use: 16,384 rays on 4,096 triangles), where the time is that
+// of a warp's longest union of node chains; such a launch takes every second
+// or fourth lane only, so fewer rays share a warp.  24.0 us before (stack of
+// children, one loop for boxes and triangles), 21.6 us with full warps, 19.2
+// at 16 rays per warp, 18.3 at 8, 18.4 at 4.
+constexpr uint32_t kRadvSpread = 2;   // at least 8 rays per warp
+constexpr uint32_t kRadvFill = 768;   // threads per SM such a launch may take
+constexpr int kRadvRows = 32;  // a complete tree of 2^25 triangles is 14 deep
+
 template <bool ANY, bool MT, bool BARY>
 __global__ void __launch_bounds__(kT) k_trace_radv(const uint8_t* __restrict__ img, const rq_ray* __restrict__ rays,
-                                                   uint32_t n, rq_hit* __restrict__ hits, float* __restrict__ bary,
-                                                   uint32_t* err) {
-    constexpr int STACK = 64;
-    __shared__ uint32_t s_stack[STACK * kT];
-    const uint32_t i = blockIdx.x * kT + threadIdx.x;
-    if (i >= n) return;
-    uint32_t* stk = s_stack + threadIdx.x;
+                                                   uint32_t n, uint32_t spread, rq_hit* __restrict__ hits,
+                                                   float* __restrict__ bary, uint32_t* err) {
+    __shared__ uint2 s_stack[kRadvRows * kT];
+    const uint32_t g = blockIdx.x * kT + threadIdx.x, i = g >> spread;
+    if (i >= n || (g & ((1u << spread) - 1u))) return;
+    uint2* stk = s_stack + threadIdx.x;
     const uint8_t* base = img + RQ_RADV_BVH_OFFSET;
     const float4* rp = reinterpret_cast<const float4*>(rays + i);
     float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
@@ -104,13 +116,26 @@ __global__ void __launch_bounds__(kT) k_trace_radv(const uint8_t* __restrict__ i
     uint32_t hit_id = 0xffffffffu;
     bool found = false;
     float hu = 0.0f, hv = 0.0f;
-    stk[0] = RQ_RADV_NODE_BOX32;
-    int sp = 1;
-    while (sp > 0) {
-        const uint32_t id = stk[(--sp) * kT];
-        const uint32_t type = id & 7u;
-        const float4* np = reinterpret_cast<const float4*>(base + (size_t(id & ~7u) << 3));
-        if (type == RQ_RADV_NODE_BOX32) {
+    auto node = [&](uint32_t id) { return base + (size_t(id & ~7u) << 3); };
+    uint32_t cur = RQ_RADV_NODE_BOX32;  // the node to visit (the root)
+    uint32_t top = 0, left = 0;         // the deepest open node, its children left
+    int sp = 0;
+    auto next = [&]() {
+        if (left == 0u) {
+            if (sp == 0) return false;
+            const uint2 e = stk[(--sp) * kT];
+            top = e.x;
+            left = e.y;
+        }
+        cur = __ldg(reinterpret_cast<const uint32_t*>(node(top)) + (left & 3u));
+        left >>= 3;
+        return true;
+    };
+    for (;;) {
+        bool have = true;
+        // box nodes, then triangles: a warp's lanes stay in one of the two
+        while (have && (cur & 7u) == RQ_RADV_NODE_BOX32) {
+            const float4* np = reinterpret_cast<const float4*>(node(cur));
             const uint4 ch = __ldg(reinterpret_cast<const uint4*>(np));
             float cf[24];
 #pragma unroll
@@ -122,47 +147,54 @@ __global__ void __launch_bounds__(kT) k_trace_radv(const uint8_t* __restrict__ i
                 cf[4 * q + 3] = v.w;
             }
             const uint32_t ac[4] = {ch.x, ch.y, ch.z, ch.w};
-            uint32_t he[4];
-            float ht[4];
-            int nh = 0;
+            float tk[4];
+            uint32_t hitm = 0;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                if (ac[k] == RQ_RADV_INVALID_NODE) continue;
-                float tn;
+            for (int k = 0; k < 4; ++k)
                 if (rq::slab(sr, tmin, best, cf[6 * k], cf[6 * k + 3], cf[6 * k + 1], cf[6 * k + 4], cf[6 * k + 2],
-                             cf[6 * k + 5], tn)) {
-                    int pos = nh;
-                    if (!ANY) {
-                        while (pos > 0 && ht[pos - 1] > tn) {
-                            he[pos] = he[pos - 1];
-                            ht[pos] = ht[pos - 1];
-                            --pos;
-                        }
+                             cf[6 * k + 5], tk[k]) &&
+                    ac[k] != RQ_RADV_INVALID_NODE)
+                    hitm |= 1u << k;
+            if (hitm) {
+                const uint32_t seq = rq::child_sequence(hitm, tk, !ANY), first = seq & 3u;
+                if (seq >> 3) {
+                    if (left) {
+                        if (sp < kRadvRows)
+                            stk[(sp++) * kT] = make_uint2(top, left);
+                        else
+                            rq::set_err(err, RQ_DERR_STACK);
                     }
-                    he[pos] = ac[k];
-                    ht[pos] = tn;
-                    ++nh;
+                    top = cur;
+                    left = seq >> 3;
                 }
+                cur = first < 2u ? (first == 0u ? ac[0] : ac[1]) : (first == 2u ? ac[2] : ac[3]);
+            } else {
+                have = next();
             }
-            if (sp + nh > STACK) {
-                rq::set_err(err, RQ_DERR_STACK);
-                nh = STACK - sp;
+        }
+        bool done = false;
+        while (have && (cur & 7u) != RQ_RADV_NODE_BOX32) {
+            if ((cur & 7u) != RQ_RADV_NODE_TRIANGLE) {  // (no other type is built)
+                have = next();
+                continue;
             }
-            for (int j = nh - 1; j >= 0; --j) stk[(sp++) * kT] = he[j];
-        } else if (type == RQ_RADV_NODE_TRIANGLE) {
-            float4 a = rq::ldg4(np), b = rq::ldg4(np + 1), c = rq::ldg4(np + 2), dd = rq::ldg4(np + 3);
+            const float4* np = reinterpret_cast<const float4*>(node(cur));
+            float4 a = rq::ldg4(np), b = rq::ldg4(np + 1), c = rq::ldg4(np + 2);
             rq::F3 v0{a.x, a.y, a.z}, v1{a.w, b.x, b.y}, v2{b.z, b.w, c.x};
             float t, u, v;
             bool ok = MT ? rq::mt_test(o, d, v0, v1, v2, 1e-7f, t, u, v) : rq::wt_test(w, o, v0, v1, v2, t, u, v);
             if (ok && t >= tmin && t < best) {
                 best = t;
-                hit_id = __float_as_uint(dd.x);  // triangle_id at byte 48
+                hit_id = __float_as_uint(__ldg(reinterpret_cast<const float*>(np + 3)));  // triangle_id at byte 48
                 found = true;
                 hu = u;
                 hv = v;
+                done = ANY;
                 if (ANY) break;
             }
+            have = next();
         }
+        if (!have || done) break;
     }
     if (found) {
         reinterpret_cast<uint4*>(hits)[i] = make_uint4(1u, __float_as_uint(best), 0u, hit_id);
@@ -407,8 +439,11 @@ int rq_launch_trace_radv(rq_ctx* ctx, const void* img, uint64_t bytes, const rq_
     if (n == 0) return RQ_OK;
     const uint8_t* im = static_cast<const uint8_t*>(img);
     const bool any = flags & RQ_TRACE_ANY, mt = flags & RQ_TRI_MT, b = bary != nullptr;
-    dim3 g((n + kT - 1) / kT);
-#define RQ_RADV_CASE(A, M, B) k_trace_radv<A, M, B><<<g, kT, 0, st>>>(im, rays, n, hits, bary, ctx->d_err)
+    // fewer rays per warp while that still leaves one wave
+    uint32_t spread = 0;
+    while (spread < kRadvSpread && (uint64_t(n) << (spread + 1)) <= uint64_t(ctx->num_sms) * kRadvFill) ++spread;
+    dim3 g(uint32_t(((uint64_t(n) << spread) + kT - 1) / kT));
+#define RQ_RADV_CASE(A, M, B) k_trace_radv<A, M, B><<<g, kT, 0, st>>>(im, rays, n, spread, hits, bary, ctx->d_err)
     if (any && mt && b) RQ_RADV_CASE(true, true, true);
     else if (any && mt) RQ_RADV_CASE(true, true, false);
     else if (any && b) RQ_RADV_CASE(true, false, true);

@@ -198,3 +198,18 @@ def test_radv_builds_replayed_from_a_graph(ctx, n):
         ctx.sync_check()
         assert np.array_equal(img.cpu().numpy(), ref)
     del g
+
+
+@pytest.mark.parametrize("flags", [0, 1, 2, 3])
+def test_trace_radv_ray_counts(ctx, flags):
+    """Launches of 8, 16 and 32 rays per warp (chosen by the number of rays) give a ray the same result."""
+    pos, idx = rq.scene_grid(40, 30, seed=12)
+    tri9 = torch.from_numpy(np.ascontiguousarray(pos[idx].reshape(-1))).cuda()
+    img = rq.build_radv(ctx, tri9)
+    rays = torch.from_numpy(rq.scene_rays_down(120000, seed=13)).cuda()
+    want, wb = rq.trace_radv(ctx, img, rays, flags=flags, bary=True)
+    assert int(want[:, 0].sum()) > 10000
+    for n in (1, 31, 33, 1000, 28416, 28417, 56832, 56833, 113665):
+        got, gb = rq.trace_radv(ctx, img, rays[:n].contiguous(), flags=flags, bary=True)
+        assert torch.equal(got, want[:n]) and torch.equal(gb, wb[:n]), n
+    ctx.sync_check()
