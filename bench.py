@@ -641,7 +641,7 @@ def percentile(xs, q):
 def run_batched(ctx, dev, steps=200, plain_steps=20):
     """Batched builds: 512 deforming grids, triangle counts log-uniform in
     [64, 65536] (seed 2), 4,096 any-hit + 4,096 closest-hit rays per mesh.
-    Batched: one deformation launch, one persistent build launch and one
+    Batched: one deformation launch, the meshes' builds together and one
     traversal launch per step, captured in a CUDA graph and replayed.  Plain:
     the same work as per-mesh rq_build + rq_trace calls (captured too when the
     driver allows, else eager).  Per-step device time p50 / p99."""
@@ -748,7 +748,7 @@ def run_batched(ctx, dev, steps=200, plain_steps=20):
     equal = bool(torch.equal(hits_b, hits_p))
     out = {
         "workload": ("batched: 512 deforming grids, triangle counts log-uniform in [64, 65536] (seed 2), rebuilt "
-                     "every step; 4,096 any-hit + 4,096 closest-hit rays per mesh; one persistent build launch and "
+                     "every step; 4,096 any-hit + 4,096 closest-hit rays per mesh; the builds together and "
                      "one traversal launch per step in a CUDA graph"),
         "meshes": len(descs), "triangles_per_step": ntri, "rays_per_step": nrays,
         "batched": {"p50_ms": round(percentile(bms, 50), 4), "p99_ms": round(percentile(bms, 99), 4),

@@ -329,8 +329,9 @@ int rq_tlas_destroy(rq_tlas* tlas);
 
 /* Launch shapes of a batch's two kernels.  Results do not depend on them. */
 typedef struct rq_batch_tuning {
-    uint32_t build_threads;       /* threads per build block: 256, 512 or 1024 */
-    uint32_t build_blocks;        /* persistent build blocks (clamped to max_build_blocks) */
+    uint32_t build_threads;       /* 256, 512 or 1024: accepted, without effect (all meshes' builds
+                                     share their launches; so do the other build_* fields) */
+    uint32_t build_blocks;        /* > 0: accepted, without effect */
     uint32_t trace_threads;       /* threads per traversal block: 64, 128 or 256 */
     uint32_t trace_chunk;         /* ray ids a warp takes per refill: 32 or 64 */
     uint32_t trace_reg_cap;       /* registers per thread the launch bounds allow: 0 (none), 64, 72
@@ -338,27 +339,23 @@ typedef struct rq_batch_tuning {
     uint32_t trace_blocks_per_sm; /* 0: as many as fit */
     uint32_t stack_entries;       /* stack room per lane as 3 entries per level; 0 or anything below
                                      3 * (depth + 2) + 1 means that bound */
-    uint32_t max_build_blocks;    /* read only: build scratch slices the batch holds */
+    uint32_t max_build_blocks;    /* read only: what build_blocks defaults to at most */
     float build_ms;               /* rq_batch_autotune: measured time of this shape */
     float trace_ms;
     uint32_t trace_refill_min;    /* idle lanes of a traversal warp get new rays once at least this
                                      many of 32 are idle (or all are): 1..32; 0 means 1 */
-    uint32_t build_cluster;       /* build blocks per thread-block cluster: 0 or 1 (none), 2 or 4;
-                                     a cluster builds one large mesh with all its blocks */
-    uint32_t cluster_min_tris;    /* meshes of at least this many triangles are built by a whole
-                                     cluster (build_cluster > 1), the others by single blocks */
+    uint32_t build_cluster;       /* 0, 1, 2 or 4: accepted, without effect */
+    uint32_t cluster_min_tris;    /* accepted, without effect */
 } rq_batch_tuning;
 
 int rq_batch_tuning_get(const rq_batch* batch, rq_batch_tuning* out);
 /* Validates the shape (RQ_ERR_INVALID_ARG for one that has no kernel). */
 int rq_batch_tuning_set(rq_batch* batch, const rq_batch_tuning* t);
 /* Autotuner: builds the batch and traces the given rays once per candidate
- * shape — every build block size with 1..occupancy blocks per SM, clusters
- * of 2 and 4 blocks of 512 and 1,024 threads for the meshes of at least
- * 8,192 or 32,768 triangles, every
- * traversal block size x refill chunk x register cap, then refill thresholds
- * for the fastest traversal shape — timing each with CUDA events (median of
- * `reps`), and keeps the fastest build and traversal shape.
+ * shape — the build (once per accepted block size), every traversal block
+ * size x refill chunk x register cap, then refill thresholds for the fastest
+ * traversal shape — timing each with CUDA events (median of `reps`), and
+ * keeps the fastest traversal shape.
  * The stack depth is the smallest safe one for the batch's deepest tree.
  * Writes up to `cap` measured candidates to `trials` (build_ms set for build
  * shapes, trace_ms for traversal shapes) and their number to *count.

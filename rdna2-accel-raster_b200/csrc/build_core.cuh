@@ -1,8 +1,7 @@
 // build_core.cuh — the per-element steps of the LBVH build, shared by the
-// grid-wide kernels of k_build.cu / k_collapse.cu (one mesh per launch) and
-// the block-level pipeline of k_batch.cu (one mesh per thread block, many
-// meshes per launch).  Both call these functions, so a mesh built either way
-// has the same bytes.
+// kernels of k_build.cu / k_collapse.cu (one mesh per launch sequence) and of
+// k_forest.cu (all meshes of a batch per launch).  Both call these functions,
+// so a mesh built either way has the same bytes.
 //
 // Loads of data written earlier in the same launch use plain (coherent)
 // loads; only the caller's vertex and index buffers go through __ldg.
@@ -142,20 +141,85 @@ __device__ __forceinline__ void leaf_step(uint32_t k, const float* __restrict__ 
     c_out[k] = c;
 }
 
-// Atomic bottom-up refit from sorted leaf k: at each node the second child
-// to arrive computes the union box and continues upward.  The arrival count
-// is an acquire-release add: it publishes the box this thread wrote last
-// (the leaf box, then each union) and, for the second arrival, makes the
-// sibling's box visible.  CTA: all leaves of the tree are in this block.
-template <bool CTA = false>
-__device__ __forceinline__ void refit_walk(uint32_t k, const int32_t* kl, const int32_t* kr, const uint32_t* par_in,
-                                           const uint32_t* par_lf, float4* box_in, const float4* box_lf,
-                                           uint32_t* refit_flag, uint32_t* err) {
-    uint32_t par = par_lf[k];
+// The leaves [L0, L1) of a tree by one block of kLocal threads (at most kLocal
+// leaves), with every node whose range lies inside refitted in shared memory.
+// A node's index is one end of its leaf range, so such a node has its index
+// inside too: it takes its arrival count and box in shared memory (CTA-scope
+// ordering), and writes the box to global memory once for the emission.  A
+// walk that reaches a node whose range crosses the block's ends there: its
+// parent link goes to hand(par) (from at most one walk per leaf), to be
+// carried on by refit_walk_up.  Unions are exact, so the boxes equal
+// refit_walk's.  Call with the whole block.
+constexpr uint32_t kLocal = 256;  // 17 KB of shared memory per block (measured: faster than 512)
+struct LocalLeaves {
+    uint32_t flag[kLocal];
+    float4 lf[2 * kLocal];  // leaf boxes (lo, hi)
+    float4 in[2 * kLocal];  // boxes of the block's inner nodes
+    uint32_t top[kLocal];   // the handed-over walks
+    uint32_t ntop, base;
+};
+
+__device__ __forceinline__ void leaves_local(LocalLeaves& S, uint32_t L0, uint32_t L1, const float* __restrict__ pos,
+                                             uint32_t sf, const uint32_t* __restrict__ idx, uint32_t max_leaf,
+                                             const uint32_t* skeys, const uint32_t* sids, const int32_t* kl,
+                                             const int32_t* kr, const uint32_t* klo, const uint32_t* khi,
+                                             const uint32_t* par_in, const uint32_t* par_lf, float4* box_in,
+                                             float4* box_lf, uint32_t* c_out, rq_triangle* tris, uint32_t* perm,
+                                             uint32_t* keys_out, uint32_t* err) {
+    for (uint32_t i = threadIdx.x; i < kLocal; i += blockDim.x) S.flag[i] = 0u;
+    if (threadIdx.x == 0) S.ntop = 0u;
+    for (uint32_t k = L0 + threadIdx.x; k < L1; k += blockDim.x) {
+        leaf_step(k, pos, sf, idx, max_leaf, skeys, sids, klo, khi, par_in, par_lf, box_lf, c_out, tris, perm,
+                  keys_out);
+        S.lf[2 * (k - L0)] = box_lf[2 * size_t(k)];
+        S.lf[2 * (k - L0) + 1] = box_lf[2 * size_t(k) + 1];
+    }
+    __syncthreads();
+    for (uint32_t k = L0 + threadIdx.x; k < L1; k += blockDim.x) {
+        uint32_t par = par_lf[k];
+        uint32_t guard = 0;
+        while (par != kNoParent) {
+            const uint32_t p = par >> 1;
+            if (__ldg(klo + p) < L0 || __ldg(khi + p) >= L1) {
+                // from here up every range crosses a block's end
+                S.top[atomicAdd(&S.ntop, 1u)] = par;
+                break;
+            }
+            const int32_t a = kl[p], b = kr[p];
+            __threadfence_block();  // release this thread's shared-memory box
+            if (atomicAdd(&S.flag[p - L0], 1u) == 0u) break;
+            __threadfence_block();  // acquire the sibling's
+            const float4* pa = a < 0 ? S.lf + 2 * ((uint32_t(a) & 0x7fffffffu) - L0) : S.in + 2 * (a - L0);
+            const float4* pb = b < 0 ? S.lf + 2 * ((uint32_t(b) & 0x7fffffffu) - L0) : S.in + 2 * (b - L0);
+            const float4 alo = pa[0], ahi = pa[1], blo = pb[0], bhi = pb[1];
+            const float4 lo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f);
+            const float4 hi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
+            S.in[2 * (p - L0)] = lo;
+            S.in[2 * (p - L0) + 1] = hi;
+            __stcg(box_in + 2 * size_t(p), lo);
+            __stcg(box_in + 2 * size_t(p) + 1, hi);
+            par = par_in[p];
+            if (++guard > 128u) {
+                set_err(err, RQ_DERR_REFIT);
+                break;
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// Atomic bottom-up refit from the parent link `par` of a node whose box is
+// final: at each node the second child to arrive computes the union box and
+// continues upward.  The arrival count is an acquire-release add: it publishes
+// the box this thread wrote last and, for the second arrival, makes the
+// sibling's box visible.
+__device__ __forceinline__ void refit_walk_up(uint32_t par, const int32_t* kl, const int32_t* kr,
+                                              const uint32_t* par_in, float4* box_in, const float4* box_lf,
+                                              uint32_t* refit_flag, uint32_t* err) {
     uint32_t guard = 0;
     while (par != kNoParent) {
         const uint32_t p = par >> 1;
-        if (atom_add_acq_rel<CTA>(&refit_flag[p], 1u) == 0u) break;
+        if (atom_add_acq_rel(&refit_flag[p], 1u) == 0u) break;
         const int32_t a = kl[p], b = kr[p];
         const float4* ba = a < 0 ? box_lf + 2 * size_t(uint32_t(a) & 0x7fffffffu) : box_in + 2 * size_t(a);
         const float4* bb = b < 0 ? box_lf + 2 * size_t(uint32_t(b) & 0x7fffffffu) : box_in + 2 * size_t(b);
@@ -175,10 +239,11 @@ __device__ __forceinline__ void refit_walk(uint32_t k, const int32_t* kl, const 
 // Depth-first pre-order node writes for primitive position p: internal node
 // p (if emitted) sits at A[lo] + L, the emitted leaf starting at p (if any)
 // at A[p] + c[p] - 1.  Returns c[p].
+template <class Scan>
 __device__ __forceinline__ uint32_t emit_step(uint32_t p, uint32_t n, uint32_t max_leaf, const int32_t* kr,
                                               const uint32_t* klo, const uint32_t* khi, const uint32_t* par_in,
                                               const uint32_t* par_lf, const float4* box_in, const float4* box_lf,
-                                              const uint32_t* c, const uint32_t* A, rq_bvh2_node* out) {
+                                              const uint32_t* c, const Scan& A, rq_bvh2_node* out) {
     if (p + 1 < n && count_in(klo, khi, p) > max_leaf) {
         uint32_t L = 0, par = par_in[p];
         while (par != kNoParent && (par & 1u) == 0u) {

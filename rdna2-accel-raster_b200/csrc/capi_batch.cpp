@@ -1,5 +1,5 @@
 // capi_batch.cpp — C ABI of batches (include/rq.h): many meshes in one
-// allocation, built by one persistent launch and traced by one launch.
+// allocation, built together and traced by one launch.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -13,7 +13,9 @@
 namespace {
 
 constexpr uint32_t kMaxBatchMeshTris = 1u << 20;
-constexpr size_t kScratchBudget = size_t(4) << 30;  // per-block build scratch, all blocks
+// Build blocks per SM and thread count of a block: the shapes a batch still
+// accepts (they have no effect on the build, k_forest.cu).
+int build_blocks_per_sm(uint32_t threads) { return int(1024u / threads); }
 
 void free_batch(rq_batch* b) {
     if (b->mem) cudaFree(b->mem);
@@ -34,13 +36,13 @@ int sync_batch_counts(rq_batch* b) {
     return RQ_OK;
 }
 
-// Default shapes: 512-thread build blocks, as many as fit; 128-thread
-// traversal blocks, 32-id refills, no register cap.
+// Default shapes: the build shape is a formality; 128-thread traversal
+// blocks, 32-id refills, no register cap.
 rq_batch_tuning default_tuning(rq_ctx* ctx, uint32_t slices) {
     rq_batch_tuning t{};
     t.build_threads = 512;
     t.build_blocks = std::min<uint32_t>(slices, uint32_t(ctx->num_sms) *
-                                                    uint32_t(std::max(1, rq_batch_build_occupancy(512))));
+                                                    uint32_t(build_blocks_per_sm(512)));
     t.trace_threads = 128;
     t.trace_chunk = 32;
     t.trace_reg_cap = 0;
@@ -98,8 +100,6 @@ int rq_batch_tuning_set(rq_batch* batch, const rq_batch_tuning* t) {
         !rq_batch_trace_shape_ok(t->trace_threads, t->trace_chunk, t->trace_reg_cap) || t->stack_entries > 128 ||
         t->trace_refill_min > 32 || (t->build_cluster > 1 && t->build_cluster != 2 && t->build_cluster != 4))
         return rq_set_error(batch->ctx, RQ_ERR_INVALID_ARG, "no kernel for this batch shape");
-    if (t->build_cluster > 1 && rq_batch_build_clusters(t->build_threads, t->build_cluster) < 1)
-        return rq_set_error(batch->ctx, RQ_ERR_UNSUPPORTED, "no resident cluster of this build shape");
     const float bm = batch->tune.build_ms, tm = batch->tune.trace_ms;
     batch->tune = *t;
     batch->tune.build_ms = bm;
@@ -127,61 +127,26 @@ int rq_batch_autotune(rq_ctx* ctx, rq_batch* batch, const float* positions, uint
         if (*count < cap) trials[*count] = t;
         ++*count;
     };
-    // build shapes
+    // the build, timed once per accepted block size (its launches are the same)
     rq_batch_tuning best_b = start;
     float best_bms = -1.0f;
     for (uint32_t bt : {256u, 512u, 1024u}) {
-        const int occ = rq_batch_build_occupancy(bt);
-        for (int k = 1; k <= occ; ++k) {
-            rq_batch_tuning t = start;
-            t.build_threads = bt;
-            t.build_blocks = std::min<uint32_t>(batch->build_slices, uint32_t(ctx->num_sms) * uint32_t(k));
-            t.build_cluster = 1;
-            if (k > 1 && t.build_blocks == std::min<uint32_t>(batch->build_slices, uint32_t(ctx->num_sms) * (k - 1)))
-                continue;  // clamped to the same grid as k - 1
-            batch->tune = t;
-            float ms = 0.0f;
-            rc = time_median(ctx, st, reps,
-                             [&] { return rq_launch_batch_build(ctx, batch, positions, stride_bytes, indices, st); },
-                             &ms);
-            if (rc) break;
-            t.build_ms = ms;
-            t.trace_ms = 0.0f;
-            record(t);
-            if (best_bms < 0.0f || ms < best_bms) {
-                best_bms = ms;
-                best_b = t;
-            }
-        }
+        rq_batch_tuning t = start;
+        t.build_threads = bt;
+        t.build_blocks = std::min<uint32_t>(batch->build_slices,
+                                            uint32_t(ctx->num_sms) * uint32_t(build_blocks_per_sm(bt)));
+        t.build_cluster = 1;
+        batch->tune = t;
+        float ms = 0.0f;
+        rc = time_median(ctx, st, reps,
+                         [&] { return rq_launch_batch_build(ctx, batch, positions, stride_bytes, indices, st); }, &ms);
         if (rc) break;
-    }
-    // clusters for the largest meshes, at full occupancy
-    for (uint32_t bt : {512u, 1024u}) {
-        if (rc) break;
-        const int occ = rq_batch_build_occupancy(bt);
-        for (uint32_t cl : {2u, 4u}) {
-            if (rc || occ < 1 || rq_batch_build_clusters(bt, cl) < 1) continue;
-            for (uint32_t min_tris : {8192u, 32768u}) {
-                rq_batch_tuning t = start;
-                t.build_threads = bt;
-                t.build_blocks = std::min<uint32_t>(batch->build_slices, uint32_t(ctx->num_sms) * uint32_t(occ));
-                t.build_cluster = cl;
-                t.cluster_min_tris = min_tris;
-                if (t.build_blocks < cl) continue;
-                batch->tune = t;
-                float ms = 0.0f;
-                rc = time_median(ctx, st, reps,
-                                 [&] { return rq_launch_batch_build(ctx, batch, positions, stride_bytes, indices, st); },
-                                 &ms);
-                if (rc) break;
-                t.build_ms = ms;
-                t.trace_ms = 0.0f;
-                record(t);
-                if (ms < best_bms) {
-                    best_bms = ms;
-                    best_b = t;
-                }
-            }
+        t.build_ms = ms;
+        t.trace_ms = 0.0f;
+        record(t);
+        if (best_bms < 0.0f || ms < best_bms) {
+            best_bms = ms;
+            best_b = t;
         }
     }
     // traversal shapes (on the batch as built)
@@ -299,21 +264,26 @@ int rq_batch_create(rq_ctx* ctx, const rq_mesh_desc* meshes, uint32_t num_meshes
     c.take<int32_t>(4 * T);
     c.take<uint32_t>(4ull * num_meshes);
     c.take<rq_mesh_desc>(num_meshes);
-    c.take<uint32_t>(num_meshes);
-    c.take<uint32_t>(64);
+    b->build_slices = std::max(1u, std::min(uint32_t(ctx->num_sms) * uint32_t(build_blocks_per_sm(256)), num_meshes));
+    b->tune = default_tuning(ctx, b->build_slices);
+    rq_forest& f = b->forest;
+    try {
+        rq_forest_plan(b->meshes, f);
+    } catch (const std::bad_alloc&) {
+        delete b;
+        return rq_set_error(ctx, RQ_ERR_OOM, "batch tables");
+    }
+    auto tables = [&f](Carve& t) {
+        f.d_segs = t.take<rq_forest_seg>(f.segs.size());
+        f.d_blocks = t.take<uint2>(f.blocks.size());
+        f.d_tiles = t.take<rq_sort_tile>(f.tiles.size());
+        f.d_seg_tiles = t.take<uint32_t>(f.seg_tiles.size());
+        f.d_order = t.take<uint32_t>(f.order.size());
+    };
+    tables(c);
     b->mem_bytes = c.off + 256;
-    b->scratch_stride = rq_batch_block_scratch(maxt);
-    // scratch slices: enough for the most resident build blocks of any
-    // block size, within the scratch budget and the mesh count
-    int occ = 0;
-    for (uint32_t t : {256u, 512u, 1024u}) occ = std::max(occ, rq_batch_build_occupancy(t));
-    uint32_t blocks = uint32_t(ctx->num_sms) * uint32_t(std::max(1, occ));
-    blocks = std::min<uint32_t>(blocks, uint32_t(std::max<size_t>(1, kScratchBudget / b->scratch_stride)));
-    blocks = std::max(1u, std::min(blocks, num_meshes));
-    b->build_slices = blocks;
-    b->tune = default_tuning(ctx, blocks);
     if (cudaMalloc(&b->mem, b->mem_bytes) != cudaSuccess ||
-        cudaMalloc(&b->scratch, b->scratch_stride * b->build_slices) != cudaSuccess) {
+        cudaMalloc(&b->scratch, rq_forest_scratch_bytes(f)) != cudaSuccess) {
         cudaGetLastError();
         free_batch(b);
         delete b;
@@ -328,17 +298,23 @@ int rq_batch_create(rq_ctx* ctx, const rq_mesh_desc* meshes, uint32_t num_meshes
     b->map4 = d.take<int32_t>(4 * T);
     b->d_counts = d.take<uint32_t>(4ull * num_meshes);
     b->d_meshes = d.take<rq_mesh_desc>(num_meshes);
-    b->d_order = d.take<uint32_t>(num_meshes);
-    b->d_ctr = d.take<uint32_t>(64);
-    // build order: largest first, so the long builds start early
-    std::vector<uint32_t> order(num_meshes);
-    std::iota(order.begin(), order.end(), 0u);
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t c2) {
-        return meshes[a].num_triangles > meshes[c2].num_triangles;
-    });
+    tables(d);
     cudaError_t e = cudaMemcpy(b->d_meshes, meshes, sizeof(rq_mesh_desc) * num_meshes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(b->d_order, order.data(), sizeof(uint32_t) * num_meshes, cudaMemcpyHostToDevice);
+    auto upload = [&](void* to, const auto& from) {
+        if (e == cudaSuccess)
+            e = cudaMemcpy(to, from.data(), sizeof(from[0]) * from.size(), cudaMemcpyHostToDevice);
+    };
+    upload(f.d_segs, f.segs);
+    upload(f.d_blocks, f.blocks);
+    upload(f.d_tiles, f.tiles);
+    upload(f.d_seg_tiles, f.seg_tiles);
+    upload(f.d_order, f.order);
+    // (the groups are what a launch needs on the host)
+    f.segs = {};
+    f.blocks = {};
+    f.tiles = {};
+    f.seg_tiles = {};
+    f.order = {};
     if (e == cudaSuccess) e = cudaMemset(b->d_counts, 0, sizeof(uint32_t) * 4 * num_meshes);
     if (e != cudaSuccess) {
         free_batch(b);

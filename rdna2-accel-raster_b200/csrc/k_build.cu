@@ -81,118 +81,41 @@ __global__ void __launch_bounds__(kT) k_karras(const uint32_t* __restrict__ keys
     if (n == 1 && blockIdx.x == 0 && threadIdx.x == 0) par_lf[0] = rq::kNoParent;
 }
 
-// Leaves and refit with the bottom of the tree refitted in shared memory.
-// Block b owns the sorted leaves [kLocal*b, kLocal*(b+1)).  A Karras node's
-// index is one end of its leaf range, so a node whose range lies inside the
-// block's has its index inside it too: such nodes take their arrival count
-// and box in shared memory (CTA-scope ordering), and write the box to global
-// memory once for the emission.  A walk that reaches a node whose range
-// crosses a block boundary stops there and lists its parent link for
-// k_refit_top, which carries every such walk on with the device-scope
-// acquire-release count of refit_walk: a block is done once its own leaves
-// and local nodes are, instead of holding its slot while a walk climbs
-// through the tree's top.  Unions are exact, so the boxes equal refit_walk's.
-constexpr uint32_t kLocal = 256;  // 17 KB of shared memory per block (measured: faster than 512)
+// Leaves and refit with the bottom of the tree refitted in shared memory
+// (leaves_local): block b owns the sorted leaves [kLocal*b, kLocal*(b+1)).
+// Walks that leave the block are listed for k_refit_top, which carries them
+// on with device-scope arrivals: a block is done once its own leaves and local
+// nodes are, instead of holding its slot while a walk climbs through the
+// tree's top.
+using rq::kLocal;
 
 __global__ void __launch_bounds__(kT) k_leaves_local(
     const float* __restrict__ pos, uint32_t sf, const uint32_t* __restrict__ idx, uint32_t n, uint32_t max_leaf,
     const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ sids, const int32_t* __restrict__ kl,
     const int32_t* __restrict__ kr, const uint32_t* __restrict__ klo, const uint32_t* __restrict__ khi,
     const uint32_t* __restrict__ par_in, const uint32_t* __restrict__ par_lf, float4* box_in,
-    float4* __restrict__ box_lf, uint32_t* refit_flag, uint32_t* __restrict__ c_out, rq_triangle* __restrict__ tris,
+    float4* __restrict__ box_lf, uint32_t* __restrict__ c_out, rq_triangle* __restrict__ tris,
     uint32_t* __restrict__ perm, uint32_t* __restrict__ keys_out, uint32_t* __restrict__ top_list,
     uint32_t* top_cnt, uint32_t* err) {
-    __shared__ uint32_t s_flag[kLocal];
-    __shared__ float4 s_lf[2 * kLocal];  // leaf boxes (lo, hi) of the block's leaves
-    __shared__ float4 s_in[2 * kLocal];  // boxes of the block's inner nodes
-    __shared__ uint32_t s_top[kLocal];   // the block's handed-over walks (at most one per leaf)
-    __shared__ uint32_t s_ntop, s_base;
+    __shared__ rq::LocalLeaves S;
     const uint32_t L0 = blockIdx.x * kLocal;
-    const uint32_t L1 = min(L0 + kLocal, n);
-    for (uint32_t i = threadIdx.x; i < kLocal; i += kT) s_flag[i] = 0u;
-    if (threadIdx.x == 0) s_ntop = 0u;
-    for (uint32_t k = L0 + threadIdx.x; k < L1; k += kT) {
-        rq::leaf_step(k, pos, sf, idx, max_leaf, skeys, sids, klo, khi, par_in, par_lf, box_lf, c_out, tris, perm,
-                      keys_out);
-        s_lf[2 * (k - L0)] = box_lf[2 * size_t(k)];
-        s_lf[2 * (k - L0) + 1] = box_lf[2 * size_t(k) + 1];
-    }
-    __syncthreads();
-    for (uint32_t k = L0 + threadIdx.x; k < L1; k += kT) {
-        uint32_t par = par_lf[k];
-        uint32_t guard = 0;
-        while (par != rq::kNoParent) {
-            const uint32_t p = par >> 1;
-            const int32_t a = kl[p], b = kr[p];
-            float4 alo, ahi, blo, bhi;
-            if (__ldg(klo + p) >= L0 && __ldg(khi + p) < L1) {
-                __threadfence_block();  // release this thread's shared-memory box
-                if (atomicAdd(&s_flag[p - L0], 1u) == 0u) break;
-                __threadfence_block();  // acquire the sibling's
-                const float4* pa = a < 0 ? s_lf + 2 * ((uint32_t(a) & 0x7fffffffu) - L0) : s_in + 2 * (a - L0);
-                const float4* pb = b < 0 ? s_lf + 2 * ((uint32_t(b) & 0x7fffffffu) - L0) : s_in + 2 * (b - L0);
-                alo = pa[0];
-                ahi = pa[1];
-                blo = pb[0];
-                bhi = pb[1];
-                const float4 lo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f);
-                const float4 hi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
-                s_in[2 * (p - L0)] = lo;
-                s_in[2 * (p - L0) + 1] = hi;
-                __stcg(box_in + 2 * size_t(p), lo);
-                __stcg(box_in + 2 * size_t(p) + 1, hi);
-            } else {
-                // from here up every range crosses a block boundary: k_refit_top
-                s_top[atomicAdd(&s_ntop, 1u)] = par;
-                break;
-            }
-            par = par_in[p];
-            if (++guard > 128u) {
-                rq::set_err(err, RQ_DERR_REFIT);
-                break;
-            }
-        }
-    }
+    rq::leaves_local(S, L0, min(L0 + kLocal, n), pos, sf, idx, max_leaf, skeys, sids, kl, kr, klo, khi, par_in, par_lf,
+                     box_in, box_lf, c_out, tris, perm, keys_out, err);
     // the block's hand-offs, with one device atomic
+    if (threadIdx.x == 0 && S.ntop) S.base = atomicAdd(top_cnt, S.ntop);
     __syncthreads();
-    const uint32_t nt = s_ntop;
-    if (threadIdx.x == 0 && nt) s_base = atomicAdd(top_cnt, nt);
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < nt; i += kT) top_list[s_base + i] = s_top[i];
+    for (uint32_t i = threadIdx.x; i < S.ntop; i += kT) top_list[S.base + i] = S.top[i];
 }
 
-// The walks k_leaves_local handed over: each starts at the parent link of a
-// node whose parent's range crosses a block boundary (that node's box is in
-// box_in or box_lf); at each node the second child to arrive forms the union
-// and carries on upward, as refit_walk.
+// The walks k_leaves_local handed over.
 __global__ void __launch_bounds__(kT) k_refit_top(const int32_t* __restrict__ kl, const int32_t* __restrict__ kr,
                                                   const uint32_t* __restrict__ par_in, float4* box_in,
                                                   const float4* box_lf, uint32_t* refit_flag,
                                                   const uint32_t* __restrict__ top_list, const uint32_t* top_cnt,
                                                   uint32_t* err) {
     const uint32_t m = *top_cnt;
-    for (uint32_t j = blockIdx.x * kT + threadIdx.x; j < m; j += gridDim.x * kT) {
-        uint32_t par = top_list[j];
-        uint32_t guard = 0;
-        while (par != rq::kNoParent) {
-            const uint32_t p = par >> 1;
-            if (rq::atom_add_acq_rel(&refit_flag[p], 1u) == 0u) break;
-            const int32_t a = kl[p], b = kr[p];
-            const float4* ba = a < 0 ? box_lf + 2 * size_t(uint32_t(a) & 0x7fffffffu) : box_in + 2 * size_t(a);
-            const float4* bb = b < 0 ? box_lf + 2 * size_t(uint32_t(b) & 0x7fffffffu) : box_in + 2 * size_t(b);
-            const float4 alo = rq::ld_cg4(ba), ahi = rq::ld_cg4(ba + 1);
-            const float4 blo = rq::ld_cg4(bb), bhi = rq::ld_cg4(bb + 1);
-            __stcg(box_in + 2 * size_t(p),
-                   make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f));
-            __stcg(box_in + 2 * size_t(p) + 1,
-                   make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f));
-            par = par_in[p];
-            if (++guard > 128u) {
-                rq::set_err(err, RQ_DERR_REFIT);
-                break;
-            }
-        }
-    }
+    for (uint32_t j = blockIdx.x * kT + threadIdx.x; j < m; j += gridDim.x * kT)
+        rq::refit_walk_up(top_list[j], kl, kr, par_in, box_in, box_lf, refit_flag, err);
 }
 
 __global__ void __launch_bounds__(kT) k_emit2(uint32_t n, uint32_t max_leaf, const int32_t* __restrict__ kr,
@@ -359,23 +282,7 @@ __device__ void sah_refit_up(uint32_t rn, float4 rlo, float4 rhi, const int32_t*
     float4* dst = rleaf ? box_lf + 2 * size_t(ri) : box_in + 2 * size_t(ri);
     __stcg(dst, rlo);
     __stcg(dst + 1, rhi);
-    uint32_t par = rleaf ? par_lf[ri] : par_in[ri];
-    for (uint32_t guard = 0; par != rq::kNoParent; ++guard) {
-        const uint32_t p = par >> 1;
-        if (rq::atom_add_acq_rel(&refit_flag[p], 1u) == 0u) break;
-        const int32_t a = kl[p], b = kr[p];
-        const float4* ba = a < 0 ? box_lf + 2 * size_t(uint32_t(a) & 0x7fffffffu) : box_in + 2 * size_t(a);
-        const float4* bb = b < 0 ? box_lf + 2 * size_t(uint32_t(b) & 0x7fffffffu) : box_in + 2 * size_t(b);
-        const float4 alo = rq::ld_cg4(ba), ahi = rq::ld_cg4(ba + 1), blo = rq::ld_cg4(bb), bhi = rq::ld_cg4(bb + 1);
-        __stcg(box_in + 2 * size_t(p), make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f));
-        __stcg(box_in + 2 * size_t(p) + 1,
-               make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f));
-        par = par_in[p];
-        if (guard > 128u) {
-            rq::set_err(err, RQ_DERR_REFIT);
-            break;
-        }
-    }
+    rq::refit_walk_up(rleaf ? par_lf[ri] : par_in[ri], kl, kr, par_in, box_in, box_lf, refit_flag, err);
 }
 
 struct SahArgs {
@@ -1875,7 +1782,7 @@ int rq_launch_build(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t stride_
     uint32_t* top_cnt = s.tile_ctr + 12;
     k_leaves_local<<<(n + kLocal - 1) / kLocal, kT, 0, st>>>(pos, sf, idx, n, max_leaf, skeys, sids, s.kl, s.kr,
                                                              s.klo, s.khi, s.par_in, s.par_lf, s.box_in, s.box_lf,
-                                                             s.refit_flag, s.c, bvh->tris, bvh->perm, bvh->skeys,
+                                                             s.c, bvh->tris, bvh->perm, bvh->skeys,
                                                              top_list, top_cnt, ctx->d_err);
     k_refit_top<<<uint32_t(sms) * 4u, kT, 0, st>>>(s.kl, s.kr, s.par_in, s.box_in, s.box_lf, s.refit_flag, top_list,
                                                    top_cnt, ctx->d_err);

@@ -31,6 +31,7 @@ constexpr int kTile = kThreads * kItems;
 constexpr uint32_t kLookBackMax = kTile * 148 * 4;  // keys sorted by look-back: one wave of tiles
 constexpr int kBigItems = 16;                   // keys per thread of a counted tile
 constexpr uint32_t kBigTile = kThreads * kBigItems;
+static_assert(kBigTile == RQ_SORT_TILE, "a counted tile");
 constexpr int kRadix = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr uint32_t kFlagAgg = 1u << 30;
@@ -260,14 +261,32 @@ __global__ void __launch_bounds__(kThreads, 4) k_onesweep(const uint32_t* __rest
 // A look-back over 8.3M keys (1,807 tiles of 4,608) took 130 us per pass: 239
 // warp instructions per 32 keys, a third of them walking status windows, and
 // a chain of L2 round trips.
+// The keys [base, base + count) of tile blockIdx.x: the next kBigTile of one
+// sort of n keys, or tiles[blockIdx.x] of a sort of segments.
+__device__ __forceinline__ void tile_range(const rq_sort_tile* tiles, uint32_t n, uint32_t& base, uint32_t& count,
+                                           uint32_t& seg) {
+    if (tiles) {
+        const rq_sort_tile t = tiles[blockIdx.x];
+        base = t.first;
+        count = t.count;
+        seg = t.seg_first;
+    } else {
+        base = blockIdx.x * kBigTile;
+        count = min(kBigTile, n - base);
+        seg = 0;
+    }
+}
+
 __global__ void __launch_bounds__(kThreads) k_tile_count(const uint32_t* __restrict__ keys, uint32_t n, uint32_t shift,
+                                                         const rq_sort_tile* __restrict__ tiles,
                                                          uint32_t* __restrict__ counts) {
     __shared__ uint32_t sh[4][kRadix];
     uint32_t* mine = sh[(threadIdx.x >> 6) & 3];
     for (int i = threadIdx.x; i < 4 * kRadix; i += kThreads) (&sh[0][0])[i] = 0;
     __syncthreads();
-    const uint32_t base = blockIdx.x * kBigTile;
-    if (base + kBigTile <= n) {
+    uint32_t base, count, seg;
+    tile_range(tiles, n, base, count, seg);
+    if (count == kBigTile && base % 4 == 0) {
         const uint4* k4 = reinterpret_cast<const uint4*>(keys + base);
 #pragma unroll
         for (int j = 0; j < kBigItems / 4; ++j) {
@@ -278,11 +297,28 @@ __global__ void __launch_bounds__(kThreads) k_tile_count(const uint32_t* __restr
             atomicAdd(mine + ((k.w >> shift) & 255u), 1u);
         }
     } else {
-        for (uint32_t i = base + threadIdx.x; i < n; i += kThreads) atomicAdd(mine + ((keys[i] >> shift) & 255u), 1u);
+        for (uint32_t i = threadIdx.x; i < count; i += kThreads) atomicAdd(mine + ((keys[base + i] >> shift) & 255u), 1u);
     }
     __syncthreads();
     const uint32_t d = threadIdx.x;
     counts[size_t(blockIdx.x) * kRadix + d] = sh[0][d] + sh[1][d] + sh[2][d] + sh[3][d];
+}
+
+// A segment's tiles by one block (thread = digit): each digit's first place in
+// the segment plus its count in the tiles before, in place of the counts.
+__global__ void __launch_bounds__(kThreads) k_segment_prefix(uint32_t* counts, const uint32_t* __restrict__ seg_tiles) {
+    __shared__ uint32_t s_warp[kWarps];
+    const uint32_t t0 = seg_tiles[blockIdx.x], t1 = seg_tiles[blockIdx.x + 1], d = threadIdx.x;
+    uint32_t total = 0;
+#pragma unroll 8
+    for (uint32_t t = t0; t < t1; ++t) total += counts[size_t(t) * kRadix + d];
+    uint32_t acc = block_exclusive_scan(total, s_warp, nullptr);
+#pragma unroll 8
+    for (uint32_t t = t0; t < t1; ++t) {
+        const uint32_t c = counts[size_t(t) * kRadix + d];
+        counts[size_t(t) * kRadix + d] = acc;
+        acc += c;
+    }
 }
 
 // Exclusive prefix of every digit's counts over the tiles, in place, and the
@@ -342,12 +378,13 @@ __global__ void __launch_bounds__(kPrefixThreads) k_tile_prefix(uint32_t* counts
 template <bool FULL>
 __device__ __forceinline__ void scatter_tile(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                                              uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
-                                             uint32_t n, uint32_t shift, const uint32_t* __restrict__ prefix,
-                                             const uint32_t* __restrict__ totals, uint32_t (*s_cnt)[kRadix],
-                                             uint32_t* s_keys, uint32_t* s_vals, uint32_t* s_glob, uint32_t* s_warp) {
+                                             uint32_t base, uint32_t n, uint32_t seg, uint32_t shift,
+                                             const uint32_t* __restrict__ prefix, const uint32_t* __restrict__ totals,
+                                             uint32_t (*s_cnt)[kRadix], uint32_t* s_keys, uint32_t* s_vals,
+                                             uint32_t* s_glob, uint32_t* s_warp) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
-    const uint32_t base = blockIdx.x * kBigTile, first = base + warp * (32 * kBigItems) + lane;
+    const uint32_t first = base + warp * (32 * kBigItems) + lane;  // (n: the tile's end)
     uint32_t key[kBigItems], val[kBigItems], rank[kBigItems];
 #pragma unroll
     for (int j = 0; j < kBigItems; ++j) {
@@ -356,13 +393,14 @@ __device__ __forceinline__ void scatter_tile(const uint32_t* __restrict__ keys_i
         val[j] = valid ? vals_in[first + j * 32] : 0u;
     }
     const uint32_t d = threadIdx.x;
-    const uint32_t tot = totals[d], pre = prefix[d];
+    const uint32_t tot = totals ? totals[d] : 0u, pre = prefix[d];
     uint32_t* cnt = s_cnt[warp];
 #pragma unroll
     for (int j = 0; j < kBigItems; ++j) {
         const bool valid = FULL || first + j * 32 < n;
         const uint32_t act = FULL ? 0xffffffffu : __ballot_sync(0xffffffffu, valid);
         rank[j] = 0;
+        if (!FULL && !act) break;
         if (valid) {
             const uint32_t dj = (key[j] >> shift) & 255u;
             const uint32_t peers = digit_peers(act, dj);
@@ -374,8 +412,10 @@ __device__ __forceinline__ void scatter_tile(const uint32_t* __restrict__ keys_i
         }
         __syncwarp();
     }
+    __syncthreads();  // every warp's counts
     // the digits' first places over all keys, and in the tile
-    const uint32_t digit_base = block_exclusive_scan(tot, s_warp, nullptr);
+    // (a segment's prefix has its digits' places in it)
+    const uint32_t digit_base = totals ? block_exclusive_scan(tot, s_warp, nullptr) : seg;
     uint32_t mine = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) mine += s_cnt[w][d];
@@ -409,7 +449,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_tile_scatter(const uint32_t* __
                                                               const uint32_t* __restrict__ vals_in,
                                                               uint32_t* __restrict__ keys_out,
                                                               uint32_t* __restrict__ vals_out, uint32_t n,
-                                                              uint32_t shift, const uint32_t* __restrict__ prefix,
+                                                              uint32_t shift, const rq_sort_tile* __restrict__ tiles,
+                                                              const uint32_t* __restrict__ prefix,
                                                               const uint32_t* __restrict__ totals) {
     __shared__ uint32_t s_cnt[kWarps][kRadix];
     __shared__ uint32_t s_keys[kBigTile];
@@ -419,12 +460,14 @@ __global__ void __launch_bounds__(kThreads, 4) k_tile_scatter(const uint32_t* __
     for (int i = threadIdx.x; i < kWarps * kRadix; i += kThreads) (&s_cnt[0][0])[i] = 0;
     __syncthreads();
     prefix += size_t(blockIdx.x) * kRadix;
-    if ((blockIdx.x + 1u) * kBigTile <= n)
-        scatter_tile<true>(keys_in, vals_in, keys_out, vals_out, n, shift, prefix, totals, s_cnt, s_keys, s_vals,
-                           s_glob, s_warp);
+    uint32_t base, count, seg;
+    tile_range(tiles, n, base, count, seg);
+    if (count == kBigTile)
+        scatter_tile<true>(keys_in, vals_in, keys_out, vals_out, base, base + count, seg, shift, prefix, totals, s_cnt,
+                           s_keys, s_vals, s_glob, s_warp);
     else
-        scatter_tile<false>(keys_in, vals_in, keys_out, vals_out, n, shift, prefix, totals, s_cnt, s_keys, s_vals,
-                            s_glob, s_warp);
+        scatter_tile<false>(keys_in, vals_in, keys_out, vals_out, base, base + count, seg, shift, prefix, totals, s_cnt,
+                            s_keys, s_vals, s_glob, s_warp);
 }
 
 // ------------------------------------------------------------------ scan
@@ -521,10 +564,10 @@ int rq_launch_sort(rq_ctx* ctx, const SortIO& io, uint32_t n, uint32_t bits, uin
             for (uint32_t p = 0; p < passes; ++p) {
                 const int a = int(p & 1), b = 1 - a;
                 const size_t o = y * io.stride;
-                k_tile_count<<<tiles, kThreads, 0, st>>>(io.keys[a] + o, n, 8 * p, counts);
+                k_tile_count<<<tiles, kThreads, 0, st>>>(io.keys[a] + o, n, 8 * p, nullptr, counts);
                 k_tile_prefix<<<kRadix / kPrefixDigits, kPrefixThreads, 0, st>>>(counts, tiles, totals);
                 k_tile_scatter<<<tiles, kThreads, 0, st>>>(io.keys[a] + o, io.vals[a] + o, io.keys[b] + o,
-                                                           io.vals[b] + o, n, 8 * p, counts, totals);
+                                                           io.vals[b] + o, n, 8 * p, nullptr, counts, totals);
             }
         return rq_cuda_status(ctx, cudaGetLastError(), "radix sort launch");
     }
@@ -549,6 +592,20 @@ int rq_launch_sort(rq_ctx* ctx, const SortIO& io, uint32_t n, uint32_t bits, uin
                                                             ticket + p * batch, ctx->d_err);
     }
     return rq_cuda_status(ctx, cudaGetLastError(), "radix sort launch");
+}
+
+int rq_launch_sort_tiles(rq_ctx* ctx, const SortIO& io, const rq_sort_tile* tiles, uint32_t ntiles,
+                         const uint32_t* seg_tiles, uint32_t nsegs, uint32_t bits, cudaStream_t st, int* result_buf) {
+    const uint32_t passes = (bits + 7) / 8;
+    for (uint32_t p = 0; p < passes; ++p) {
+        const int a = int(p & 1), b = 1 - a;
+        k_tile_count<<<ntiles, kThreads, 0, st>>>(io.keys[a], 0, 8 * p, tiles, io.words);
+        k_segment_prefix<<<nsegs, kThreads, 0, st>>>(io.words, seg_tiles);
+        k_tile_scatter<<<ntiles, kThreads, 0, st>>>(io.keys[a], io.vals[a], io.keys[b], io.vals[b], 0, 8 * p, tiles,
+                                                    io.words, nullptr);
+    }
+    *result_buf = int(passes & 1);
+    return rq_cuda_status(ctx, cudaGetLastError(), "segment sort launch");
 }
 
 void rq_launch_scan(rq_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* status,

@@ -1,5 +1,5 @@
 // rq_batch.h — host-side state of a batch handle (many meshes, one
-// allocation) and the launchers of k_batch.cu.
+// allocation) and the launchers of k_batch.cu and k_forest.cu.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -8,6 +8,35 @@
 #include <vector>
 
 #include "rq_internal.h"
+
+// One mesh in a group of meshes built together: where its elements lie in the
+// scratch arrays, its descriptor's offsets, its triangles, its number.
+struct rq_forest_seg {
+    uint32_t first, tri, vert, n, mesh;
+};
+struct rq_forest_group {
+    uint32_t seg0 = 0, segs = 0;      // segments (meshes)
+    uint32_t block0 = 0, blocks = 0;  // element blocks
+    uint32_t tile0 = 0, tiles = 0;    // sort tiles
+    uint32_t begin0 = 0;              // first tile of each segment, and the end: segs + 1 entries
+    uint32_t tris = 0;
+};
+// The tables that deal a batch's builds out to blocks (k_forest.cu).
+struct rq_forest {
+    std::vector<rq_forest_group> groups;
+    std::vector<rq_forest_seg> segs;
+    std::vector<uint2> blocks;        // (segment in the group, first element)
+    std::vector<rq_sort_tile> tiles;
+    std::vector<uint32_t> seg_tiles;
+    std::vector<uint32_t> order;      // a group's segments, largest first
+    rq_forest_seg* d_segs = nullptr;
+    uint2* d_blocks = nullptr;
+    rq_sort_tile* d_tiles = nullptr;
+    uint32_t* d_seg_tiles = nullptr;
+    uint32_t* d_order = nullptr;
+};
+void rq_forest_plan(const std::vector<rq_mesh_desc>& meshes, rq_forest& f);
+size_t rq_forest_scratch_bytes(const rq_forest& f);
 
 struct rq_batch {
     rq_ctx* ctx = nullptr;
@@ -29,12 +58,9 @@ struct rq_batch {
     int32_t* map4 = nullptr;
     uint32_t* d_counts = nullptr;  // 4 per mesh: nodes2, nodes4, depth4, max leaf
     rq_mesh_desc* d_meshes = nullptr;
-    uint32_t* d_order = nullptr;   // build order: largest mesh first
-    uint32_t* d_ctr = nullptr;     // build queue counters: [0] clusters, [1] single blocks
-    // per-block build scratch, sized for the largest mesh
-    void* scratch = nullptr;
-    size_t scratch_stride = 0;
-    uint32_t build_slices = 0;     // scratch slices: the most build blocks a launch may use
+    rq_forest forest;              // how the builds are dealt out
+    void* scratch = nullptr;       // build scratch, sized for the largest group
+    uint32_t build_slices = 0;     // reported as max_build_blocks
     rq_batch_tuning tune{};        // launch shapes
     std::vector<uint32_t> h_counts;
     bool counts_valid = false;
@@ -43,11 +69,6 @@ struct rq_batch {
     cudaStream_t last_stream = nullptr;
 };
 
-size_t rq_batch_block_scratch(uint32_t max_tris);
-// Resident build blocks per SM for a build block size (0 if none).
-int rq_batch_build_occupancy(uint32_t threads);
-// Resident clusters of `cluster` (2 or 4) build blocks of `threads` (0 if none).
-int rq_batch_build_clusters(uint32_t threads, uint32_t cluster);
 // Whether a traversal kernel exists for this shape.
 bool rq_batch_trace_shape_ok(uint32_t threads, uint32_t chunk, uint32_t regs);
 int rq_launch_batch_build(rq_ctx* ctx, rq_batch* b, const float* pos, uint32_t stride_bytes, const uint32_t* idx,

@@ -168,6 +168,17 @@ size_t rq_sort_words(uint32_t n, uint32_t batch);
 // end in buffer index returned (0 or 1).
 int rq_launch_sort(rq_ctx* ctx, const SortIO& io, uint32_t n, uint32_t bits, uint32_t batch, cudaStream_t st,
                    int* result_buf);
+// One tile (at most RQ_SORT_TILE keys) of a sort of many segments: keys
+// [first, first + count) of the segment that starts at key seg_first.
+#define RQ_SORT_TILE 4096u
+struct rq_sort_tile {
+    uint32_t first, count, seg_first, pad;
+};
+// Stable LSD radix sort of every segment by itself: tiles[0, ntiles), segment
+// s's from seg_tiles[s] to seg_tiles[s + 1] (device arrays); io.words holds 256
+// words per tile.
+int rq_launch_sort_tiles(rq_ctx* ctx, const SortIO& io, const rq_sort_tile* tiles, uint32_t ntiles,
+                         const uint32_t* seg_tiles, uint32_t nsegs, uint32_t bits, cudaStream_t st, int* result_buf);
 uint32_t rq_scan_tiles(uint32_t n);
 // Exclusive scan of in[0..n).
 void rq_launch_scan(rq_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* status,

@@ -176,3 +176,34 @@ def test_autotune_keeps_a_measured_shape(ctx):
     got = b.trace(rays_t, mesh_t, flags_t)[0].cpu().numpy()
     assert got.tobytes() == want.tobytes()
     b.destroy()
+
+
+def test_batch_mesh_sizes_and_places(ctx):
+    """Meshes at the edges of the build's blocks and sort tiles, listed in any order, with gaps between their triangle
+    ranges and vertices that are not in the meshes' order."""
+    sizes = [1, 255, 256, 257, 513, 4095, 4096, 4097, 8193, 2, 70001]
+    rng = np.random.default_rng(3)
+    pos_l, idx_l, descs, v, t = [], [], [], 0, 5
+    idx_l.append(np.zeros((5, 3), np.uint32))
+    for n in sizes:
+        p = (rng.uniform(-1, 1, (n, 1, 3)) + rng.uniform(-0.05, 0.05, (n, 3, 3))).astype(np.float32).reshape(-1, 3)
+        pos_l.append(p)
+        idx_l.append(rng.permutation(3 * n).astype(np.uint32).reshape(-1, 3))
+        idx_l.append(np.zeros((n % 7, 3), np.uint32))
+        descs.append((v, 3 * n, t, n))
+        v, t = v + 3 * n, t + n + n % 7
+    pos, idx = np.concatenate(pos_l), np.concatenate(idx_l)
+    order = rng.permutation(len(descs))
+    p, i = torch.from_numpy(pos).cuda(), torch.from_numpy(idx.view(np.int32)).cuda()
+    for leaf in (4, 1):
+        b = rq.Batch(ctx, [descs[k] for k in order], max_leaf=leaf)
+        b.build(p, i)
+        b.build(p, i)
+        ctx.sync_check()
+        for m, k in enumerate(order):
+            vo, nv, to, nt = descs[k]
+            s = rq.Bvh.build(ctx, p[vo:vo + nv].contiguous(), i[to:to + nt].contiguous(), max_leaf=leaf)
+            for g, w, name in zip(b.download(m), s.download(), ("nodes2", "tris", "nodes4", "perm")):
+                assert g.tobytes() == w.tobytes(), (nt, name)
+            s.destroy()
+        b.destroy()
