@@ -99,115 +99,6 @@ __device__ __forceinline__ uint32_t count_in(const uint32_t* klo, const uint32_t
     return khi[i] - klo[i] + 1u;
 }
 
-// Sorted leaf k: leaf-ordered triangle copy, permutation, sorted key, leaf box,
-// and the depth-first emission count of the leaf starting at k: the emitted
-// leaf holding k is its highest ancestor with count <= max_leaf; if it starts
-// at k, c = 1 + (consecutive left-child links above it).
-__device__ __forceinline__ void leaf_step(uint32_t k, const float* __restrict__ pos, uint32_t sf,
-                                          const uint32_t* __restrict__ idx, uint32_t max_leaf, const uint32_t* skeys,
-                                          const uint32_t* sids, const uint32_t* klo, const uint32_t* khi,
-                                          const uint32_t* par_in, const uint32_t* par_lf, float4* box_lf,
-                                          uint32_t* c_out, rq_triangle* tris, uint32_t* perm, uint32_t* keys_out) {
-    const uint32_t id = sids[k];
-    F3 p0, p1, p2;
-    load_tri(pos, sf, idx, id, p0, p1, p2);
-    float4* tp = reinterpret_cast<float4*>(tris + k);
-    tp[0] = make_float4(p0.x, p0.y, p0.z, 0.0f);
-    tp[1] = make_float4(p1.x, p1.y, p1.z, 0.0f);
-    tp[2] = make_float4(p2.x, p2.y, p2.z, 0.0f);
-    perm[k] = id;
-    keys_out[k] = skeys[k];
-    box_lf[2 * size_t(k)] = make_float4(fminf(p0.x, fminf(p1.x, p2.x)), fminf(p0.y, fminf(p1.y, p2.y)),
-                                        fminf(p0.z, fminf(p1.z, p2.z)), 0.0f);
-    box_lf[2 * size_t(k) + 1] = make_float4(fmaxf(p0.x, fmaxf(p1.x, p2.x)), fmaxf(p0.y, fmaxf(p1.y, p2.y)),
-                                            fmaxf(p0.z, fmaxf(p1.z, p2.z)), 0.0f);
-    uint32_t par = par_lf[k];
-    uint32_t ulo = k;
-    while (par != kNoParent) {
-        const uint32_t pp = par >> 1;
-        if (count_in(klo, khi, pp) > max_leaf) break;
-        ulo = klo[pp];
-        par = par_in[pp];
-    }
-    uint32_t c = 0;
-    if (ulo == k) {
-        uint32_t L = 0;
-        while (par != kNoParent && (par & 1u) == 0u) {
-            ++L;
-            par = par_in[par >> 1];
-        }
-        c = 1u + L;
-    }
-    c_out[k] = c;
-}
-
-// The leaves [L0, L1) of a tree by one block of kLocal threads (at most kLocal
-// leaves), with every node whose range lies inside refitted in shared memory.
-// A node's index is one end of its leaf range, so such a node has its index
-// inside too: it takes its arrival count and box in shared memory (CTA-scope
-// ordering), and writes the box to global memory once for the emission.  A
-// walk that reaches a node whose range crosses the block's ends there: its
-// parent link goes to hand(par) (from at most one walk per leaf), to be
-// carried on by refit_walk_up.  Unions are exact, so the boxes equal
-// refit_walk's.  Call with the whole block.
-constexpr uint32_t kLocal = 256;  // 17 KB of shared memory per block (measured: faster than 512)
-struct LocalLeaves {
-    uint32_t flag[kLocal];
-    float4 lf[2 * kLocal];  // leaf boxes (lo, hi)
-    float4 in[2 * kLocal];  // boxes of the block's inner nodes
-    uint32_t top[kLocal];   // the handed-over walks
-    uint32_t ntop, base;
-};
-
-__device__ __forceinline__ void leaves_local(LocalLeaves& S, uint32_t L0, uint32_t L1, const float* __restrict__ pos,
-                                             uint32_t sf, const uint32_t* __restrict__ idx, uint32_t max_leaf,
-                                             const uint32_t* skeys, const uint32_t* sids, const int32_t* kl,
-                                             const int32_t* kr, const uint32_t* klo, const uint32_t* khi,
-                                             const uint32_t* par_in, const uint32_t* par_lf, float4* box_in,
-                                             float4* box_lf, uint32_t* c_out, rq_triangle* tris, uint32_t* perm,
-                                             uint32_t* keys_out, uint32_t* err) {
-    for (uint32_t i = threadIdx.x; i < kLocal; i += blockDim.x) S.flag[i] = 0u;
-    if (threadIdx.x == 0) S.ntop = 0u;
-    for (uint32_t k = L0 + threadIdx.x; k < L1; k += blockDim.x) {
-        leaf_step(k, pos, sf, idx, max_leaf, skeys, sids, klo, khi, par_in, par_lf, box_lf, c_out, tris, perm,
-                  keys_out);
-        S.lf[2 * (k - L0)] = box_lf[2 * size_t(k)];
-        S.lf[2 * (k - L0) + 1] = box_lf[2 * size_t(k) + 1];
-    }
-    __syncthreads();
-    for (uint32_t k = L0 + threadIdx.x; k < L1; k += blockDim.x) {
-        uint32_t par = par_lf[k];
-        uint32_t guard = 0;
-        while (par != kNoParent) {
-            const uint32_t p = par >> 1;
-            if (__ldg(klo + p) < L0 || __ldg(khi + p) >= L1) {
-                // from here up every range crosses a block's end
-                S.top[atomicAdd(&S.ntop, 1u)] = par;
-                break;
-            }
-            const int32_t a = kl[p], b = kr[p];
-            __threadfence_block();  // release this thread's shared-memory box
-            if (atomicAdd(&S.flag[p - L0], 1u) == 0u) break;
-            __threadfence_block();  // acquire the sibling's
-            const float4* pa = a < 0 ? S.lf + 2 * ((uint32_t(a) & 0x7fffffffu) - L0) : S.in + 2 * (a - L0);
-            const float4* pb = b < 0 ? S.lf + 2 * ((uint32_t(b) & 0x7fffffffu) - L0) : S.in + 2 * (b - L0);
-            const float4 alo = pa[0], ahi = pa[1], blo = pb[0], bhi = pb[1];
-            const float4 lo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f);
-            const float4 hi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
-            S.in[2 * (p - L0)] = lo;
-            S.in[2 * (p - L0) + 1] = hi;
-            __stcg(box_in + 2 * size_t(p), lo);
-            __stcg(box_in + 2 * size_t(p) + 1, hi);
-            par = par_in[p];
-            if (++guard > 128u) {
-                set_err(err, RQ_DERR_REFIT);
-                break;
-            }
-        }
-    }
-    __syncthreads();
-}
-
 // Atomic bottom-up refit from the parent link `par` of a node whose box is
 // final: at each node the second child to arrive computes the union box and
 // continues upward.  The arrival count is an acquire-release add: it publishes
@@ -236,50 +127,320 @@ __device__ __forceinline__ void refit_walk_up(uint32_t par, const int32_t* kl, c
     }
 }
 
-// Depth-first pre-order node writes for primitive position p: internal node
-// p (if emitted) sits at A[lo] + L, the emitted leaf starting at p (if any)
-// at A[p] + c[p] - 1.  Returns c[p].
+// ------------------------------------------------- the LBVH's tree, bottom up
+// The binary radix tree of the sorted codes (Karras 2012, ties by position)
+// built from the leaves up as Apetrei 2014: a range's parent splits it off at
+// whichever end shares the longer prefix with its neighbour, so a node needs
+// only its own range and the two gaps at its ends, and its box, its place in
+// the depth-first order and its children's emission come from the same climb.
+// A node is named by its gap: the first position of its right child.
+//
+// What the climb leaves for the emission, all by position:
+//   ch[x]     bits 0..7: emitted nodes whose range starts at x and that are
+//             not below another starting there, counted down the left links
+//             (c: the inner ones and the emitted leaf; 0: no emitted node);
+//             bits 8..15: emitted nodes on the left links of the node with gap
+//             x, itself included (h; 0: not emitted)
+//   rec[2x]   the node with gap x, if emitted: (min, range start), (max, -)
+//   leaf[2x]  the emitted leaf that starts at x: (min, count), (max, -)
+// With A the exclusive scan of c, the chain of emitted nodes starting at x
+// takes the places A[x] .. A[x] + c[x] - 1, outermost first: the node with gap
+// x and range start lo goes to A[lo + 1] - 1 - h, its right child to A[x].
+// (Depths stay below 30 + 27 levels, so c and h fit a byte.)
+//
+// A block takes kTreeLeaves sorted leaves and climbs in shared memory; nodes
+// whose sibling lies outside go on in tree_climb_top with the same steps over
+// global memory.  The form this replaces searched each node's range (Karras),
+// wrote children, ranges and parents to memory, and read them again in the
+// refit and in two chains of dependent loads per leaf and node.  On 8.3M
+// triangles (1,132 us before, 593 us now, scan included): search 235 us, leaves
+// and refit 549 -> 382, its top 113 -> 62, node writes 165 -> 111; 512 meshes of
+// 4.73M triangles together 733 -> 383.  The climb's blocks are bound by the L1
+// (LSU wavefronts at 73 %: scattered vertex reads 40 % of the time, shared
+// memory the rest); 512 leaves per block doubled the top's time, 128 threads of
+// 8 leaves took 493 us.
+constexpr uint32_t kTreeT = 256, kTreeItems = 4, kTreeLeaves = kTreeT * kTreeItems;
+constexpr uint32_t kTreeBlocks = 5;  // per SM (registers and shared memory; 4: 422 us for 382 us on 8.3M)
+
+struct TreeOut {
+    rq_triangle* tris;
+    uint32_t *perm, *keys;
+    uint16_t* ch;
+    float4 *rec, *leaf;
+    // unfinished nodes: (min, other end), (max, h) at the end that touches the
+    // sibling, and one arrival bit per gap (zeroed)
+    float4* slot;
+    uint32_t* seen;
+};
+
+// Slots are padded so that a warp's neighbouring quadruples fall in distinct banks.
+__device__ __forceinline__ uint32_t tree_slot(uint32_t i) { return i + (i >> 5); }
+
+struct TreeShared {
+    float box[6][kTreeLeaves + kTreeLeaves / 32];
+    uint8_t adj[kTreeLeaves + 1];   // common prefix + 1 across the gap before a position; 0: none
+    uint32_t seen[kTreeLeaves / 16 + 1];  // arrivals per gap: bit 0 the left child, bit 1 the right one
+    uint32_t count, base;
+    union {
+        float4 stage[kTreeT / 32][96];  // a warp's 32 triangles as they are written; then
+        struct {
+            uint16_t end[kTreeLeaves];  // an unfinished node's other end
+            uint8_t h[kTreeLeaves];
+            uint16_t ch[kTreeLeaves + 2];
+            uint16_t list[kTreeLeaves + 2];  // (gap << 1) | is_right
+        };
+    };
+};
+
+// Common prefix + 1 of the sorted codes on both sides of the gap before x (0: no gap).
+__device__ __forceinline__ uint32_t tree_gap(const uint32_t* keys, uint32_t n, uint32_t x) {
+    if (x == 0u || x >= n) return 0u;
+    const uint32_t d = keys[x - 1u] ^ keys[x];
+    return d ? uint32_t(__clz(d)) + 1u : 33u + uint32_t(__clz((x - 1u) ^ x));
+}
+
+struct TreeBox {
+    float v[6];  // min, max
+};
+__device__ __forceinline__ TreeBox tree_union(const TreeBox& a, const TreeBox& b) {
+    TreeBox r;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        r.v[k] = fminf(a.v[k], b.v[k]);
+        r.v[3 + k] = fmaxf(a.v[3 + k], b.v[3 + k]);
+    }
+    return r;
+}
+__device__ __forceinline__ void tree_put(float4* at, const TreeBox& b, uint32_t lo_w, uint32_t hi_w) {
+    __stcg(at, make_float4(b.v[0], b.v[1], b.v[2], __uint_as_float(lo_w)));
+    __stcg(at + 1, make_float4(b.v[3], b.v[4], b.v[5], __uint_as_float(hi_w)));
+}
+
+// A finished node [lo, hi] with gap x: its records and its children's.
+// Returns the word ch[x] gets; h: in, the left child's; out, the node's.
+__device__ __forceinline__ uint32_t tree_emit(const TreeOut& O, uint32_t max_leaf, uint32_t lo, uint32_t x, uint32_t hi,
+                                              const TreeBox& l, const TreeBox& r, const TreeBox& b, uint32_t& h,
+                                              uint32_t hr) {
+    if (hi - lo + 1u <= max_leaf) {
+        h = 0u;
+        return 0u;
+    }
+    h += 1u;
+    tree_put(O.rec + 2 * size_t(x), b, lo, 0u);
+    if (x - lo <= max_leaf) tree_put(O.leaf + 2 * size_t(lo), l, x - lo, 0u);
+    if (hi - x + 1u <= max_leaf) tree_put(O.leaf + 2 * size_t(x), r, hi - x + 1u, 0u);
+    return (h << 8) | (hr + 1u);
+}
+// The root's own place (and the leaf it is, if it is one).
+__device__ __forceinline__ uint32_t tree_root(const TreeOut& O, uint32_t max_leaf, uint32_t n, const TreeBox& b,
+                                              uint32_t h) {
+    if (n <= max_leaf) tree_put(O.leaf, b, n, 0u);
+    return h + 1u;
+}
+
+// The vertices of the warp's 32 triangles (lane's triangle: id), component by
+// component: neighbouring lanes read neighbouring words, 11 rows per load
+// instead of 32.  stage[3 * lane + c] = vertex c of the lane's triangle (its
+// fourth word holds the vertex index).
+__device__ __forceinline__ void tree_gather(float4* stage, uint32_t id, const float* __restrict__ pos, uint32_t sf,
+                                            const uint32_t* __restrict__ idx) {
+    const uint32_t lane = threadIdx.x & 31u;
+    float* s = reinterpret_cast<float*>(stage);
+#pragma unroll
+    for (uint32_t j = 0; j < 3; ++j) {
+        const uint32_t e = j * 32u + lane, t = e / 3u, i = __shfl_sync(0xffffffffu, id, int(t)) * 3u + (e - 3u * t);
+        s[4u * e + 3u] = __uint_as_float(idx ? __ldg(idx + i) : i);
+    }
+    __syncwarp();
+    float v[9];
+#pragma unroll
+    for (uint32_t j = 0; j < 9; ++j) {
+        const uint32_t f = j * 32u + lane, e = f / 3u;
+        v[j] = __ldg(pos + size_t(__float_as_uint(s[4u * e + 3u])) * sf + (f - 3u * e));
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 9; ++j) {
+        const uint32_t f = j * 32u + lane, e = f / 3u;
+        s[4u * e + (f - 3u * e)] = v[j];
+    }
+    __syncwarp();
+}
+
+// The leaves [L0, min(L0 + kTreeLeaves, n)) by one block of kTreeT threads:
+// the leaf-ordered triangles, permutation and keys, and every node whose range
+// lies inside.  On return S.list[0 .. S.count) holds the unfinished nodes
+// (gaps from L0), their slots written to O.slot.
+__device__ __forceinline__ void tree_climb_block(TreeShared& S, uint32_t L0, uint32_t n, const float* __restrict__ pos,
+                                                 uint32_t sf, const uint32_t* __restrict__ idx, uint32_t max_leaf,
+                                                 const uint32_t* __restrict__ keys, const uint32_t* __restrict__ ids,
+                                                 const TreeOut& O) {
+    const uint32_t m = min(kTreeLeaves, n - L0), lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    for (uint32_t i = threadIdx.x; i < kTreeLeaves / 16 + 1; i += kTreeT) S.seen[i] = 0u;
+    for (uint32_t i = threadIdx.x; i <= m; i += kTreeT) S.adj[i] = uint8_t(tree_gap(keys, n, L0 + i));
+    if (threadIdx.x == 0) S.count = 0u;
+    float4* stage = S.stage[warp];
+#pragma unroll 1
+    for (uint32_t r = 0; r < kTreeItems; ++r) {
+        const uint32_t i0 = (r * (kTreeT / 32) + warp) * 32u, i = i0 + lane;
+        if (i0 >= m) break;
+        const uint32_t id = ids[L0 + min(i, m - 1u)];
+        tree_gather(stage, id, pos, sf, idx);
+        const float4 a = stage[3 * lane], b = stage[3 * lane + 1], c = stage[3 * lane + 2];
+        if (i < m) {
+            O.perm[L0 + i] = id;
+            O.keys[L0 + i] = keys[L0 + i];
+            const uint32_t s = tree_slot(i);
+            S.box[0][s] = fminf(a.x, fminf(b.x, c.x));
+            S.box[1][s] = fminf(a.y, fminf(b.y, c.y));
+            S.box[2][s] = fminf(a.z, fminf(b.z, c.z));
+            S.box[3][s] = fmaxf(a.x, fmaxf(b.x, c.x));
+            S.box[4][s] = fmaxf(a.y, fmaxf(b.y, c.y));
+            S.box[5][s] = fmaxf(a.z, fmaxf(b.z, c.z));
+        }
+        float4* out = reinterpret_cast<float4*>(O.tris + L0 + i0);
+#pragma unroll
+        for (uint32_t j = 0; j < 3; ++j) {
+            const uint32_t e = j * 32u + lane;
+            float4 v = stage[e];
+            v.w = 0.0f;
+            if (i0 + e / 3u < m) out[e] = v;
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i <= m; i += kTreeT) S.ch[i] = 0;
+    __syncthreads();
+
+    // ---- the climb: a thread takes four neighbours, all but its last climb end early
+    auto load = [&](uint32_t at) {
+        TreeBox b;
+        const uint32_t s = tree_slot(at);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) b.v[k] = S.box[k][s];
+        return b;
+    };
+#pragma unroll 1
+    for (uint32_t j = 0; j < kTreeItems; ++j) {
+        const uint32_t k = threadIdx.x * kTreeItems + j;
+        if (k >= m) break;
+        uint32_t lo = k, hi = k, h = 0;  // positions from L0
+        TreeBox b = load(k);
+        for (;;) {
+            const uint32_t dl = S.adj[lo], dr = S.adj[hi + 1u];
+            if (!(dl | dr)) {
+                S.ch[0] = uint16_t(tree_root(O, max_leaf, n, b, h));
+                break;
+            }
+            const bool right = dl > dr;
+            const uint32_t x = right ? lo : hi + 1u;
+            volatile uint32_t* sw = S.seen + (x >> 4);
+            const uint32_t sh = 2u * (x & 15u), own = (right ? 2u : 1u) << sh, other = (right ? 1u : 2u) << sh;
+            if (*sw & other) {
+                atomicOr(const_cast<uint32_t*>(sw), own);
+            } else {
+                const uint32_t at = right ? lo : hi, s = tree_slot(at);
+#pragma unroll
+                for (int q = 0; q < 6; ++q) S.box[q][s] = b.v[q];
+                S.end[at] = uint16_t(right ? hi : lo);
+                S.h[at] = uint8_t(h);
+                __threadfence_block();  // the node before its arrival
+                if (!(atomicOr(const_cast<uint32_t*>(sw), own) & other)) break;
+            }
+            __threadfence_block();
+            const uint32_t at = right ? x - 1u : x, he = S.h[at];
+            const TreeBox sib = load(at);
+            uint32_t hr = he;
+            if (right) {
+                lo = S.end[at];
+                hr = h;
+                h = he;
+            } else {
+                hi = S.end[at];
+            }
+            const TreeBox l = right ? sib : b, r = right ? b : sib;
+            b = tree_union(l, r);
+            S.ch[x] = uint16_t(tree_emit(O, max_leaf, L0 + lo, L0 + x, L0 + hi, l, r, b, h, hr));
+        }
+    }
+    __syncthreads();
+
+    // ---- the emission words; the nodes whose sibling has not come
+    for (uint32_t i = threadIdx.x; i <= m; i += kTreeT) {
+        if (i < m) O.ch[L0 + i] = S.ch[i];
+        const uint32_t a = (S.seen[i >> 4] >> (2u * (i & 15u))) & 3u;
+        if (a == 1u || a == 2u) {
+            const uint32_t at = a == 1u ? i - 1u : i;
+            S.list[atomicAdd(&S.count, 1u)] = uint16_t((i << 1) | (a - 1u));
+            tree_put(O.slot + 2 * size_t(L0 + at), load(at), L0 + S.end[at], S.h[at]);
+        }
+    }
+    __syncthreads();
+}
+
+// Carries an unfinished node on over global memory (entry: (gap << 1) | is_right).
+__device__ __forceinline__ void tree_climb_top(uint32_t entry, uint32_t n, uint32_t max_leaf,
+                                               const uint32_t* __restrict__ keys, const TreeOut& O) {
+    auto load = [&](uint32_t at, TreeBox& b, uint32_t& end, uint32_t& h) {
+        const float4 lo = ld_cg4(O.slot + 2 * size_t(at)), hi = ld_cg4(O.slot + 2 * size_t(at) + 1);
+        b = TreeBox{{lo.x, lo.y, lo.z, hi.x, hi.y, hi.z}};
+        end = __float_as_uint(lo.w);
+        h = __float_as_uint(hi.w);
+    };
+    uint32_t x = entry >> 1;
+    bool right = entry & 1u;
+    TreeBox b;
+    uint32_t lo = x, hi = x - 1u, h;
+    if (right)
+        load(x, b, hi, h);
+    else
+        load(x - 1u, b, lo, h);
+    for (;;) {
+        const uint32_t bit = 1u << (x & 31u);
+        if (!(atom_or_acq_rel(O.seen + (x >> 5), bit) & bit)) return;
+        TreeBox sib;
+        uint32_t end, he, hr;
+        load(right ? x - 1u : x, sib, end, he);
+        if (right) {
+            lo = end;
+            hr = h;
+            h = he;
+        } else {
+            hi = end;
+            hr = he;
+        }
+        const TreeBox l = right ? sib : b, r = right ? b : sib;
+        b = tree_union(l, r);
+        O.ch[x] = uint16_t(tree_emit(O, max_leaf, lo, x, hi, l, r, b, h, hr));
+        const uint32_t dl = tree_gap(keys, n, lo), dr = tree_gap(keys, n, hi + 1u);
+        if (!(dl | dr)) {
+            O.ch[0] = uint16_t(tree_root(O, max_leaf, n, b, h));
+            return;
+        }
+        right = dl > dr;
+        x = right ? lo : hi + 1u;
+        tree_put(O.slot + 2 * size_t(right ? lo : hi), b, right ? hi : lo, h);
+    }
+}
+
+// The nodes that position x emits: the inner node with gap x and the leaf that
+// starts at x.  Returns the number of nodes emitted up to x.
 template <class Scan>
-__device__ __forceinline__ uint32_t emit_step(uint32_t p, uint32_t n, uint32_t max_leaf, const int32_t* kr,
-                                              const uint32_t* klo, const uint32_t* khi, const uint32_t* par_in,
-                                              const uint32_t* par_lf, const float4* box_in, const float4* box_lf,
-                                              const uint32_t* c, const Scan& A, rq_bvh2_node* out) {
-    if (p + 1 < n && count_in(klo, khi, p) > max_leaf) {
-        uint32_t L = 0, par = par_in[p];
-        while (par != kNoParent && (par & 1u) == 0u) {
-            ++L;
-            par = par_in[par >> 1];
-        }
-        const uint32_t pre = A[klo[p]] + L;
-        const int32_t r = kr[p];
-        const uint32_t rlo = r < 0 ? (uint32_t(r) & 0x7fffffffu) : klo[r];
-        // refit boxes were stored with st.cg: read them from L2
-        const float4 lo = ld_cg4(box_in + 2 * size_t(p)), hi = ld_cg4(box_in + 2 * size_t(p) + 1);
-        float4* o = reinterpret_cast<float4*>(out + pre);
-        o[0] = make_float4(lo.x, lo.y, lo.z, __int_as_float(int32_t(pre + 1)));
-        o[1] = make_float4(hi.x, hi.y, hi.z, __int_as_float(int32_t(A[rlo])));
+__device__ __forceinline__ uint32_t tree_write(uint32_t x, const TreeOut& O, const Scan& A, rq_bvh2_node* out) {
+    const uint32_t w = O.ch[x], c = w & 255u, h = w >> 8, a = A[x];
+    if (h) {
+        const float4 lo = ldg4(O.rec + 2 * size_t(x)), hi = ldg4(O.rec + 2 * size_t(x) + 1);
+        const uint32_t at = A[__float_as_uint(lo.w) + 1u] - 1u - h;
+        float4* o = reinterpret_cast<float4*>(out + at);
+        o[0] = make_float4(lo.x, lo.y, lo.z, __int_as_float(int32_t(at + 1u)));
+        o[1] = make_float4(hi.x, hi.y, hi.z, __int_as_float(int32_t(a)));
     }
-    const uint32_t cp = c[p];
-    if (cp) {
-        uint32_t par = par_lf[p];
-        uint32_t node = p;
-        bool is_leaf = true;
-        while (par != kNoParent) {
-            const uint32_t pp = par >> 1;
-            if (count_in(klo, khi, pp) > max_leaf) break;
-            node = pp;
-            is_leaf = false;
-            par = par_in[pp];
-        }
-        const uint32_t cnt = is_leaf ? 1u : count_in(klo, khi, node);
-        const float4* b = is_leaf ? box_lf + 2 * size_t(node) : box_in + 2 * size_t(node);
-        const float4 lo = ld_cg4(b), hi = ld_cg4(b + 1);
-        const uint32_t pre = A[p] + cp - 1u;
-        float4* o = reinterpret_cast<float4*>(out + pre);
-        o[0] = make_float4(lo.x, lo.y, lo.z, __int_as_float(~int32_t(p)));
-        o[1] = make_float4(hi.x, hi.y, hi.z, __int_as_float(int32_t(cnt)));
+    if (c) {
+        const float4 lo = ldg4(O.leaf + 2 * size_t(x)), hi = ldg4(O.leaf + 2 * size_t(x) + 1);
+        float4* o = reinterpret_cast<float4*>(out + a + c - 1u);
+        o[0] = make_float4(lo.x, lo.y, lo.z, __int_as_float(~int32_t(x)));
+        o[1] = make_float4(hi.x, hi.y, hi.z, lo.w);  // (count)
     }
-    return cp;
+    return a + c;
 }
 
 // ------------------------------------------------------------- collapse

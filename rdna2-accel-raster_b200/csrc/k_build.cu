@@ -3,19 +3,19 @@
 //   1. per-triangle centroid ((p0+p1)+p2)/3 (software_bvh.hpp:53) and
 //      centroid bounds (ordered-uint atomics);
 //   2. 30-bit Morton code in the cube of the largest centroid extent;
-//   3. onesweep radix sort of (code, triangle id)              [k_sort.cu]
-//   4. Karras 2012 internal nodes, parent links;
-//   5. one thread per sorted leaf: leaf-ordered triangle copy, permutation,
-//      leaf box, the depth-first emission count of the leaf starting there,
-//      then the atomic bottom-up box refit;
-//   6. exclusive scan of the emission counts                    [k_sort.cu]
-//   7. depth-first pre-order node writes: every emitted node v sits at
-//      A[lo(v)] + L(v), where lo(v) is its first primitive, A the scan and
-//      L(v) the number of consecutive left-child links above v — the order of
-//      SoftwareBVH::recursiveBuild (software_bvh.hpp:90-175): left child at
-//      parent + 1, right child after the left subtree;
-//   8. the greedy 4-wide collapse                               [k_collapse.cu]
-// The per-element steps live in build_core.cuh (shared with k_batch.cu).
+//   3. radix sort of (code, triangle id)                       [k_sort.cu]
+//   4. the leaf-ordered triangles and permutation, and the binary radix tree
+//      with its boxes, from the leaves up              [build_core.cuh]
+//   5. exclusive scan of the emission counts                    [k_sort.cu]
+//   6. depth-first pre-order node writes: left child at parent + 1, right child
+//      after the left subtree, the order of SoftwareBVH::recursiveBuild
+//      (software_bvh.hpp:90-175): a node sits at A[lo(v)] + L(v), where lo(v)
+//      is its first primitive, A the scan and L(v) the number of consecutive
+//      left-child links above v;
+//   7. the greedy 4-wide collapse                               [k_collapse.cu]
+// With SAH subtrees (RQ_BUILD_SAH) step 4 is Karras 2012's search per node and
+// the steps further down.  The per-element steps live in build_core.cuh (shared
+// with k_forest.cu).
 // Also the refit of an existing handle (k_parents2, k_refit2, k_refit4).
 #include <algorithm>
 
@@ -81,54 +81,43 @@ __global__ void __launch_bounds__(kT) k_karras(const uint32_t* __restrict__ keys
     if (n == 1 && blockIdx.x == 0 && threadIdx.x == 0) par_lf[0] = rq::kNoParent;
 }
 
-// Leaves and refit with the bottom of the tree refitted in shared memory
-// (leaves_local): block b owns the sorted leaves [kLocal*b, kLocal*(b+1)).
-// Walks that leave the block are listed for k_refit_top, which carries them
-// on with device-scope arrivals: a block is done once its own leaves and local
-// nodes are, instead of holding its slot while a walk climbs through the
-// tree's top.
-using rq::kLocal;
+// The leaf order's outputs and the tree with its boxes (tree_climb_block):
+// block b owns the sorted leaves [kTreeLeaves * b, ...).  Nodes that leave the
+// block are listed for k_tree_top, which carries them on with device-scope
+// arrivals: a block is done once its own leaves and nodes are, instead of
+// holding its slot while a climb goes through the tree's top.
+using rq::kTreeLeaves;
 
-__global__ void __launch_bounds__(kT) k_leaves_local(
-    const float* __restrict__ pos, uint32_t sf, const uint32_t* __restrict__ idx, uint32_t n, uint32_t max_leaf,
-    const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ sids, const int32_t* __restrict__ kl,
-    const int32_t* __restrict__ kr, const uint32_t* __restrict__ klo, const uint32_t* __restrict__ khi,
-    const uint32_t* __restrict__ par_in, const uint32_t* __restrict__ par_lf, float4* box_in,
-    float4* __restrict__ box_lf, uint32_t* __restrict__ c_out, rq_triangle* __restrict__ tris,
-    uint32_t* __restrict__ perm, uint32_t* __restrict__ keys_out, uint32_t* __restrict__ top_list,
-    uint32_t* top_cnt, uint32_t* err) {
-    __shared__ rq::LocalLeaves S;
-    const uint32_t L0 = blockIdx.x * kLocal;
-    rq::leaves_local(S, L0, min(L0 + kLocal, n), pos, sf, idx, max_leaf, skeys, sids, kl, kr, klo, khi, par_in, par_lf,
-                     box_in, box_lf, c_out, tris, perm, keys_out, err);
+__global__ void __launch_bounds__(rq::kTreeT, rq::kTreeBlocks) k_tree(const float* __restrict__ pos, uint32_t sf,
+                                             const uint32_t* __restrict__ idx, uint32_t n, uint32_t max_leaf,
+                                             const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ sids,
+                                             const __grid_constant__ rq::TreeOut out, uint32_t* __restrict__ top_list,
+                                             uint32_t* top_cnt) {
+    __shared__ rq::TreeShared S;
+    rq::tree_climb_block(S, blockIdx.x * kTreeLeaves, n, pos, sf, idx, max_leaf, skeys, sids, out);
     // the block's hand-offs, with one device atomic
-    if (threadIdx.x == 0 && S.ntop) S.base = atomicAdd(top_cnt, S.ntop);
+    if (threadIdx.x == 0 && S.count) S.base = atomicAdd(top_cnt, S.count);
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < S.ntop; i += kT) top_list[S.base + i] = S.top[i];
+    for (uint32_t i = threadIdx.x; i < S.count; i += rq::kTreeT)
+        top_list[S.base + i] = 2u * blockIdx.x * kTreeLeaves + S.list[i];
 }
 
-// The walks k_leaves_local handed over.
-__global__ void __launch_bounds__(kT) k_refit_top(const int32_t* __restrict__ kl, const int32_t* __restrict__ kr,
-                                                  const uint32_t* __restrict__ par_in, float4* box_in,
-                                                  const float4* box_lf, uint32_t* refit_flag,
-                                                  const uint32_t* __restrict__ top_list, const uint32_t* top_cnt,
-                                                  uint32_t* err) {
+__global__ void __launch_bounds__(kT) k_tree_top(uint32_t n, uint32_t max_leaf, const uint32_t* __restrict__ skeys,
+                                                 const __grid_constant__ rq::TreeOut out,
+                                                 const uint32_t* __restrict__ top_list, const uint32_t* top_cnt) {
     const uint32_t m = *top_cnt;
     for (uint32_t j = blockIdx.x * kT + threadIdx.x; j < m; j += gridDim.x * kT)
-        rq::refit_walk_up(top_list[j], kl, kr, par_in, box_in, box_lf, refit_flag, err);
+        rq::tree_climb_top(top_list[j], n, max_leaf, skeys, out);
 }
 
-__global__ void __launch_bounds__(kT) k_emit2(uint32_t n, uint32_t max_leaf, const int32_t* __restrict__ kr,
-                                              const uint32_t* __restrict__ klo, const uint32_t* __restrict__ khi,
-                                              const uint32_t* __restrict__ par_in,
-                                              const uint32_t* __restrict__ par_lf, const float4* __restrict__ box_in,
-                                              const float4* __restrict__ box_lf, const uint32_t* __restrict__ c,
-                                              const uint32_t* __restrict__ A, rq_bvh2_node* __restrict__ out,
+// The binary nodes at their depth-first places (A: the scan of the emission counts).
+__global__ void __launch_bounds__(kT) k_emit2(uint32_t n, uint32_t max_leaf, const __grid_constant__ rq::TreeOut out,
+                                              const uint32_t* __restrict__ A, rq_bvh2_node* __restrict__ nodes,
                                               uint32_t* __restrict__ counts) {
     for (uint32_t p = blockIdx.x * kT + threadIdx.x; p < n; p += gridDim.x * kT) {
-        const uint32_t cp = rq::emit_step(p, n, max_leaf, kr, klo, khi, par_in, par_lf, box_in, box_lf, c, A, out);
+        const uint32_t end = rq::tree_write(p, out, A, nodes);
         if (p == n - 1) {
-            counts[0] = A[p] + cp;  // binary node count
+            counts[0] = end;
             counts[3] = max_leaf;
         }
     }
@@ -1585,16 +1574,8 @@ size_t rq_build_scratch_carve(void* base, uint32_t n, BuildScratch& s, bool sah)
     s.vals[1] = c.take<uint32_t>(N);
     s.sort_words = c.take<uint32_t>(rq_sort_words(uint32_t(N), 1));
     s.tile_ctr = c.take<uint32_t>(16);
-    s.kl = c.take<int32_t>(N);
-    s.kr = c.take<int32_t>(N);
-    s.klo = c.take<uint32_t>(N);
-    s.khi = c.take<uint32_t>(N);
-    s.par_in = c.take<uint32_t>(N);
-    s.par_lf = c.take<uint32_t>(N);
     s.box_in = c.take<float4>(2 * N);
     s.box_lf = c.take<float4>(2 * N);
-    s.refit_flag = c.take<uint32_t>(N);
-    s.c = c.take<uint32_t>(N);
     s.a = c.take<uint32_t>(N);
     s.scan_status = c.take<uint32_t>(stiles + 1);
     s.q = c.take<uint32_t>(N);
@@ -1604,6 +1585,25 @@ size_t rq_build_scratch_carve(void* base, uint32_t n, BuildScratch& s, bool sah)
     s.cpar = c.take<uint32_t>(N);
     s.cacc = c.take<unsigned long long>(N);
     s.coll_ctl = c.take<uint32_t>(256);
+    s.kl = s.kr = nullptr;
+    s.klo = s.khi = s.par_in = s.par_lf = s.refit_flag = s.c = nullptr;
+    s.slot = nullptr;
+    s.ch = nullptr;
+    s.seen = nullptr;
+    if (sah) {
+        s.kl = c.take<int32_t>(N);
+        s.kr = c.take<int32_t>(N);
+        s.klo = c.take<uint32_t>(N);
+        s.khi = c.take<uint32_t>(N);
+        s.par_in = c.take<uint32_t>(N);
+        s.par_lf = c.take<uint32_t>(N);
+        s.refit_flag = c.take<uint32_t>(N);
+        s.c = c.take<uint32_t>(N);
+    } else {
+        s.slot = c.take<float4>(2 * N);
+        s.ch = c.take<uint16_t>(N);
+        s.seen = c.take<uint32_t>(N / 32 + 1);
+    }
     s.sah_hi = s.sah_L = s.sah_node = s.sah_list = s.sah_depth = s.sah_rec_l = nullptr;
     s.sah_rec = s.sah_plo = s.sah_phi = s.sah_mrec = nullptr;
     s.sah_pcz = nullptr;
@@ -1760,7 +1760,6 @@ int rq_launch_build(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t stride_
     cudaMemsetAsync(s.bounds, 0xff, 3 * sizeof(uint32_t), st);
     cudaMemsetAsync(s.bounds + 3, 0x00, 3 * sizeof(uint32_t), st);
     cudaMemsetAsync(s.tile_ctr, 0, 16 * sizeof(uint32_t), st);
-    if (n > 1) cudaMemsetAsync(s.refit_flag, 0, sizeof(uint32_t) * (n - 1), st);
 
     k_centroids<<<grid_for(n, sms), kT, 0, st>>>(pos, sf, idx, n, s.cent, s.bounds);
     k_morton<<<grid_for(n, sms), kT, 0, st>>>(s.cent, n, s.bounds, s.keys[0], s.vals[0]);
@@ -1769,26 +1768,25 @@ int rq_launch_build(rq_ctx* ctx, rq_bvh* bvh, const float* pos, uint32_t stride_
     if (rc) return rc;
     const uint32_t* skeys = s.keys[rb];
     const uint32_t* sids = s.vals[rb];
-    k_karras<<<grid_for(n, sms), kT, 0, st>>>(skeys, n, s.kl, s.kr, s.klo, s.khi, s.par_in, s.par_lf);
     if (sah) {
+        if (n > 1) cudaMemsetAsync(s.refit_flag, 0, sizeof(uint32_t) * (n - 1), st);
+        k_karras<<<grid_for(n, sms), kT, 0, st>>>(skeys, n, s.kl, s.kr, s.klo, s.khi, s.par_in, s.par_lf);
         rc = launch_sah(ctx, bvh, s, pos, sf, idx, n, max_leaf, sah_max, skeys, sids, st);
         if (rc) return rc;
         if (collapse) return rq_launch_collapse(ctx, bvh, s, st);
         return RQ_OK;
     }
-    // the handed-over walks: listed in the centroid array (free after the
+    // the unfinished nodes: listed in the centroid array (free after the
     // Morton codes), counted in tile_ctr[12] (zeroed above, unused by the sort)
     uint32_t* top_list = reinterpret_cast<uint32_t*>(s.cent);
     uint32_t* top_cnt = s.tile_ctr + 12;
-    k_leaves_local<<<(n + kLocal - 1) / kLocal, kT, 0, st>>>(pos, sf, idx, n, max_leaf, skeys, sids, s.kl, s.kr,
-                                                             s.klo, s.khi, s.par_in, s.par_lf, s.box_in, s.box_lf,
-                                                             s.c, bvh->tris, bvh->perm, bvh->skeys,
-                                                             top_list, top_cnt, ctx->d_err);
-    k_refit_top<<<uint32_t(sms) * 4u, kT, 0, st>>>(s.kl, s.kr, s.par_in, s.box_in, s.box_lf, s.refit_flag, top_list,
-                                                   top_cnt, ctx->d_err);
-    rq_launch_scan(ctx, s.c, s.a, n, s.scan_status, s.tile_ctr + 8, st);
-    k_emit2<<<grid_for(n, sms), kT, 0, st>>>(n, max_leaf, s.kr, s.klo, s.khi, s.par_in, s.par_lf, s.box_in, s.box_lf,
-                                             s.c, s.a, bvh->nodes2, bvh->d_counts);
+    const rq::TreeOut out{bvh->tris, bvh->perm, bvh->skeys, s.ch, s.box_in, s.box_lf, s.slot, s.seen};
+    cudaMemsetAsync(s.seen, 0, sizeof(uint32_t) * (n / 32 + 1), st);
+    k_tree<<<(n + kTreeLeaves - 1) / kTreeLeaves, rq::kTreeT, 0, st>>>(pos, sf, idx, n, max_leaf, skeys, sids, out, top_list,
+                                                               top_cnt);
+    k_tree_top<<<uint32_t(sms) * 4u, kT, 0, st>>>(n, max_leaf, skeys, out, top_list, top_cnt);
+    rq_launch_scan(ctx, s.ch, s.a, n, s.scan_status, s.tile_ctr + 8, st);
+    k_emit2<<<grid_for(n, sms), kT, 0, st>>>(n, max_leaf, out, s.a, bvh->nodes2, bvh->d_counts);
     rc = rq_cuda_status(ctx, cudaGetLastError(), "build launch");
     if (rc) return rc;
     if (collapse) return rq_launch_collapse(ctx, bvh, s, st);

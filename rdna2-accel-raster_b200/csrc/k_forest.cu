@@ -6,9 +6,9 @@
 //
 // A build by one block or cluster per mesh, the form this replaces, was bound
 // by the largest meshes' chains of steps on one SM: 2.06 ms for 512 meshes of
-// 64 to 65,536 triangles (4.73M).  All meshes together take 1.31 ms: leaves
-// and refit 0.46, the collapse (still a block per mesh: its levels are short)
-// 0.26, the sort 0.22, the radix trees 0.12, the node writes 0.11.
+// 64 to 65,536 triangles (4.73M).  All meshes together take 0.94 ms: the tree
+// 0.28, the collapse (still a block per mesh: its levels are short) 0.26, the
+// sort 0.22, the node writes 0.07.
 // Batches of more than kGroupTris triangles go in groups of whole meshes that
 // use the scratch in turn.
 #include <algorithm>
@@ -27,7 +27,7 @@ using namespace rq;
 constexpr int kT = 256;
 constexpr uint32_t kGroupTris = 16u << 20;
 constexpr uint32_t kMaxLevels = 120;
-static_assert(kLocal == kT, "a block of elements is a block of leaves");
+static_assert(kTreeLeaves % kT == 0, "a block of elements is a block of leaves");
 
 struct ForestScratch {
     float4* cent;
@@ -37,9 +37,9 @@ struct ForestScratch {
     size_t zero_bytes;  // ... to here
     uint32_t *keys[2], *vals[2];
     uint32_t* counts;   // sort: 256 per tile
-    int32_t *kl, *kr;
-    uint32_t *klo, *khi, *par_in, *par_lf, *refit_flag, *c, *a, *scan_status;
-    float4 *box_in, *box_lf;
+    float4 *rec, *leaf, *slot;
+    uint16_t* ch;
+    uint32_t *seen, *a, *scan_status;
     uint2* top_list;
     uint32_t* q;
     int32_t *cand, *child_q;
@@ -52,24 +52,19 @@ size_t carve(void* base, const rq_forest_group& g, ForestScratch& s) {
     const size_t N = g.tris;
     s.bounds = c.take<uint32_t>(6ull * g.segs);
     s.misc = c.take<uint32_t>(16);
+    s.seen = c.take<uint32_t>(g.seen_words);
     s.zero = s.bounds;
     s.zero_bytes = c.off;
     s.cent = c.take<float4>(N);
     for (int k = 0; k < 2; ++k) s.keys[k] = c.take<uint32_t>(N);
     for (int k = 0; k < 2; ++k) s.vals[k] = c.take<uint32_t>(N);
     s.counts = c.take<uint32_t>(256ull * g.tiles);
-    s.kl = c.take<int32_t>(N);
-    s.kr = c.take<int32_t>(N);
-    s.klo = c.take<uint32_t>(N);
-    s.khi = c.take<uint32_t>(N);
-    s.par_in = c.take<uint32_t>(N);
-    s.par_lf = c.take<uint32_t>(N);
-    s.refit_flag = c.take<uint32_t>(N);
-    s.c = c.take<uint32_t>(N);
+    s.rec = c.take<float4>(2 * N);
+    s.leaf = c.take<float4>(2 * N);
+    s.slot = c.take<float4>(2 * N);
+    s.ch = c.take<uint16_t>(N);
     s.a = c.take<uint32_t>(N);
     s.scan_status = c.take<uint32_t>(rq_scan_tiles(uint32_t(N)) + 1);
-    s.box_in = c.take<float4>(2 * N);
-    s.box_lf = c.take<float4>(2 * N);
     s.top_list = c.take<uint2>(N);
     s.q = c.take<uint32_t>(N);
     s.cand = c.take<int32_t>(4 * N);
@@ -103,14 +98,13 @@ __global__ void __launch_bounds__(kT) k_forest_centroids(const __grid_constant__
     __shared__ float s_red[6][kT / 32];
     const uint2 b = A.blocks[blockIdx.x];
     const rq_forest_seg g = A.segs[b.x];
-    const uint32_t i = b.y + threadIdx.x;
     float v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    if (i < g.n) {
+    const uint32_t end = min(b.y + kTreeLeaves, g.n);
+    for (uint32_t i = b.y + threadIdx.x; i < end; i += kT) {
         F3 p0, p1, p2;
         load_tri(A.pos + size_t(g.vert) * A.sf, A.sf, A.idx + 3ull * g.tri, i, p0, p1, p2);
         const float4 c = centroid(p0, p1, p2);
         A.s.cent[g.first + i] = c;
-        A.s.refit_flag[g.first + i] = 0u;
         const float x[3] = {c.x, c.y, c.z};
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -140,47 +134,41 @@ __global__ void __launch_bounds__(kT) k_forest_centroids(const __grid_constant__
 __global__ void __launch_bounds__(kT) k_forest_morton(const __grid_constant__ ForestArgs A) {
     const uint2 b = A.blocks[blockIdx.x];
     const rq_forest_seg g = A.segs[b.x];
-    const uint32_t i = b.y + threadIdx.x;
-    if (i >= g.n) return;
     const uint32_t* bd = A.s.bounds + 6ull * b.x;
     const float lx = o2f(~bd[0]), ly = o2f(~bd[1]), lz = o2f(~bd[2]);
     const float scale = morton_scale(lx, ly, lz, o2f(bd[3]), o2f(bd[4]), o2f(bd[5]));
-    A.s.keys[0][g.first + i] = morton30(A.s.cent[g.first + i], lx, ly, lz, scale);
-    A.s.vals[0][g.first + i] = i;
+    const uint32_t end = min(b.y + kTreeLeaves, g.n);
+    for (uint32_t i = b.y + threadIdx.x; i < end; i += kT) {
+        A.s.keys[0][g.first + i] = morton30(A.s.cent[g.first + i], lx, ly, lz, scale);
+        A.s.vals[0][g.first + i] = i;
+    }
 }
 
-__global__ void __launch_bounds__(kT) k_forest_karras(const __grid_constant__ ForestArgs A) {
-    const uint2 b = A.blocks[blockIdx.x];
-    const rq_forest_seg g = A.segs[b.x];
-    const uint32_t i = b.y + threadIdx.x;
+// A mesh's part of the tree arrays.
+__device__ __forceinline__ TreeOut tree_of(const ForestArgs& A, const rq_forest_seg& g) {
     const size_t o = g.first;
-    if (i + 1 < g.n)
-        karras_node(A.s.keys[0] + o, int(g.n), int(i), A.s.kl + o, A.s.kr + o, A.s.klo + o, A.s.khi + o, A.s.par_in + o,
-                    A.s.par_lf + o);
-    if (g.n == 1 && i == 0) A.s.par_lf[o] = kNoParent;
+    return TreeOut{A.tris + g.tri,    A.perm + g.tri,    A.skeys + g.tri,   A.s.ch + o,
+                   A.s.rec + 2 * o,   A.s.leaf + 2 * o,  A.s.slot + 2 * o,  A.s.seen + g.seen};
 }
 
-__global__ void __launch_bounds__(kT) k_forest_leaves(const __grid_constant__ ForestArgs A) {
-    __shared__ LocalLeaves S;
+__global__ void __launch_bounds__(kTreeT, kTreeBlocks) k_forest_tree(const __grid_constant__ ForestArgs A) {
+    __shared__ TreeShared S;
     const uint2 b = A.blocks[blockIdx.x];
     const rq_forest_seg g = A.segs[b.x];
-    const size_t o = g.first;
-    leaves_local(S, b.y, min(b.y + kLocal, g.n), A.pos + size_t(g.vert) * A.sf, A.sf, A.idx + 3ull * g.tri, A.max_leaf,
-                 A.s.keys[0] + o, A.s.vals[0] + o, A.s.kl + o, A.s.kr + o, A.s.klo + o, A.s.khi + o, A.s.par_in + o,
-                 A.s.par_lf + o, A.s.box_in + 2 * o, A.s.box_lf + 2 * o, A.s.c + o, A.tris + g.tri, A.perm + g.tri,
-                 A.skeys + g.tri, A.err);
-    if (threadIdx.x == 0 && S.ntop) S.base = atomicAdd(A.s.misc, S.ntop);
+    tree_climb_block(S, b.y, g.n, A.pos + size_t(g.vert) * A.sf, A.sf, A.idx + 3ull * g.tri, A.max_leaf,
+                     A.s.keys[0] + g.first, A.s.vals[0] + g.first, tree_of(A, g));
+    if (threadIdx.x == 0 && S.count) S.base = atomicAdd(A.s.misc, S.count);
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < S.ntop; i += kT) A.s.top_list[S.base + i] = make_uint2(b.x, S.top[i]);
+    for (uint32_t i = threadIdx.x; i < S.count; i += kTreeT)
+        A.s.top_list[S.base + i] = make_uint2(b.x, 2u * b.y + S.list[i]);
 }
 
-__global__ void __launch_bounds__(kT) k_forest_refit_top(const __grid_constant__ ForestArgs A) {
+__global__ void __launch_bounds__(kT) k_forest_tree_top(const __grid_constant__ ForestArgs A) {
     const uint32_t m = A.s.misc[0];
     for (uint32_t j = blockIdx.x * kT + threadIdx.x; j < m; j += gridDim.x * kT) {
         const uint2 w = A.s.top_list[j];
-        const size_t o = A.segs[w.x].first;
-        refit_walk_up(w.y, A.s.kl + o, A.s.kr + o, A.s.par_in + o, A.s.box_in + 2 * o, A.s.box_lf + 2 * o,
-                      A.s.refit_flag + o, A.err);
+        const rq_forest_seg g = A.segs[w.x];
+        tree_climb_top(w.y, g.n, A.max_leaf, A.s.keys[0] + g.first, tree_of(A, g));
     }
 }
 
@@ -194,16 +182,15 @@ struct ScanFrom {
 __global__ void __launch_bounds__(kT) k_forest_emit(const __grid_constant__ ForestArgs A) {
     const uint2 b = A.blocks[blockIdx.x];
     const rq_forest_seg g = A.segs[b.x];
-    const uint32_t p = b.y + threadIdx.x;
-    if (p >= g.n) return;
-    const size_t o = g.first;
-    const ScanFrom scan{A.s.a + o, A.s.a[o]};
-    const uint32_t cp = emit_step(p, g.n, A.max_leaf, A.s.kr + o, A.s.klo + o, A.s.khi + o, A.s.par_in + o,
-                                  A.s.par_lf + o, A.s.box_in + 2 * o, A.s.box_lf + 2 * o, A.s.c + o, scan,
-                                  A.nodes2 + 2ull * g.tri);
-    if (p == g.n - 1) {
-        A.counts[4ull * g.mesh] = scan[p] + cp;
-        A.counts[4ull * g.mesh + 3] = A.max_leaf;
+    const TreeOut out = tree_of(A, g);
+    const ScanFrom scan{A.s.a + g.first, A.s.a[g.first]};
+    const uint32_t end = min(b.y + kTreeLeaves, g.n);
+    for (uint32_t p = b.y + threadIdx.x; p < end; p += kT) {
+        const uint32_t total = tree_write(p, out, scan, A.nodes2 + 2ull * g.tri);
+        if (p == g.n - 1) {
+            A.counts[4ull * g.mesh] = total;
+            A.counts[4ull * g.mesh + 3] = A.max_leaf;
+        }
     }
 }
 
@@ -266,8 +253,9 @@ void rq_forest_plan(const std::vector<rq_mesh_desc>& meshes, rq_forest& f) {
             g.tile0 = uint32_t(f.tiles.size());
             g.begin0 = uint32_t(f.seg_tiles.size());
         }
-        f.segs.push_back(rq_forest_seg{g.tris, d.triangle_offset, d.vertex_offset, d.num_triangles, m});
-        for (uint32_t i = 0; i < d.num_triangles; i += kT, ++g.blocks) f.blocks.push_back(make_uint2(g.segs, i));
+        f.segs.push_back(rq_forest_seg{g.tris, d.triangle_offset, d.vertex_offset, d.num_triangles, m, g.seen_words});
+        g.seen_words += d.num_triangles / 32 + 1;
+        for (uint32_t i = 0; i < d.num_triangles; i += kTreeLeaves, ++g.blocks) f.blocks.push_back(make_uint2(g.segs, i));
         f.seg_tiles.push_back(g.tiles);
         for (uint32_t i = 0; i < d.num_triangles; i += RQ_SORT_TILE, ++g.tiles)
             f.tiles.push_back(rq_sort_tile{g.tris + i, std::min(RQ_SORT_TILE, d.num_triangles - i), g.tris, 0u});
@@ -315,10 +303,9 @@ int rq_launch_batch_build(rq_ctx* ctx, rq_batch* b, const float* pos, uint32_t s
                                       &rb);
         if (rc) return rc;
         if (rb != 0) return rq_set_error(ctx, RQ_ERR_STATE, "sorted keys in the other buffer");
-        k_forest_karras<<<g.blocks, kT, 0, st>>>(a);
-        k_forest_leaves<<<g.blocks, kT, 0, st>>>(a);
-        k_forest_refit_top<<<uint32_t(ctx->num_sms) * 4u, kT, 0, st>>>(a);
-        rq_launch_scan(ctx, a.s.c, a.s.a, g.tris, a.s.scan_status, a.s.misc + 1, st);
+        k_forest_tree<<<g.blocks, kTreeT, 0, st>>>(a);
+        k_forest_tree_top<<<uint32_t(ctx->num_sms) * 4u, kT, 0, st>>>(a);
+        rq_launch_scan(ctx, a.s.ch, a.s.a, g.tris, a.s.scan_status, a.s.misc + 1, st);
         k_forest_emit<<<g.blocks, kT, 0, st>>>(a);
         k_forest_collapse<<<g.segs, kCollapseT, 0, st>>>(a);
         e = cudaGetLastError();

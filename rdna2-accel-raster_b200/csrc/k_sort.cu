@@ -474,7 +474,22 @@ __global__ void __launch_bounds__(kThreads, 4) k_tile_scatter(const uint32_t* __
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kThreads * kScanItems;
 
-__global__ void __launch_bounds__(kThreads) k_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+__device__ __forceinline__ void scan_words(const uint32_t* in, uint32_t (&v)[kScanItems]) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(in)), b = __ldg(reinterpret_cast<const uint4*>(in) + 1);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+__device__ __forceinline__ void scan_words(const uint16_t* in, uint32_t (&v)[kScanItems]) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(in));
+    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) v[i] = (w[i >> 1] >> (16 * (i & 1))) & 255u;
+}
+__device__ __forceinline__ uint32_t scan_word(const uint32_t* in) { return *in; }
+__device__ __forceinline__ uint32_t scan_word(const uint16_t* in) { return *in & 255u; }
+
+// In: 32-bit words, or the low bytes of 16-bit ones (16-byte aligned).
+template <class In>
+__global__ void __launch_bounds__(kThreads) k_scan(const In* __restrict__ in, uint32_t* __restrict__ out,
                                                    uint32_t n, uint32_t* status, uint32_t* tile_ctr, uint32_t* err) {
     __shared__ uint32_t s_warp[kWarps];
     __shared__ uint32_t s_tile, s_prefix;
@@ -484,11 +499,15 @@ __global__ void __launch_bounds__(kThreads) k_scan(const uint32_t* __restrict__ 
     const uint32_t base = tile * kScanTile + threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
     uint32_t sum = 0;
+    const bool full = base + kScanItems <= n;
+    if (full) {
+        scan_words(in + base, v);
+    } else {
 #pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        v[i] = base + i < n ? in[base + i] : 0u;
-        sum += v[i];
+        for (int i = 0; i < kScanItems; ++i) v[i] = base + i < n ? scan_word(in + base + i) : 0u;
     }
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) sum += v[i];
     uint32_t total;
     uint32_t ex = block_exclusive_scan(sum, s_warp, &total);
     if (threadIdx.x < 32) {
@@ -533,8 +552,18 @@ __global__ void __launch_bounds__(kThreads) k_scan(const uint32_t* __restrict__ 
     uint32_t run = s_prefix + ex;
 #pragma unroll
     for (int i = 0; i < kScanItems; ++i) {
-        if (base + i < n) out[base + i] = run;
-        run += v[i];
+        const uint32_t x = v[i];
+        v[i] = run;
+        run += x;
+    }
+    if (full) {
+        uint4* o = reinterpret_cast<uint4*>(out + base);
+        o[0] = make_uint4(v[0], v[1], v[2], v[3]);
+        o[1] = make_uint4(v[4], v[5], v[6], v[7]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i)
+            if (base + i < n) out[base + i] = v[i];
     }
 }
 
@@ -608,9 +637,18 @@ int rq_launch_sort_tiles(rq_ctx* ctx, const SortIO& io, const rq_sort_tile* tile
     return rq_cuda_status(ctx, cudaGetLastError(), "segment sort launch");
 }
 
-void rq_launch_scan(rq_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* status,
-                    uint32_t* tile_ctr, cudaStream_t st) {
+template <class In>
+static void launch_scan(rq_ctx* ctx, const In* in, uint32_t* out, uint32_t n, uint32_t* status, uint32_t* tile_ctr,
+                        cudaStream_t st) {
     const uint32_t tiles = rq_scan_tiles(n);
     cudaMemsetAsync(status, 0, sizeof(uint32_t) * tiles, st);
     k_scan<<<tiles, kThreads, 0, st>>>(in, out, n, status, tile_ctr, ctx->d_err);
+}
+void rq_launch_scan(rq_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* status, uint32_t* tile_ctr,
+                    cudaStream_t st) {
+    launch_scan(ctx, in, out, n, status, tile_ctr, st);
+}
+void rq_launch_scan(rq_ctx* ctx, const uint16_t* in, uint32_t* out, uint32_t n, uint32_t* status, uint32_t* tile_ctr,
+                    cudaStream_t st) {
+    launch_scan(ctx, in, out, n, status, tile_ctr, st);
 }

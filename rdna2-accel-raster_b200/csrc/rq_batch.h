@@ -10,9 +10,10 @@
 #include "rq_internal.h"
 
 // One mesh in a group of meshes built together: where its elements lie in the
-// scratch arrays, its descriptor's offsets, its triangles, its number.
+// scratch arrays, its descriptor's offsets, its triangles, its number, its
+// first word of arrival bits.
 struct rq_forest_seg {
-    uint32_t first, tri, vert, n, mesh;
+    uint32_t first, tri, vert, n, mesh, seen;
 };
 struct rq_forest_group {
     uint32_t seg0 = 0, segs = 0;      // segments (meshes)
@@ -20,6 +21,7 @@ struct rq_forest_group {
     uint32_t tile0 = 0, tiles = 0;    // sort tiles
     uint32_t begin0 = 0;              // first tile of each segment, and the end: segs + 1 entries
     uint32_t tris = 0;
+    uint32_t seen_words = 0;          // arrival bits, a whole number of words per segment
 };
 // The tables that deal a batch's builds out to blocks (k_forest.cu).
 struct rq_forest {

@@ -35,13 +35,14 @@ __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
 // Fetch-and-add with acquire-release semantics: releases this thread's
 // earlier stores and acquires those released by earlier adds on the same
 // word (the hand-off of a bottom-up refit, without separate fences).
-template <bool CTA = false>
 __device__ __forceinline__ uint32_t atom_add_acq_rel(uint32_t* p, uint32_t v) {
     uint32_t old;
-    if (CTA)
-        asm volatile("atom.acq_rel.cta.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-    else
-        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    return old;
+}
+__device__ __forceinline__ uint32_t atom_or_acq_rel(uint32_t* p, uint32_t v) {
+    uint32_t old;
+    asm volatile("atom.acq_rel.gpu.global.or.b32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
     return old;
 }
 // L2-coherent 16-B load (bypasses L1), for data written by other blocks in

@@ -96,14 +96,19 @@ struct BuildScratch {
     uint32_t* vals[2];     // N each
     uint32_t* sort_words;  // rq_sort_words(N, 1)
     uint32_t* tile_ctr;    // 16 counters
+    float4* box_in;        // 2N: node boxes (lo, hi), or by gap the emitted nodes' records
+    float4* box_lf;        // 2N: leaf boxes, or by first position the emitted leaves' records
+    // the plain LBVH (null with SAH subtrees; see build_core.cuh)
+    float4* slot;          // 2N unfinished nodes
+    uint16_t* ch;          // N  emission words
+    uint32_t* seen;        // N bits: arrivals
+    // LBVH with SAH-rebuilt subtrees (null otherwise)
     int32_t* kl;           // N-1 Karras left child (bit 31: leaf)
     int32_t* kr;           // N-1 right child
     uint32_t* klo;         // N-1 range start
     uint32_t* khi;         // N-1 range end (inclusive)
     uint32_t* par_in;      // N-1 parent of internal node: (parent << 1) | is_right
     uint32_t* par_lf;      // N   parent of leaf
-    float4* box_in;        // 2(N-1): lo, hi
-    float4* box_lf;        // 2N
     uint32_t* refit_flag;  // N-1
     uint32_t* c;           // N   emission counts
     uint32_t* a;           // N   exclusive scan of c
@@ -182,7 +187,10 @@ int rq_launch_sort_tiles(rq_ctx* ctx, const SortIO& io, const rq_sort_tile* tile
 uint32_t rq_scan_tiles(uint32_t n);
 // Exclusive scan of in[0..n).
 void rq_launch_scan(rq_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* status,
-                    uint32_t* tile_ctr, cudaStream_t st);
+                    uint32_t* tile_ctr, cudaStream_t s);
+// The same over the low bytes of 16-bit words.
+void rq_launch_scan(rq_ctx* ctx, const uint16_t* in, uint32_t* out, uint32_t n, uint32_t* status,
+                    uint32_t* tile_ctr, cudaStream_t s);
 
 // ---------------------------------------------------------------- k_collapse
 int rq_launch_collapse(rq_ctx* ctx, rq_bvh* bvh, BuildScratch& s, cudaStream_t st);

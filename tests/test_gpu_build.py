@@ -71,6 +71,16 @@ def test_small_build_parity(ctx, n, max_leaf):
     assert_same_as_oracle(ctx, soup(n, 400 + n), None, max_leaf)
 
 
+@pytest.mark.parametrize("equal", [0, 3000, 1 << 30])
+@pytest.mark.parametrize("n,max_leaf", [(5119, 1), (5120, 4), (5121, 16), (6145, 2), (9217, 3)])
+def test_tree_blocks_parity(ctx, n, max_leaf, equal):
+    """Sizes at the edges of the tree's 1,024-leaf blocks, with runs of equal codes inside and across them."""
+    pos = soup(n, 500 + n)
+    m = min(n, equal)
+    pos[:3 * m] = np.tile(pos[:3], (m, 1))
+    assert_same_as_oracle(ctx, pos, None, max_leaf)
+
+
 @pytest.mark.parametrize("n", [1023, 1024, 1025, 606207, 606208, 606209, 610304, 610305])
 def test_sort_forms_parity(ctx, n):
     """The sort's tile edges in both its forms and on both sides of the length where one takes over from the other."""
