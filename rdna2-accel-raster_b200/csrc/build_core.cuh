@@ -465,12 +465,20 @@ __device__ __forceinline__ N2 load_n2(const rq_bvh2_node* n2, int32_t i) {
     return o;
 }
 
+// The collapse's surface area of a node.
+__device__ __forceinline__ float node_area(const N2& nd) {
+    const float dx = nd.mx[0] - nd.mn[0], dy = nd.mx[1] - nd.mn[1], dz = nd.mx[2] - nd.mn[2];
+    return 2.0f * ((dx * dy + dy * dz) + dz * dx);
+}
+
 // Greedy candidates of SoftwareBVH4::collapse (software_bvh.hpp:225-247)
 // for inner binary node u: open the inner candidate with the largest
 // surface area (strict >, first wins) until four.  Returns the count;
-// inner[i]: candidate i is an inner binary node.
+// inner[i]: candidate i is an inner binary node.  end, ce: in a pre-order tree,
+// the end of u's range and of each candidate's.
 template <bool NC>
-__device__ __forceinline__ int greedy_candidates(const rq_bvh2_node* n2, int32_t u, int32_t c[4], bool inner[4]) {
+__device__ __forceinline__ int greedy_candidates(const rq_bvh2_node* n2, int32_t u, int32_t c[4], bool inner[4],
+                                                 int32_t end, int32_t (&ce)[4]) {
     // each candidate's children and surface area, loaded once (slots are
     // static indices, so the records stay in registers)
     int32_t cl[4], cr[4];
@@ -479,10 +487,7 @@ __device__ __forceinline__ int greedy_candidates(const rq_bvh2_node* n2, int32_t
         c[i] = id;
         cl[i] = nd.l;
         cr[i] = nd.r;
-        const float dx = nd.mx[0] - nd.mn[0];
-        const float dy = nd.mx[1] - nd.mn[1];
-        const float dz = nd.mx[2] - nd.mn[2];
-        sa[i] = 2.0f * ((dx * dy + dy * dz) + dz * dx);
+        sa[i] = node_area(nd);
     };
     const N2 nd = load_n2<NC>(n2, u);
     {
@@ -490,6 +495,9 @@ __device__ __forceinline__ int greedy_candidates(const rq_bvh2_node* n2, int32_t
         set(0, nd.l, a);
         set(1, nd.r, b);
     }
+    ce[0] = nd.r;
+    ce[1] = end;
+    ce[2] = ce[3] = 0;
     c[2] = c[3] = -1;
     cl[2] = cl[3] = -1;
     cr[2] = cr[3] = -1;
@@ -506,13 +514,18 @@ __device__ __forceinline__ int greedy_candidates(const rq_bvh2_node* n2, int32_t
                 best = i;
             }
         if (best < 0) break;
-        int32_t l = 0, r = 0;
+        int32_t l = 0, r = 0, e = 0;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (i == best) {
                 l = cl[i];
                 r = cr[i];
+                e = ce[i];
+                ce[i] = r;
             }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i == nc) ce[i] = e;
         const N2 a = load_n2<NC>(n2, l), b = load_n2<NC>(n2, r);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -526,13 +539,11 @@ __device__ __forceinline__ int greedy_candidates(const rq_bvh2_node* n2, int32_t
     return nc;
 }
 
-// Writes 4-wide node p from its candidates; inner children get pre-order
-// positions p+1, p+1 + size(first inner child), ... (sizes by queue index).
-template <bool NC, class SizeOf, class PreOut>
-__device__ __forceinline__ void write_node4(const rq_bvh2_node* n2, const int32_t cand[4], const int32_t cq[4],
-                                            uint32_t p, SizeOf size_of, PreOut pre_out, rq_bvh4_node* out4,
-                                            int32_t* map4) {
-    uint32_t off = p + 1u;
+// Writes 4-wide node p from its candidates and the places of the inner ones
+// (-1: a leaf).
+template <bool NC>
+__device__ __forceinline__ void write_node4(const rq_bvh2_node* n2, const int32_t (&cand)[4], const int32_t (&at)[4],
+                                            uint32_t p, rq_bvh4_node* out4, int32_t* map4) {
     float mnx[4], mxx[4], mny[4], mxy[4], mnz[4], mxz[4];
     int32_t ci[4], cc[4];
 #pragma unroll
@@ -548,18 +559,16 @@ __device__ __forceinline__ void write_node4(const rq_bvh2_node* n2, const int32_
             mxy[k] = nd.mx[1];
             mnz[k] = nd.mn[2];
             mxz[k] = nd.mx[2];
-            if (cq[k] >= 0) {
-                pre_out(cq[k], off);
-                ci[k] = int32_t(off);
+            if (at[k] >= 0) {
+                ci[k] = at[k];
                 cc[k] = -1;
-                off += size_of(cq[k]);
             } else {
                 ci[k] = nd.l;
                 cc[k] = nd.r;
             }
         }
-        map4[4 * size_t(p) + k] = cand[k];
     }
+    reinterpret_cast<int4*>(map4)[p] = make_int4(cand[0], cand[1], cand[2], cand[3]);
     float4* o = reinterpret_cast<float4*>(out4 + p);
     o[0] = make_float4(mnx[0], mnx[1], mnx[2], mnx[3]);
     o[1] = make_float4(mxx[0], mxx[1], mxx[2], mxx[3]);
@@ -605,16 +614,13 @@ __device__ __forceinline__ uint32_t inner_children(const CollapseIO& io, uint32_
 //      1 + the sizes of the earlier inner siblings (a walk up that stops at
 //      the first ancestor whose position a written parent already
 //      published), then the node write.
-// LEVELS: phases 2 and 3 level by level instead (bottom-up sizes, then
-// top-down positions, one sync per level; `acc` holds the positions) — the
-// faster form when sync() is a block barrier.  NARROW > 0 (grid-wide use):
+// NARROW > 0 (grid-wide use):
 // block 0 alone expands the top levels while they hold at most NARROW
 // entries.  io.tail holds 16 control words.
-// s_lvl (shared, max_levels + 2 entries) records the level boundaries.
 // Data written inside the collapse is read with ld.cg: other blocks wrote it.
-template <bool NC, bool LEVELS, uint32_t NARROW, class Sync>
+template <bool NC, uint32_t NARROW, class Sync>
 __device__ __forceinline__ bool collapse_levels(const CollapseIO& io, uint32_t tid, uint32_t nthreads,
-                                                uint32_t* s_lvl, uint32_t max_levels, Sync sync, uint32_t* err,
+                                                uint32_t max_levels, Sync sync, uint32_t* err,
                                                 uint32_t* total_out, uint32_t* depth_out) {
     const bool root_leaf = load_n2<NC>(io.n2, 0).l < 0;
     // Entries of level L+1 are appended at end(L) + an atomic count of their
@@ -628,12 +634,12 @@ __device__ __forceinline__ bool collapse_levels(const CollapseIO& io, uint32_t t
     // depend on them.
     auto expand = [&](uint32_t e, uint32_t end, uint32_t depth) {
         const int32_t u = int32_t(__ldcg(io.q + e));
-        int32_t c[4] = {-1, -1, -1, -1};
+        int32_t c[4] = {-1, -1, -1, -1}, ce[4];
         bool inner[4] = {false, false, false, false};
         if (root_leaf)
             c[0] = 0;
         else
-            greedy_candidates<NC>(io.n2, u, c, inner);
+            greedy_candidates<NC>(io.n2, u, c, inner, 0, ce);
         const uint32_t cnt = uint32_t(inner[0]) + uint32_t(inner[1]) + uint32_t(inner[2]) + uint32_t(inner[3]);
         const uint32_t act = __activemask();
         const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
@@ -691,7 +697,6 @@ __device__ __forceinline__ bool collapse_levels(const CollapseIO& io, uint32_t t
         depth = __ldcg(io.tail + 10);
     }
     while (start < end) {
-        if (threadIdx.x == 0) s_lvl[depth] = start;
         if (tid == 0) atomicExch(lvl_cnt + (depth + 1) % 3u, 0u);
         for (uint32_t e = start + tid; e < end; e += nthreads) expand(e, end, depth);
         if (!sync()) return false;
@@ -704,104 +709,65 @@ __device__ __forceinline__ bool collapse_levels(const CollapseIO& io, uint32_t t
             return false;
         }
     }
-    if (threadIdx.x == 0) s_lvl[depth] = end;
-    struct SizeOf {
-        const uint32_t* sz;
-        __device__ uint32_t operator()(int32_t i) const { return __ldcg(sz + i); }
-    };
-    if constexpr (LEVELS) {
-        __syncthreads();
-        uint32_t* pre = reinterpret_cast<uint32_t*>(io.acc);  // acc[0] = 0: the root at 0
-        for (int lv = int(depth) - 1; lv >= 0; --lv) {
-            for (uint32_t e = s_lvl[lv] + tid; e < s_lvl[lv + 1]; e += nthreads) {
-                uint32_t s = 1;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int32_t cq = __ldcg(io.child_q + 4 * size_t(e) + k);
-                    if (cq >= 0) s += __ldcg(io.sz + cq);
-                }
-                __stcg(io.sz + e, s);
+    for (uint32_t e = tid; e < end; e += nthreads) {
+        if (inner_children(io, e) != 0u) continue;
+        uint32_t cur = e, s = 1u;
+        __stcg(io.sz + cur, s);
+        for (uint32_t guard = 0;; ++guard) {
+            const uint32_t pk = __ldcg(io.par + cur);
+            if (pk == kNoParent) break;
+            if (guard >= max_levels) {
+                set_err(err, RQ_DERR_QUEUE);
+                break;
             }
-            if (!sync()) return false;
+            const uint32_t p = pk >> 2;
+            const unsigned long long old = atomicAdd(io.acc + p, (1ull << 32) | s);
+            if (uint32_t(old >> 32) + 1u < inner_children(io, p)) break;
+            s = 1u + uint32_t(old) + s;
+            __stcg(io.sz + p, s);
+            cur = p;
         }
-        struct PreOut {
-            uint32_t* pre;
-            __device__ void operator()(int32_t i, uint32_t v) const { __stcg(pre + i, v); }
-        };
-        for (uint32_t lv = 0; lv < depth; ++lv) {
-            for (uint32_t e = s_lvl[lv] + tid; e < s_lvl[lv + 1]; e += nthreads) {
-                int32_t cand[4], cq[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    cand[k] = __ldcg(io.cand + 4 * size_t(e) + k);
-                    cq[k] = __ldcg(io.child_q + 4 * size_t(e) + k);
-                }
-                write_node4<NC>(io.n2, cand, cq, __ldcg(pre + e), SizeOf{io.sz}, PreOut{pre}, io.out4, io.map4);
-            }
-            if (!sync()) return false;
-        }
-        *total_out = end;
-        *depth_out = depth;
-        return true;
-    } else {
-        for (uint32_t e = tid; e < end; e += nthreads) {
-            if (inner_children(io, e) != 0u) continue;
-            uint32_t cur = e, s = 1u;
-            __stcg(io.sz + cur, s);
-            for (uint32_t guard = 0;; ++guard) {
-                const uint32_t pk = __ldcg(io.par + cur);
-                if (pk == kNoParent) break;
-                if (guard >= max_levels) {
-                    set_err(err, RQ_DERR_QUEUE);
-                    break;
-                }
-                const uint32_t p = pk >> 2;
-                const unsigned long long old = atomicAdd(io.acc + p, (1ull << 32) | s);
-                if (uint32_t(old >> 32) + 1u < inner_children(io, p)) break;
-                s = 1u + uint32_t(old) + s;
-                __stcg(io.sz + p, s);
-                cur = p;
-            }
-        }
-        if (!sync()) return false;
-        // a written node publishes its inner children's positions in `acc`
-        // (bit 63 set; phase 2 never sets it), so most walks stop at once
-        struct PrePublish {
-            unsigned long long* acc;
-            __device__ void operator()(int32_t i, uint32_t v) const { __stcg(acc + i, (1ull << 63) | v); }
-        };
-        for (uint32_t e = tid; e < end; e += nthreads) {
-            uint32_t pre = 0, cur = e;
-            for (;;) {
-                const unsigned long long a = __ldcg(io.acc + cur);
-                if (a >> 63) {
-                    pre += uint32_t(a);
-                    break;
-                }
-                const uint32_t pk = __ldcg(io.par + cur);
-                if (pk == kNoParent) break;  // the root, at 0
-                const uint32_t p = pk >> 2, slot = pk & 3u;
-                uint32_t off = 1u;
-                for (uint32_t j = 0; j < slot; ++j) {
-                    const int32_t cq = __ldcg(io.child_q + 4 * size_t(p) + j);
-                    if (cq >= 0) off += __ldcg(io.sz + cq);
-                }
-                pre += off;
-                cur = p;
-            }
-            int32_t cand[4], cq[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                cand[k] = __ldcg(io.cand + 4 * size_t(e) + k);
-                cq[k] = __ldcg(io.child_q + 4 * size_t(e) + k);
-            }
-            write_node4<NC>(io.n2, cand, cq, pre, SizeOf{io.sz}, PrePublish{io.acc}, io.out4, io.map4);
-        }
-        if (!sync()) return false;
-        *total_out = end;
-        *depth_out = depth;
-        return true;
     }
+    if (!sync()) return false;
+    // a written node publishes its inner children's positions in `acc`
+    // (bit 63 set; phase 2 never sets it), so most walks stop at once
+    for (uint32_t e = tid; e < end; e += nthreads) {
+        uint32_t pre = 0, cur = e;
+        for (;;) {
+            const unsigned long long a = __ldcg(io.acc + cur);
+            if (a >> 63) {
+                pre += uint32_t(a);
+                break;
+            }
+            const uint32_t pk = __ldcg(io.par + cur);
+            if (pk == kNoParent) break;  // the root, at 0
+            const uint32_t p = pk >> 2, slot = pk & 3u;
+            uint32_t off = 1u;
+            for (uint32_t j = 0; j < slot; ++j) {
+                const int32_t cq = __ldcg(io.child_q + 4 * size_t(p) + j);
+                if (cq >= 0) off += __ldcg(io.sz + cq);
+            }
+            pre += off;
+            cur = p;
+        }
+        uint32_t off = pre + 1u;
+        int32_t cand[4], at[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            cand[k] = __ldcg(io.cand + 4 * size_t(e) + k);
+            const int32_t cq = __ldcg(io.child_q + 4 * size_t(e) + k);
+            at[k] = -1;
+            if (cq < 0) continue;
+            at[k] = int32_t(off);
+            __stcg(io.acc + cq, (1ull << 63) | off);
+            off += __ldcg(io.sz + cq);
+        }
+        write_node4<NC>(io.n2, cand, at, pre, io.out4, io.map4);
+    }
+    if (!sync()) return false;
+    *total_out = end;
+    *depth_out = depth;
+    return true;
 }
 
 }  // namespace rq

@@ -278,7 +278,6 @@ int rq_batch_create(rq_ctx* ctx, const rq_mesh_desc* meshes, uint32_t num_meshes
         f.d_blocks = t.take<uint2>(f.blocks.size());
         f.d_tiles = t.take<rq_sort_tile>(f.tiles.size());
         f.d_seg_tiles = t.take<uint32_t>(f.seg_tiles.size());
-        f.d_order = t.take<uint32_t>(f.order.size());
     };
     tables(c);
     b->mem_bytes = c.off + 256;
@@ -308,13 +307,11 @@ int rq_batch_create(rq_ctx* ctx, const rq_mesh_desc* meshes, uint32_t num_meshes
     upload(f.d_blocks, f.blocks);
     upload(f.d_tiles, f.tiles);
     upload(f.d_seg_tiles, f.seg_tiles);
-    upload(f.d_order, f.order);
     // (the groups are what a launch needs on the host)
     f.segs = {};
     f.blocks = {};
     f.tiles = {};
     f.seg_tiles = {};
-    f.order = {};
     if (e == cudaSuccess) e = cudaMemset(b->d_counts, 0, sizeof(uint32_t) * 4 * num_meshes);
     if (e != cudaSuccess) {
         free_batch(b);

@@ -7,7 +7,9 @@
 // pre-order (a node precedes its subtree; inner children in slot order), so
 // the bytes equal fromBVH2's for the same binary BVH.
 //
-// One persistent cooperative launch, all blocks co-resident:
+// Trees in depth-first pre-order (every build's) are collapsed by treelets
+// (collapse_core.cuh).  Imported trees, whose nodes may lie in any order, by one
+// persistent cooperative launch, all blocks co-resident:
 //   phase 1  top-down, one grid barrier per 4-wide level (the narrow top
 //            levels by one block): candidates of each frontier node, inner
 //            candidates appended to a queue;
@@ -20,6 +22,7 @@
 #include <algorithm>
 
 #include "build_core.cuh"
+#include "collapse_core.cuh"
 #include "rq_device.cuh"
 #include "rq_internal.h"
 
@@ -69,7 +72,6 @@ __device__ bool grid_sync(uint32_t* ctl, uint32_t* err) {
 }
 
 __global__ void __launch_bounds__(kT) k_collapse(CollapseArgs A) {
-    __shared__ uint32_t s_lvl[kMaxLevels + 2];
     rq::CollapseIO io;
     io.n2 = A.n2;
     io.q = A.q;
@@ -84,7 +86,7 @@ __global__ void __launch_bounds__(kT) k_collapse(CollapseArgs A) {
     uint32_t total = 0, depth = 0;
     auto sync = [&]() { return grid_sync(A.ctl, A.err); };
     // levels of at most 256 entries by block 0 alone (measured: a little faster than a grid barrier each)
-    if (!rq::collapse_levels<true, false, 256>(io, blockIdx.x * kT + threadIdx.x, gridDim.x * kT, s_lvl, kMaxLevels,
+    if (!rq::collapse_levels<true, 256>(io, blockIdx.x * kT + threadIdx.x, gridDim.x * kT, kMaxLevels,
                                                sync, A.err, &total, &depth))
         return;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -92,6 +94,11 @@ __global__ void __launch_bounds__(kT) k_collapse(CollapseArgs A) {
         A.counts[2] = depth;
     }
 }
+
+struct OneTree {
+    rq::CollapseTree t;
+    __device__ const rq::CollapseTree& operator()(uint32_t) const { return t; }
+};
 
 }  // namespace
 
@@ -106,6 +113,16 @@ int rq_collapse_blocks(int device, int num_sms) {
 int rq_launch_collapse(rq_ctx* ctx, rq_bvh* bvh, BuildScratch& s, cudaStream_t st) {
     if (ctx->collapse_blocks <= 0) return rq_set_error(ctx, RQ_ERR_CUDA, "collapse kernel cannot be co-resident");
     cudaMemsetAsync(s.coll_ctl, 0, 256 * sizeof(uint32_t), st);
+    if (!bvh->foreign) {
+        // the node, leaf and centroid arrays of the build are free by now
+        OneTree t;
+        t.t = rq::CollapseTree{bvh->nodes2, bvh->nodes4, bvh->map4, bvh->d_counts, s.q, s.cpar, s.sz, s.cand, s.child_q,
+                               s.coll_ctl + 16, reinterpret_cast<uint4*>(s.box_in)};
+        const rq::Treelets T{s.coll_ctl, reinterpret_cast<uint4*>(s.cent), reinterpret_cast<uint4*>(s.box_lf),
+                             rq::kTreeletMax, ctx->d_err};
+        rq::launch_collapse(t, T, 1, ctx->num_sms, st);
+        return rq_cuda_status(ctx, cudaGetLastError(), "collapse launch");
+    }
     CollapseArgs a;
     a.n2 = bvh->nodes2;
     a.counts = bvh->d_counts;

@@ -6,9 +6,8 @@
 //
 // A build by one block or cluster per mesh, the form this replaces, was bound
 // by the largest meshes' chains of steps on one SM: 2.06 ms for 512 meshes of
-// 64 to 65,536 triangles (4.73M).  All meshes together take 0.94 ms: the tree
-// 0.28, the collapse (still a block per mesh: its levels are short) 0.26, the
-// sort 0.22, the node writes 0.07.
+// 64 to 65,536 triangles (4.73M).  All meshes together take 0.80 ms: the tree
+// 0.28, the sort 0.22, the collapse 0.13, the node writes 0.07.
 // Batches of more than kGroupTris triangles go in groups of whole meshes that
 // use the scratch in turn.
 #include <algorithm>
@@ -16,6 +15,7 @@
 #include <vector>
 
 #include "build_core.cuh"
+#include "collapse_core.cuh"
 #include "rq_batch.h"
 #include "rq_device.cuh"
 #include "rq_internal.h"
@@ -26,14 +26,13 @@ using namespace rq;
 
 constexpr int kT = 256;
 constexpr uint32_t kGroupTris = 16u << 20;
-constexpr uint32_t kMaxLevels = 120;
 static_assert(kTreeLeaves % kT == 0, "a block of elements is a block of leaves");
 
 struct ForestScratch {
     float4* cent;
     uint32_t* zero;     // zeroed per build, from here ...
     uint32_t* bounds;   // 6 per mesh: maxima of f2o, of ~f2o
-    uint32_t* misc;     // [0] walks, [1] scan ticket
+    uint32_t* misc;     // [0] unfinished nodes, [1] scan ticket, [2] treelets
     size_t zero_bytes;  // ... to here
     uint32_t *keys[2], *vals[2];
     uint32_t* counts;   // sort: 256 per tile
@@ -43,8 +42,7 @@ struct ForestScratch {
     uint2* top_list;
     uint32_t* q;
     int32_t *cand, *child_q;
-    uint32_t *sz, *par, *tail;
-    unsigned long long* acc;
+    uint32_t *sz, *end, *levels;
 };
 
 size_t carve(void* base, const rq_forest_group& g, ForestScratch& s) {
@@ -70,9 +68,8 @@ size_t carve(void* base, const rq_forest_group& g, ForestScratch& s) {
     s.cand = c.take<int32_t>(4 * N);
     s.child_q = c.take<int32_t>(4 * N);
     s.sz = c.take<uint32_t>(N);
-    s.par = c.take<uint32_t>(N);
-    s.tail = c.take<uint32_t>(16ull * g.segs);
-    s.acc = c.take<unsigned long long>(N);
+    s.end = c.take<uint32_t>(N);
+    s.levels = c.take<uint32_t>(size_t(kLevelWords) * g.segs);
     return c.off + 256;
 }
 
@@ -83,7 +80,6 @@ struct ForestArgs {
     uint32_t max_leaf;
     const rq_forest_seg* segs;
     const uint2* blocks;   // (segment, first element)
-    const uint32_t* order; // segments, largest first
     rq_bvh2_node* nodes2;
     rq_triangle* tris;
     uint32_t *perm, *skeys;
@@ -194,35 +190,18 @@ __global__ void __launch_bounds__(kT) k_forest_emit(const __grid_constant__ Fore
     }
 }
 
-// A mesh's 4-wide collapse by one block, the largest meshes' blocks first.
-constexpr int kCollapseT = 1024;
-__global__ void __launch_bounds__(kCollapseT) k_forest_collapse(const __grid_constant__ ForestArgs A) {
-    __shared__ uint32_t s_lvl[kMaxLevels + 2];
-    const uint32_t seg = A.order[blockIdx.x];
-    const rq_forest_seg g = A.segs[seg];
-    CollapseIO io;
-    io.n2 = A.nodes2 + 2ull * g.tri;
-    io.q = A.s.q + g.first;
-    io.cand = A.s.cand + 4ull * g.first;
-    io.child_q = A.s.child_q + 4ull * g.first;
-    io.sz = A.s.sz + g.first;
-    io.par = A.s.par + g.first;
-    io.acc = A.s.acc + g.first;
-    io.tail = A.s.tail + 16ull * seg;
-    io.out4 = A.nodes4 + g.tri;
-    io.map4 = A.map4 + 4ull * g.tri;
-    uint32_t total = 0, depth = 0;
-    auto sync = [] {
-        __syncthreads();
-        return true;
-    };
-    if (collapse_levels<true, true, 0>(io, threadIdx.x, kCollapseT, s_lvl, kMaxLevels, sync, A.err, &total, &depth) &&
-        threadIdx.x == 0) {
-        A.counts[4ull * g.mesh + 1] = total;
-        A.counts[4ull * g.mesh + 2] = depth;
+// The meshes as the collapse sees them.
+struct ForestTrees {
+    ForestArgs A;
+    __device__ CollapseTree operator()(uint32_t seg) const {
+        const rq_forest_seg g = A.segs[seg];
+        const size_t o = g.first;
+        return CollapseTree{A.nodes2 + 2ull * g.tri, A.nodes4 + g.tri,   A.map4 + 4ull * g.tri, A.counts + 4ull * g.mesh,
+                            A.s.q + o,               A.s.end + o,        A.s.sz + o,            A.s.cand + 4 * o,
+                            A.s.child_q + 4 * o,     A.s.levels + size_t(kLevelWords) * seg,
+                            reinterpret_cast<uint4*>(A.s.rec) + 2 * o};
     }
-}
-
+};
 }  // namespace
 
 void rq_forest_plan(const std::vector<rq_mesh_desc>& meshes, rq_forest& f) {
@@ -233,13 +212,6 @@ void rq_forest_plan(const std::vector<rq_mesh_desc>& meshes, rq_forest& f) {
     rq_forest_group g{};
     auto close = [&] {
         if (!g.segs) return;
-        // segments, largest first
-        const size_t o = f.order.size();
-        f.order.resize(o + g.segs);
-        std::iota(f.order.begin() + o, f.order.end(), 0u);
-        std::stable_sort(f.order.begin() + o, f.order.end(), [&](uint32_t a, uint32_t b) {
-            return f.segs[g.seg0 + a].n > f.segs[g.seg0 + b].n;
-        });
         f.seg_tiles.push_back(g.tiles);
         f.groups.push_back(g);
     };
@@ -284,7 +256,6 @@ int rq_launch_batch_build(rq_ctx* ctx, rq_batch* b, const float* pos, uint32_t s
         a.max_leaf = b->max_leaf;
         a.segs = f.d_segs + g.seg0;
         a.blocks = f.d_blocks + g.block0;
-        a.order = f.d_order + g.seg0;
         a.nodes2 = b->nodes2;
         a.tris = b->tris;
         a.perm = b->perm;
@@ -307,7 +278,11 @@ int rq_launch_batch_build(rq_ctx* ctx, rq_batch* b, const float* pos, uint32_t s
         k_forest_tree_top<<<uint32_t(ctx->num_sms) * 4u, kT, 0, st>>>(a);
         rq_launch_scan(ctx, a.s.ch, a.s.a, g.tris, a.s.scan_status, a.s.misc + 1, st);
         k_forest_emit<<<g.blocks, kT, 0, st>>>(a);
-        k_forest_collapse<<<g.segs, kCollapseT, 0, st>>>(a);
+        // (the tree's records and the centroids are free by now)
+        launch_collapse(ForestTrees{a},
+                        Treelets{a.s.misc + 2, reinterpret_cast<uint4*>(a.s.cent), reinterpret_cast<uint4*>(a.s.leaf),
+                                 kTreeletMax, a.err},
+                        g.segs, ctx->num_sms, st);
         e = cudaGetLastError();
         if (e != cudaSuccess) return rq_cuda_status(ctx, e, "batch build launch");
     }

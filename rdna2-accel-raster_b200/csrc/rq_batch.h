@@ -30,12 +30,10 @@ struct rq_forest {
     std::vector<uint2> blocks;        // (segment in the group, first element)
     std::vector<rq_sort_tile> tiles;
     std::vector<uint32_t> seg_tiles;
-    std::vector<uint32_t> order;      // a group's segments, largest first
     rq_forest_seg* d_segs = nullptr;
     uint2* d_blocks = nullptr;
     rq_sort_tile* d_tiles = nullptr;
     uint32_t* d_seg_tiles = nullptr;
-    uint32_t* d_order = nullptr;
 };
 void rq_forest_plan(const std::vector<rq_mesh_desc>& meshes, rq_forest& f);
 size_t rq_forest_scratch_bytes(const rq_forest& f);

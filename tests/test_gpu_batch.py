@@ -207,3 +207,32 @@ def test_batch_mesh_sizes_and_places(ctx):
                 assert g.tobytes() == w.tobytes(), (nt, name)
             s.destroy()
         b.destroy()
+
+
+@pytest.mark.parametrize("max_leaf", [1, 16])
+def test_batch_collapse_treelets(ctx, max_leaf):
+    """Trees of 2,047, 2,049 and more binary nodes (a subtree of at most 2,048 is collapsed by one block), evenly spread
+    and as a chain of ever smaller clusters."""
+    rng = np.random.default_rng(8)
+    pos_l, descs, v, t = [], [], 0, 0
+    for n in (1, 2, 1023, 1024, 1025, 1026, 4097, 30000):
+        for skew in (False, True):
+            c = rng.uniform(0, 1, (n, 1, 3))
+            if skew:
+                c = c * 0.5 ** rng.integers(0, 10, (n, 1, 1))
+            pos_l.append((c + rng.uniform(0, 1e-3, (n, 3, 3))).astype(np.float32).reshape(-1, 3))
+            descs.append((v, 3 * n, t, n))
+            v, t = v + 3 * n, t + n
+    pos = np.concatenate(pos_l)
+    idx = np.concatenate([np.arange(3 * d[3], dtype=np.int32).reshape(-1, 3) for d in descs])
+    p, i = torch.from_numpy(pos).cuda(), torch.from_numpy(idx).cuda()
+    b = rq.Batch(ctx, descs, max_leaf=max_leaf)
+    b.build(p, i)
+    ctx.sync_check()
+    for m, (vo, nv, to, nt) in enumerate(descs):
+        o = O.lbvh_build(pos[vo:vo + nv].reshape(-1), None, max_leaf)
+        g = b.download(m)
+        for a, name in zip(g, ("nodes2", "tris", "nodes4")):
+            assert a.tobytes() == o[name].tobytes(), (nt, name)
+        assert np.array_equal(g[3], o["sorted"])
+    b.destroy()
