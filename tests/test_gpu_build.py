@@ -71,6 +71,15 @@ def test_small_build_parity(ctx, n, max_leaf):
     assert_same_as_oracle(ctx, soup(n, 400 + n), None, max_leaf)
 
 
+@pytest.mark.parametrize("n", [4194303, 4194304, 4202497])
+def test_scan_forms_parity(ctx, n):
+    """Both sides of the length where the emission counts' scan takes larger tiles, and a last tile of one."""
+    pos = soup(n, 31)
+    b = rq.Bvh.build(ctx, torch.from_numpy(pos).cuda(), None)
+    assert b.download()[0].tobytes() == O.lbvh_build(pos.reshape(-1), None)["nodes2"].tobytes()
+    b.destroy()
+
+
 @pytest.mark.parametrize("equal", [0, 3000, 1 << 30])
 @pytest.mark.parametrize("n,max_leaf", [(5119, 1), (5120, 4), (5121, 16), (6145, 2), (9217, 3)])
 def test_tree_blocks_parity(ctx, n, max_leaf, equal):
