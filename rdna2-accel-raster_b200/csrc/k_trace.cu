@@ -61,20 +61,20 @@ struct BufSrc {
     }
 };
 
-// `max_depth`: levels the stack's `rows` entries cover.
+// `max_depth`: levels the stack's `rows` entries cover.  lanes: rays that share a warp.
 template <bool ANY, bool MT, bool STATS, bool BARY, bool WIDE>
 __global__ void __launch_bounds__(kT, kTraceBlocksPerSm) k_trace4(const rq_bvh4_node* __restrict__ nodes,
                                                const rq_triangle* __restrict__ tris,
                                                const __grid_constant__ BufSrc<STATS, BARY> src,
                                                const uint32_t* __restrict__ counts, uint32_t* ctr, uint32_t* err,
-                                               int rows, uint32_t max_depth) {
+                                               int rows, uint32_t max_depth, uint32_t lanes) {
     extern __shared__ __align__(16) char s_stack[];
     // the rows were picked from the host's copy of the depth; the live depth
     // (after an in-place rebuild) must still fit
     if (blockIdx.x == 0 && threadIdx.x == 0 && __ldg(counts + 2) > max_depth) rq::set_err(err, RQ_DERR_STACK);
     using Entry = typename rq::OpenNode<ANY, WIDE>::Entry;
     rq::trace_persistent<ANY, MT, STATS, kT, const BufSrc<STATS, BARY>, 32, WIDE>(
-        nodes, tris, src, ctr, reinterpret_cast<Entry*>(s_stack) + threadIdx.x, rows, err, kTraceRefill);
+        nodes, tris, src, ctr, reinterpret_cast<Entry*>(s_stack) + threadIdx.x, rows, err, lanes == 32u ? kTraceRefill : 1, lanes);
 }
 
 // One ray per thread over a RADV image.  Open nodes as in trace_engine.cuh: one
@@ -363,9 +363,17 @@ cudaError_t launch4(rq_ctx* ctx, const rq_bvh* b, const rq_ray* rays, uint32_t n
     auto kern = wide ? k_trace4<ANY, MT, EX, EX, !ANY> : k_trace4<ANY, MT, EX, EX, false>;
     const int rows = int(max_depth) + 2;
     const size_t smem = size_t(rows) * kT * (wide ? 8 : 4);
-    // persistent grid: every SM filled, never more blocks than 32-ray chunks
+    // persistent grid: every SM filled, never more blocks than there are chunks
     uint32_t blocks = uint32_t(ctx->num_sms) * uint32_t(wide && rows > 24 ? 4 : kTraceBlocksPerSm);
-    const uint32_t need = (n + kT - 1) / kT;
+    // A batch of less than one ray per resident lane takes the time of its
+    // slowest warp, whose length grows with the rays that share it: it is
+    // spread over all the warps there are, at 4, 8 or 16 rays each (999,698
+    // triangles, closest hit, us at 32 -> fewer: 8,192 rays 108 -> 74, 32,768
+    // 106 -> 94, 65,536 108 -> 100; 99,458 triangles 62 -> 45, 59 -> 53, 59 -> 61).
+    const uint32_t warps = blocks * (kT / 32);
+    uint32_t lanes = 4;
+    while (lanes < 32u && n > lanes * warps) lanes *= 2;
+    const uint32_t need = (n + (kT / 32) * lanes - 1) / ((kT / 32) * lanes);
     if (blocks > need) blocks = need;
     BufSrc<EX, EX> src;
     src.total = n;
@@ -376,7 +384,7 @@ cudaError_t launch4(rq_ctx* ctx, const rq_bvh* b, const rq_ray* rays, uint32_t n
     src.stats = stats;
     cudaError_t e = cudaMemsetAsync(ctx->d_ctr, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    kern<<<blocks, kT, smem, st>>>(b->nodes4, b->tris, src, b->d_counts, ctx->d_ctr, ctx->d_err, rows, max_depth);
+    kern<<<blocks, kT, smem, st>>>(b->nodes4, b->tris, src, b->d_counts, ctx->d_ctr, ctx->d_err, rows, max_depth, lanes);
     return cudaGetLastError();
 }
 

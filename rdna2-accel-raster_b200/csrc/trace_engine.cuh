@@ -170,12 +170,15 @@ constexpr int kFewSearch = 8, kLeafWait = 8;
 // stk: this lane's column of `rows` stack entries, STRIDE apart.  CHUNK: ray
 // ids taken per atomic.  refill_min: idle lanes get new rays only once at
 // least this many lanes of the warp are idle (or all are), so that lanes join
-// in groups and a warp's rays stay closer in position and direction.
+// in groups and a warp's rays stay closer in position and direction.  lanes:
+// lanes of a warp that take rays, as many ids at a time (32: all, CHUNK ids).
 template <int ANY, bool MT, bool STATS, int STRIDE, class Src, int CHUNK = int(kChunk), bool WIDE = false>
 __device__ __forceinline__ void trace_persistent(const rq_bvh4_node* __restrict__ nodes,
                                                  const rq_triangle* __restrict__ tris, Src& src, uint32_t* ctr,
                                                  typename OpenNode<ANY == 1, WIDE>::Entry* stk, int rows,
-                                                 uint32_t* err, int refill_min = 1) {
+                                                 uint32_t* err, int refill_min = 1, uint32_t lanes = 32u) {
+    const uint32_t takers = lanes == 32u ? kFull : (1u << lanes) - 1u;
+    const uint32_t chunk = lanes == 32u ? uint32_t(CHUNK) : lanes;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
     // warp-uniform chunk of ray ids
@@ -201,19 +204,19 @@ __device__ __forceinline__ void trace_persistent(const rq_bvh4_node* __restrict_
 
     for (;;) {
         // ---- new rays for idle lanes, once refill_min of them are idle
-        uint32_t idle = __ballot_sync(kFull, !active);
-        const bool go = __popc(idle) >= refill_min || idle == kFull;
+        uint32_t idle = __ballot_sync(kFull, !active) & takers;
+        const bool go = __popc(idle) >= refill_min || idle == takers;
         while (go && idle && !exhausted) {
             if (next == end) {
                 uint32_t base = 0;
-                if (lane == 0) base = atomicAdd(ctr, uint32_t(CHUNK));
+                if (lane == 0) base = atomicAdd(ctr, chunk);
                 base = __shfl_sync(kFull, base, 0);
                 if (base >= src.total) {
                     exhausted = true;
                     break;
                 }
                 next = base;
-                end = min(base + uint32_t(CHUNK), src.total);
+                end = min(base + chunk, src.total);
             }
             const uint32_t take = min(uint32_t(__popc(idle)), end - next);
             const uint32_t rank = __popc(idle & lt_mask);
@@ -241,7 +244,7 @@ __device__ __forceinline__ void trace_persistent(const rq_bvh4_node* __restrict_
             next += take;
             // lanes whose id made no ray (a light behind the surface, an
             // empty pixel) take the next id at once
-            idle = __ballot_sync(kFull, !active);
+            idle = __ballot_sync(kFull, !active) & takers;
         }
         if (!__any_sync(kFull, active)) {
             if (exhausted) break;

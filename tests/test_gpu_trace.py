@@ -225,3 +225,19 @@ def test_handle_with_room_for_many_nodes(ctx):
     ctx.sync_check()
     for h in (ta, tb, roomy, own):
         h.destroy()
+
+
+@pytest.mark.parametrize("any_hit", [False, True])
+@pytest.mark.parametrize("n", [1, 5, 18943, 18944, 18945, 37889, 75776, 75777])
+def test_small_batches_fill_few_lanes(ctx, n, any_hit):
+    """Batches on both sides of the sizes where 4, 8, 16 or 32 rays share a warp (4,736 warps on 148 SMs)."""
+    pos, idx = rq.scene_grid(40, 40, seed=2)
+    b = rq.Bvh.build(ctx, torch.from_numpy(pos).cuda(), torch.from_numpy(idx.view(np.int32)).cuda())
+    rays = rq.scene_rays_down(n, -1.0, 1.0, -1.0, 1.0, 2.0, 0.3, 0.01, 1000.0, 5)
+    flags = rq.RQ_TRACE_ANY if any_hit else 0
+    hits, _, _ = rq.trace(ctx, b, torch.from_numpy(rays).cuda(), flags=flags)
+    ctx.sync_check()
+    o = O.lbvh_build(pos.reshape(-1), idx.reshape(-1))
+    want, _, _ = O.trace_bvh4(o["nodes4"], o["tris"], o["sorted"], rays, flags=flags)
+    assert hits.cpu().numpy().tobytes() == want.tobytes()
+    b.destroy()
