@@ -23,6 +23,7 @@ constexpr int kT = 128;
 // triangles, incoherent).
 constexpr int kTraceRefill = 16;
 constexpr int kTraceBlocksPerSm = 8;
+constexpr uint32_t kSmallTree = 4096;  // 4-wide nodes
 
 __device__ __forceinline__ void store_miss(rq_hit* hits, uint32_t i) {
     reinterpret_cast<uint4*>(hits)[i] = make_uint4(0u, __float_as_uint(-1.0f), 0xffffffffu, 0xffffffffu);
@@ -62,19 +63,21 @@ struct BufSrc {
 };
 
 // `max_depth`: levels the stack's `rows` entries cover.  lanes: rays that share a warp.
+// few: trace_persistent's.
 template <bool ANY, bool MT, bool STATS, bool BARY, bool WIDE>
 __global__ void __launch_bounds__(kT, kTraceBlocksPerSm) k_trace4(const rq_bvh4_node* __restrict__ nodes,
                                                const rq_triangle* __restrict__ tris,
                                                const __grid_constant__ BufSrc<STATS, BARY> src,
                                                const uint32_t* __restrict__ counts, uint32_t* ctr, uint32_t* err,
-                                               int rows, uint32_t max_depth, uint32_t lanes) {
+                                               int rows, uint32_t max_depth, uint32_t lanes, int few) {
     extern __shared__ __align__(16) char s_stack[];
     // the rows were picked from the host's copy of the depth; the live depth
     // (after an in-place rebuild) must still fit
     if (blockIdx.x == 0 && threadIdx.x == 0 && __ldg(counts + 2) > max_depth) rq::set_err(err, RQ_DERR_STACK);
     using Entry = typename rq::OpenNode<ANY, WIDE>::Entry;
     rq::trace_persistent<ANY, MT, STATS, kT, const BufSrc<STATS, BARY>, 32, WIDE>(
-        nodes, tris, src, ctr, reinterpret_cast<Entry*>(s_stack) + threadIdx.x, rows, err, lanes == 32u ? kTraceRefill : 1, lanes);
+        nodes, tris, src, ctr, reinterpret_cast<Entry*>(s_stack) + threadIdx.x, rows, err,
+        lanes == 32u ? kTraceRefill : 1, lanes, few);
 }
 
 // One ray per thread over a RADV image.  Open nodes as in trace_engine.cuh: one
@@ -373,6 +376,11 @@ cudaError_t launch4(rq_ctx* ctx, const rq_bvh* b, const rq_ray* rays, uint32_t n
     const uint32_t warps = blocks * (kT / 32);
     uint32_t lanes = 4;
     while (lanes < 32u && n > lanes * warps) lanes *= 2;
+    // On small trees a node phase is a few steps, and leaving it early costs more
+    // than the idle lanes do (2^20 rays, us with and without: 968 triangles
+    // incoherent 166 / 156, coherent 101 / 98, 8,192 coherent 113 / 110; 99,458
+    // equal; 999,698 incoherent 419 / 432).
+    const int few = b->h_counts[1] <= kSmallTree ? 0 : rq::kFewSearch;
     const uint32_t need = (n + (kT / 32) * lanes - 1) / ((kT / 32) * lanes);
     if (blocks > need) blocks = need;
     BufSrc<EX, EX> src;
@@ -384,7 +392,8 @@ cudaError_t launch4(rq_ctx* ctx, const rq_bvh* b, const rq_ray* rays, uint32_t n
     src.stats = stats;
     cudaError_t e = cudaMemsetAsync(ctx->d_ctr, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    kern<<<blocks, kT, smem, st>>>(b->nodes4, b->tris, src, b->d_counts, ctx->d_ctr, ctx->d_err, rows, max_depth, lanes);
+    kern<<<blocks, kT, smem, st>>>(b->nodes4, b->tris, src, b->d_counts, ctx->d_ctr, ctx->d_err, rows, max_depth,
+                                   lanes, few);
     return cudaGetLastError();
 }
 

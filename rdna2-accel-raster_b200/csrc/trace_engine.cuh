@@ -164,7 +164,8 @@ __device__ __forceinline__ void child_of(const rq_bvh4_node* __restrict__ nodes,
 // Leaves of the node phase: it ends once at most kFewSearch lanes search while
 // kLeafWait hold a leaf (measured on B200: 8 and 8; without it the 1080p
 // frame's shadow pass was 3 %, the depth-AO pass 13 % slower, 16 and 8 were
-// 3 % and 4 % slower than 8 and 8).
+// 3 % and 4 % slower than 8 and 8).  few: kFewSearch, or 0 where the whole phase
+// is short.
 constexpr int kFewSearch = 8, kLeafWait = 8;
 
 // stk: this lane's column of `rows` stack entries, STRIDE apart.  CHUNK: ray
@@ -176,7 +177,8 @@ template <int ANY, bool MT, bool STATS, int STRIDE, class Src, int CHUNK = int(k
 __device__ __forceinline__ void trace_persistent(const rq_bvh4_node* __restrict__ nodes,
                                                  const rq_triangle* __restrict__ tris, Src& src, uint32_t* ctr,
                                                  typename OpenNode<ANY == 1, WIDE>::Entry* stk, int rows,
-                                                 uint32_t* err, int refill_min = 1, uint32_t lanes = 32u) {
+                                                 uint32_t* err, int refill_min = 1, uint32_t lanes = 32u,
+                                                 int few = kFewSearch) {
     const uint32_t takers = lanes == 32u ? kFull : (1u << lanes) - 1u;
     const uint32_t chunk = lanes == 32u ? uint32_t(CHUNK) : lanes;
     const uint32_t lane = threadIdx.x & 31u;
@@ -257,7 +259,7 @@ __device__ __forceinline__ void trace_persistent(const rq_bvh4_node* __restrict_
             const bool search = active && leaf == kNoLeaf && (top.left != 0u || sp > 0);
             const uint32_t sm = __ballot_sync(kFull, search);
             if (!sm) break;
-            if (__popc(sm) <= kFewSearch && __popc(__ballot_sync(kFull, leaf != kNoLeaf)) >= kLeafWait) break;
+            if (__popc(sm) <= few && __popc(__ballot_sync(kFull, leaf != kNoLeaf)) >= kLeafWait) break;
             if (!search) continue;
             if (top.left == 0u) top.unpack(stk[(--sp) * STRIDE]);
             const uint32_t slot = top.take();
