@@ -124,7 +124,7 @@ int rq_deform_wave_step(rq_ctx* ctx, const float* base, float* out, uint32_t num
                         uint32_t* state, float dt, float amp, float freq, rq_stream stream);
 
 /* ------------------------------------------------------------------ */
-/* BVH build (LBVH: Morton codes, onesweep radix sort, Karras emission, */
+/* BVH build (LBVH: Morton codes, radix sort, radix tree from the leaves up, */
 /* atomic bottom-up refit, BVH4 collapse)                              */
 /* ------------------------------------------------------------------ */
 
