@@ -236,3 +236,21 @@ def test_batch_collapse_treelets(ctx, max_leaf):
             assert a.tobytes() == o[name].tobytes(), (nt, name)
         assert np.array_equal(g[3], o["sorted"])
     b.destroy()
+
+
+def test_batch_groups(ctx):
+    """More triangles than one group of meshes holds (16,777,216): meshes of both groups equal a build of their own."""
+    pos, idx = rq.scene_grid(1000, 500, seed=6)
+    n, count = len(idx), 17
+    p = torch.from_numpy(pos).cuda()
+    i = torch.from_numpy(idx.view(np.int32)).cuda()
+    b = rq.Batch(ctx, [(0, len(pos), k * n, n) for k in range(count)])
+    b.build(p, i.repeat(count, 1))
+    ctx.sync_check()
+    s = rq.Bvh.build(ctx, p, i)
+    want = s.download()
+    for m in (0, 15, 16):
+        for g, w in zip(b.download(m), want):
+            assert g.tobytes() == w.tobytes(), m
+    s.destroy()
+    b.destroy()
