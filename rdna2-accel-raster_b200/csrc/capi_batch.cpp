@@ -313,6 +313,10 @@ int rq_batch_create(rq_ctx* ctx, const rq_mesh_desc* meshes, uint32_t num_meshes
     f.tiles = {};
     f.seg_tiles = {};
     if (e == cudaSuccess) e = cudaMemset(b->d_counts, 0, sizeof(uint32_t) * 4 * num_meshes);
+    // Copies from pageable memory and fills return once they are queued on the
+    // legacy stream, which a non-blocking stream does not wait for: without
+    // this wait a first rq_batch_build there could read tables not yet written.
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
         free_batch(b);
         delete b;

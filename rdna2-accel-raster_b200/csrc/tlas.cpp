@@ -99,7 +99,9 @@ int build(rq_ctx* ctx, const rq_instance* instances, uint32_t n, rq_tlas** out, 
     if (e == cudaSuccess) {
         t->d_fwd = reinterpret_cast<float*>(reinterpret_cast<char*>(t->d_inst) + inst_bytes);
         t->d_tri9 = t->d_fwd + 12ull * n;
-        e = cudaMemcpy(t->d_inst, table.data(), inst_bytes + fwd_bytes, cudaMemcpyHostToDevice);
+        // on `st`, where k_instance_boxes follows (pageable memory is staged
+        // before the call returns, so the table may go)
+        e = cudaMemcpyAsync(t->d_inst, table.data(), inst_bytes + fwd_bytes, cudaMemcpyHostToDevice, st);
     }
     int rc = e == cudaSuccess ? RQ_OK : rq_cuda_status(ctx, e, "instance table");
     if (rc == RQ_OK) rc = rq_launch_instance_boxes(ctx, t->d_inst, t->d_fwd, n, t->d_tri9, st);
