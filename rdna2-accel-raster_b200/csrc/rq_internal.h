@@ -27,6 +27,9 @@
 // Largest triangle count a leaf stack entry can address (27-bit first prim).
 #define RQ_MAX_TRIANGLES (1u << 27)
 
+// Largest leaf a traversal's parked leaf can hold (4 bits of count).
+#define RQ_MAX_LEAF 16u
+
 // 4-wide nodes a closest-hit traversal's 32-bit stack entry can name (23 bits
 // beside 9 of child order); trees with room for more use 64-bit entries.
 #define RQ_NARROW_NODES (1u << 23)

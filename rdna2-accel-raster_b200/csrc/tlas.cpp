@@ -71,6 +71,8 @@ int build(rq_ctx* ctx, const rq_instance* instances, uint32_t n, rq_tlas** out, 
             rq_bvh_info inf{};
             int rc = rq_bvh_info_get(const_cast<rq_bvh*>(s.blas), &inf);
             if (rc) return rc;
+            if (inf.max_leaf > RQ_MAX_LEAF)  // (median splits stop at coincident centroids)
+                return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "instance BLAS with a leaf of more than 16 primitives");
             seen = depths.emplace(s.blas, inf.depth4).first;
         }
         if (!s.blas->has4 || s.blas->device != ctx->device)

@@ -117,3 +117,28 @@ def test_tlas_instance_forms(ctx):
     for g in got[1:]:
         assert torch.equal(g, got[0])
     assert int(got[0][:, 0].sum()) > 0
+
+
+def coincident(n):
+    """n unit triangles in one place: a median build's single leaf."""
+    return np.tile(np.array([[-1, -1, 0], [1, -1, 0], [0, 1, 0]], np.float32), (n, 1))
+
+
+@pytest.mark.parametrize("n", [16, 17])
+def test_tlas_refuses_leaves_it_cannot_hold(ctx, n):
+    """Coincident centroids stop a median split, so its leaves have any size: 16 triangles is the traversal's largest."""
+    b = rq.Bvh.build(ctx, torch.from_numpy(coincident(n)).cuda(), median=True)
+    assert b.info()["max_leaf"] == n
+    eye = np.hstack([np.eye(3), np.zeros((3, 1))]).astype(np.float32)
+    if n > 16:
+        with pytest.raises(rq.RqError) as e:
+            rq.Tlas(ctx, [(eye, 7, 0xFF, b)])
+        assert e.value.status == rq.RQ_ERR_UNSUPPORTED
+    else:
+        ray = torch.tensor([[0, 0, -1, 0, 0, 0, 1, 10]], dtype=torch.float32, device="cuda")
+        t = rq.Tlas(ctx, [(eye, 7, 0xFF, b)])
+        got = rq.hits_numpy(t.trace(ray))[0]
+        ctx.sync_check()
+        assert (got["hit"], got["t"], got["instance_id"]) == (1, 1.0, 7)
+        t.destroy()
+    b.destroy()
