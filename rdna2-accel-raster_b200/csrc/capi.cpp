@@ -194,6 +194,8 @@ int rq_ctx_check(rq_ctx* ctx, rq_stream stream) {
     cudaMemset(ctx->d_err, 0, sizeof(uint32_t));
     if (w == RQ_DERR_STACK)
         return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "traversal stack too small for the tree's live depth");
+    if (!(w & ~(RQ_DERR_STACK | RQ_DERR_LEAF)))
+        return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "rebuilt tree has a leaf with more than 16 primitives");
     if (w == RQ_DERR_RADV_IMAGE)
         return rq_set_error(ctx, RQ_ERR_STATE, "rq_refit_radv: the image was not built for this triangle count");
     return rq_set_error(ctx, RQ_ERR_DEVICE_TIMEOUT, "device error word 0x" + std::to_string(w));
@@ -415,7 +417,7 @@ int rq_bvh_import4(rq_ctx* ctx, const rq_bvh4_node* nodes, uint32_t num_nodes, c
     b->last_stream = st;
     rc = rq_launch_analyze4(ctx, b, st);
     if (rc == RQ_OK) rc = sync_counts(b);
-    if (rc == RQ_OK && b->h_counts[3] > 16)
+    if (rc == RQ_OK && b->h_counts[3] > RQ_MAX_LEAF)
         rc = rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "leaf with more than 16 primitives");
     if (rc) {
         rq_bvh_destroy(b);
@@ -506,7 +508,8 @@ int rq_trace(rq_ctx* ctx, const rq_bvh* bvh, const rq_ray* rays, uint32_t n, uin
         int rc = sync_counts(const_cast<rq_bvh*>(bvh));
         if (rc) return rc;
     }
-    if (bvh->h_counts[3] > 16) return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "leaf with more than 16 primitives");
+    if (bvh->h_counts[3] > RQ_MAX_LEAF)
+        return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "leaf with more than 16 primitives");
     return rq_launch_trace(ctx, bvh, rays, n, flags, hits, bary, stats, S(stream));
 }
 
@@ -542,7 +545,8 @@ static int frame_checks(rq_ctx* ctx, const rq_bvh* bvh) {
         int rc = sync_counts(const_cast<rq_bvh*>(bvh));
         if (rc) return rc;
     }
-    if (bvh->h_counts[3] > 16) return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "leaf with more than 16 primitives");
+    if (bvh->h_counts[3] > RQ_MAX_LEAF)
+        return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "leaf with more than 16 primitives");
     if (3u * bvh->h_counts[2] + 1u > 128u)
         return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "4-wide tree deeper than 42 levels");
     return RQ_OK;

@@ -230,8 +230,10 @@ __global__ void __launch_bounds__(kT) k_gbuffer_seq(const rq_bvh4_node* __restri
 template <bool MT, int TT, int REGS, bool WIDE>
 __global__ void __launch_bounds__(TT, 65536 / (TT * REGS))
     k_gbuffer_eng(const rq_bvh4_node* __restrict__ nodes, const rq_triangle* __restrict__ tris,
-                  const __grid_constant__ GbufSrc src0, uint32_t* ctr, uint32_t* err, int rows, int refill_min) {
+                  const uint32_t* __restrict__ counts, const __grid_constant__ GbufSrc src0, uint32_t* ctr,
+                  uint32_t* err, int rows, int refill_min) {
     extern __shared__ __align__(16) char s_stack[];
+    rq::check_leaves(counts, err);
     GbufSrc src = src0;
     using Entry = typename rq::OpenNode<false, WIDE>::Entry;
     rq::trace_persistent<0, MT, false, TT, GbufSrc, 32, WIDE>(
@@ -245,10 +247,11 @@ __global__ void __launch_bounds__(TT, 65536 / (TT * REGS))
 template <bool MT, bool STATS, int TT, int CHUNK, int REGS>
 __global__ void __launch_bounds__(TT, 65536 / (TT * (REGS ? REGS : 65536 / TT)))
     k_shadow_ao(const rq_bvh4_node* __restrict__ nodes, const rq_triangle* __restrict__ tris,
-                const rq_gbuffer_px* __restrict__ gbuf, const __grid_constant__ ShadeArgs sa,
-                unsigned long long* words, unsigned long long* counters, uint32_t* ctr, uint32_t* err, int rows,
-                int refill_min) {
+                const uint32_t* __restrict__ counts, const rq_gbuffer_px* __restrict__ gbuf,
+                const __grid_constant__ ShadeArgs sa, unsigned long long* words, unsigned long long* counters,
+                uint32_t* ctr, uint32_t* err, int rows, int refill_min) {
     extern __shared__ __align__(16) uint32_t s_entries[];
+    rq::check_leaves(counts, err);
     ShadeSrc<STATS> src;
     src.kinds = sa.nl + sa.spp;
     src.tiles_x = (sa.w + kTileW - 1) / kTileW;
@@ -328,8 +331,10 @@ struct ReflSrc {
 template <bool MT, int TT, int REGS, bool WIDE>
 __global__ void __launch_bounds__(TT, 65536 / (TT * REGS))
     k_reflect(const rq_bvh4_node* __restrict__ nodes, const rq_triangle* __restrict__ tris,
-              const __grid_constant__ ReflSrc src0, uint32_t* ctr, uint32_t* err, int rows) {
+              const uint32_t* __restrict__ counts, const __grid_constant__ ReflSrc src0, uint32_t* ctr, uint32_t* err,
+              int rows) {
     extern __shared__ __align__(16) char s_stack[];
+    rq::check_leaves(counts, err);
     ReflSrc src = src0;
     using Entry = typename rq::OpenNode<false, WIDE>::Entry;
     rq::trace_persistent<0, MT, false, TT, ReflSrc, 32, WIDE>(
@@ -409,9 +414,11 @@ struct AoDepthSrc {
 template <bool MT, int TT, int REGS>
 __global__ void __launch_bounds__(TT, 65536 / (TT * REGS))
     k_ao_depth(const rq_bvh4_node* __restrict__ nodes, const rq_triangle* __restrict__ tris,
-               const float* __restrict__ depth, const __grid_constant__ AoDepthArgs a, uint32_t* words,
+               const uint32_t* __restrict__ counts, const float* __restrict__ depth,
+               const __grid_constant__ AoDepthArgs a, uint32_t* words,
                unsigned long long* counters, uint32_t* ctr, uint32_t* err, int rows) {
     extern __shared__ __align__(16) uint32_t s_entries[];
+    rq::check_leaves(counts, err);
     AoDepthSrc src;
     src.tiles_x = (a.w + kTileW - 1) / kTileW;
     src.total = src.tiles_x * ((a.h + kTileH - 1) / kTileH) * a.spp * 32u;
@@ -521,10 +528,11 @@ int rq_launch_gbuffer(rq_ctx* ctx, const rq_bvh* bvh, const rq_camera& cam, rq_g
         if (e == cudaSuccess) {
             const rq_bvh4_node* nodes = bvh->nodes4;
             const rq_triangle* tris = bvh->tris;
+            const uint32_t* counts = bvh->d_counts;
             uint32_t* ctr = ctx->d_ctr;
             uint32_t* err = ctx->d_err;
             int rm = int(ctx->camera.refill_min);
-            void* args[] = {&nodes, &tris, &src, &ctr, &err, &rows, &rm};
+            void* args[] = {&nodes, &tris, &counts, &src, &ctr, &err, &rows, &rm};
             e = cudaLaunchKernel(k, dim3(blocks), dim3(kET), args, smem, st);
         }
         return rq_cuda_status(ctx, e, "gbuffer launch");
@@ -580,9 +588,10 @@ int rq_launch_shadow_ao(rq_ctx* ctx, const rq_bvh* bvh, const rq_gbuffer_px* gbu
             const uint32_t blocks = uint32_t(ctx->num_sms) * uint32_t(per_sm > 0 ? per_sm : 1);
             const rq_bvh4_node* nodes = bvh->nodes4;
             const rq_triangle* tris = bvh->tris;
+            const uint32_t* counts = bvh->d_counts;
             uint32_t* err = ctx->d_err;
             int refill_min = int(shape.refill_min ? shape.refill_min : 1u);
-            void* args[] = {&nodes, &tris, &gbuf, &s, &words, &counter, &ctr, &err, &rows, &refill_min};
+            void* args[] = {&nodes, &tris, &counts, &gbuf, &s, &words, &counter, &ctr, &err, &rows, &refill_min};
             e = cudaLaunchKernel(k, dim3(blocks), dim3(shape.threads), args, smem, st);
         }
     }
@@ -627,9 +636,10 @@ int rq_launch_reflect(rq_ctx* ctx, const rq_bvh* bvh, const rq_gbuffer_px* gbuf,
     if (e == cudaSuccess) {
         const rq_bvh4_node* nodes = bvh->nodes4;
         const rq_triangle* tris = bvh->tris;
+        const uint32_t* counts = bvh->d_counts;
         uint32_t* ctr = ctx->d_ctr;
         uint32_t* err = ctx->d_err;
-        void* args[] = {&nodes, &tris, &src, &ctr, &err, &rows};
+        void* args[] = {&nodes, &tris, &counts, &src, &ctr, &err, &rows};
         e = cudaLaunchKernel(k, dim3(blocks), dim3(kReflThreads), args, smem, st);
     }
     return rq_cuda_status(ctx, e, "reflection launch");
@@ -664,9 +674,10 @@ int rq_launch_ao_depth(rq_ctx* ctx, const rq_bvh* bvh, const float* depth, const
     if (e == cudaSuccess) {
         const rq_bvh4_node* nodes = bvh->nodes4;
         const rq_triangle* tris = bvh->tris;
+        const uint32_t* counts = bvh->d_counts;
         uint32_t* ctr = ctx->d_ctr;
         uint32_t* err = ctx->d_err;
-        void* args[] = {&nodes, &tris, &depth, &a, &words, &counters, &ctr, &err, &rows};
+        void* args[] = {&nodes, &tris, &counts, &depth, &a, &words, &counters, &ctr, &err, &rows};
         e = cudaLaunchKernel(k, dim3(blocks), dim3(kAoThreads), args, smem, st);
     }
     if (e == cudaSuccess) {

@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(kT, kTraceBlocksPerSm) k_trace4(const rq_bvh4_
     // the rows were picked from the host's copy of the depth; the live depth
     // (after an in-place rebuild) must still fit
     if (blockIdx.x == 0 && threadIdx.x == 0 && __ldg(counts + 2) > max_depth) rq::set_err(err, RQ_DERR_STACK);
+    rq::check_leaves(counts, err);
     using Entry = typename rq::OpenNode<ANY, WIDE>::Entry;
     rq::trace_persistent<ANY, MT, STATS, kT, const BufSrc<STATS, BARY>, 32, WIDE>(
         nodes, tris, src, ctr, reinterpret_cast<Entry*>(s_stack) + threadIdx.x, rows, err,

@@ -18,6 +18,7 @@
 #define RQ_DERR_STACK 16u
 #define RQ_DERR_QUEUE 32u
 #define RQ_DERR_WAIT_CHECK 64u
+#define RQ_DERR_LEAF 256u        // a traversed tree's live largest leaf is above RQ_MAX_LEAF
 #define RQ_DERR_RADV_IMAGE 128u  // rq_refit_radv: the image's header is not for this triangle count
 
 // Word of rq_ctx::d_err that holds the RADV build's finishing ticket: 0

@@ -168,6 +168,13 @@ __device__ __forceinline__ void child_of(const rq_bvh4_node* __restrict__ nodes,
 // is short.
 constexpr int kFewSearch = 8, kLeafWait = 8;
 
+// A parked leaf holds RQ_MAX_LEAF primitives.  The host refuses trees with
+// larger leaves by its copy of the counts; after an in-place rebuild that it
+// has not read back the live count (counts[3]) tells.  One thread of a launch.
+__device__ __forceinline__ void check_leaves(const uint32_t* __restrict__ counts, uint32_t* err) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && __ldg(counts + 3) > RQ_MAX_LEAF) set_err(err, RQ_DERR_LEAF);
+}
+
 // stk: this lane's column of `rows` stack entries, STRIDE apart.  CHUNK: ray
 // ids taken per atomic.  refill_min: idle lanes get new rays only once at
 // least this many lanes of the warp are idle (or all are), so that lanes join

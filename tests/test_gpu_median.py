@@ -176,3 +176,43 @@ def test_median_matches_its_statement(ctx, n, same, max_leaf):
     assert np.array_equal(perm, want)
     assert n2g.tobytes() == n2.tobytes()
     assert np.array_equal(trg["v1"][:, :3], pos.reshape(-1, 3, 3)[want, 1])
+
+
+@pytest.mark.parametrize("call", ["trace", "shadow_ao", "reflect", "ao_depth", "gbuffer"])
+def test_rebuild_to_leaves_too_large_is_reported(ctx, call):
+    """The host's largest leaf is from the first build; an in-place rebuild that ends in a leaf of 17 is found on the
+    device, by every kernel that cannot hold one."""
+    from rq import workloads as W
+    first = np.ascontiguousarray(tie_free_soup(40, 9)[:51])
+    pos = torch.from_numpy(first).cuda()
+    b = rq.Bvh.build(ctx, pos, median=True)
+    assert b.info()["max_leaf"] <= 4
+    cam, params = W.shadow_camera(), W.shadow_params()
+    cam.width, cam.height = params.width, params.height = 32, 16
+    gbuf = torch.zeros((32 * 16, 8), dtype=torch.int32, device="cuda")
+
+    def run():
+        if call == "trace":
+            rq.trace(ctx, b, torch.tensor([[0, 0, -9, 0, 0, 0, 1, 99]], dtype=torch.float32, device="cuda"))
+        elif call == "shadow_ao":
+            rq.render_shadow_ao(ctx, b, gbuf, params)
+        elif call == "reflect":
+            rq.render_reflect(ctx, b, gbuf, rq.ReflectParams(width=32, height=16))
+        elif call == "ao_depth":
+            p = rq.AoDepthParams(width=32, height=16, spp=1)
+            rq.render_ao_depth(ctx, b, torch.ones(32 * 16, device="cuda"), p)
+        else:
+            ctx.set_camera_tuning(1)
+            rq.render_gbuffer(ctx, b, cam, gbuf)
+        ctx.sync_check()
+
+    try:
+        run()
+        pos.copy_(torch.from_numpy(np.tile(first[:3], (17, 1))))
+        rq.Bvh.build(ctx, pos, median=True, into=b)
+        with pytest.raises(rq.RqError) as e:
+            run()
+        assert e.value.status == rq.RQ_ERR_UNSUPPORTED
+    finally:
+        ctx.set_camera_tuning(0)
+    b.destroy()
