@@ -241,3 +241,29 @@ def test_small_batches_fill_few_lanes(ctx, n, any_hit):
     want, _, _ = O.trace_bvh4(o["nodes4"], o["tris"], o["sorted"], rays, flags=flags)
     assert hits.cpu().numpy().tobytes() == want.tobytes()
     b.destroy()
+
+
+@pytest.mark.parametrize("tmax", [np.float32(np.inf), np.finfo(np.float32).max])
+def test_boxes_at_infinity_and_rays_without_an_end(ctx, tmax):
+    """Triangles parked at infinity: a child's entry distance is then infinite like a missed child's stand-in, and the
+    children left to visit are the hit ones alone (hits, barycentrics and test counts as the oracle's)."""
+    pos, idx = rq.scene_grid(40, 30, seed=3)
+    tri = pos[idx.reshape(-1)].reshape(-1, 9).copy()
+    tri[np.arange(len(tri)) // 8 % 3 == 1] = np.inf  # (codes are all 0 then, so leaves are runs of the input)
+    b = rq.Bvh.build(ctx, torch.from_numpy(tri.reshape(-1, 3)).cuda())
+    n2, tr, n4, perm = b.download()
+    rng = np.random.default_rng(4)
+    rays = np.zeros(20000, rq.RAY)
+    rays["org"] = rng.uniform(-1.2, 1.2, (20000, 3))
+    rays["dir"] = rng.uniform(0.05, 1.0, (20000, 3)) * rng.choice([1, 1, 1, -1], (20000, 3))
+    rays["tmax"] = tmax
+    rt = torch.from_numpy(rays.view(np.float32).reshape(-1, 8)).cuda()
+    for flags in range(4):
+        hits, bary, stats = rq.trace(ctx, b, rt, flags=flags, bary=True, stats=True)
+        ctx.sync_check()
+        oh, ob, os_ = O.trace_bvh4(n4, tr, perm, rays.view(O.RAY), flags, want_bary=True, want_stats=True)
+        assert rq.hits_numpy(hits).tobytes() == oh.tobytes(), flags
+        assert bary.cpu().numpy().reshape(-1).tobytes() == ob.tobytes(), flags
+        assert rq.stats_numpy(stats).tobytes() == os_.tobytes(), flags
+    assert np.isinf(n4["min_x"]).any() and 0.05 < oh["hit"].mean() < 0.95
+    b.destroy()
