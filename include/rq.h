@@ -590,7 +590,9 @@ int rq_radv_validate(rq_ctx* ctx, const void* as_image, uint64_t as_bytes, rq_ra
 
 /* Trace rays through a RADV image (the rayQueryEXT role of
  * shaders/verify_rayquery.comp:41-59): primitive IDs are the nodes'
- * triangle_id; `bary` as in rq_trace. */
+ * triangle_id; `bary` as in rq_trace.  as_bytes: the image's size.  A ray may
+ * have 64 box nodes behind it with children left to visit; beyond that
+ * rq_ctx_check reports RQ_ERR_UNSUPPORTED. */
 int rq_trace_radv(rq_ctx* ctx, const void* as_image, uint64_t as_bytes, const rq_ray* rays,
                   uint32_t n, uint32_t flags, rq_hit* hits, float* bary, rq_stream stream);
 

@@ -92,16 +92,25 @@ __global__ void __launch_bounds__(kT, kTraceBlocksPerSm) k_trace4(const rq_bvh4_
 // at 16 rays per warp, 18.3 at 8, 18.4 at 4.
 constexpr uint32_t kRadvSpread = 2;   // at least 8 rays per warp
 constexpr uint32_t kRadvFill = 768;   // threads per SM such a launch may take
-constexpr int kRadvRows = 32;  // a complete tree of 2^25 triangles is 14 deep
+// Open nodes that a ray may leave behind it.  This builder's trees are complete
+// (2^25 triangles: 14 deep), but any image may come in: a stack of 64 children,
+// the form before, held a chain of 63 two-child nodes, so as many rows hold all
+// it held.  An entry is 32 bits, a box node's offset (23 bits of 64 bytes) over
+// the order of its children left; images past 512 MiB (WIDE) take the order's
+// first child in the id's type bits and the others in a byte beside them.
+constexpr int kRadvRows = 64;
+constexpr uint64_t kRadvNarrow = uint64_t(64) << 23;
 
-template <bool ANY, bool MT, bool BARY>
+template <bool ANY, bool MT, bool BARY, bool WIDE>
 __global__ void __launch_bounds__(kT) k_trace_radv(const uint8_t* __restrict__ img, const rq_ray* __restrict__ rays,
                                                    uint32_t n, uint32_t spread, rq_hit* __restrict__ hits,
                                                    float* __restrict__ bary, uint32_t* err) {
-    __shared__ uint2 s_stack[kRadvRows * kT];
+    __shared__ uint32_t s_stack[kRadvRows * kT];
+    __shared__ uint8_t s_more[WIDE ? kRadvRows * kT : 1];
     const uint32_t g = blockIdx.x * kT + threadIdx.x, i = g >> spread;
     if (i >= n || (g & ((1u << spread) - 1u))) return;
-    uint2* stk = s_stack + threadIdx.x;
+    uint32_t* stk = s_stack + threadIdx.x;
+    uint8_t* more = s_more + (WIDE ? threadIdx.x : 0u);
     const uint8_t* base = img + RQ_RADV_BVH_OFFSET;
     const float4* rp = reinterpret_cast<const float4*>(rays + i);
     float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
@@ -127,9 +136,9 @@ __global__ void __launch_bounds__(kT) k_trace_radv(const uint8_t* __restrict__ i
     auto next = [&]() {
         if (left == 0u) {
             if (sp == 0) return false;
-            const uint2 e = stk[(--sp) * kT];
-            top = e.x;
-            left = e.y;
+            const uint32_t e = stk[(--sp) * kT];
+            top = WIDE ? e : e >> 6;  // (node() drops the lowest three bits)
+            left = WIDE ? (e & 7u) | uint32_t(more[sp * kT]) << 3 : e & 511u;
         }
         cur = __ldg(reinterpret_cast<const uint32_t*>(node(top)) + (left & 3u));
         left >>= 3;
@@ -163,10 +172,12 @@ __global__ void __launch_bounds__(kT) k_trace_radv(const uint8_t* __restrict__ i
                 const uint32_t seq = rq::child_sequence(hitm, tk, !ANY), first = seq & 3u;
                 if (seq >> 3) {
                     if (left) {
-                        if (sp < kRadvRows)
-                            stk[(sp++) * kT] = make_uint2(top, left);
-                        else
+                        if (sp < kRadvRows) {
+                            if (WIDE) more[sp * kT] = uint8_t(left >> 3);
+                            stk[(sp++) * kT] = WIDE ? (top & ~7u) | (left & 7u) : (top >> 3) << 9 | left;
+                        } else {
                             rq::set_err(err, RQ_DERR_STACK);
+                        }
                     }
                     top = cur;
                     left = seq >> 3;
@@ -453,7 +464,6 @@ int rq_launch_trace_ref2(rq_ctx* ctx, const rq_bvh2_node* nodes, const rq_triang
 
 int rq_launch_trace_radv(rq_ctx* ctx, const void* img, uint64_t bytes, const rq_ray* rays, uint32_t n,
                          uint32_t flags, rq_hit* hits, float* bary, cudaStream_t st) {
-    (void)bytes;
     if (n == 0) return RQ_OK;
     const uint8_t* im = static_cast<const uint8_t*>(img);
     const bool any = flags & RQ_TRACE_ANY, mt = flags & RQ_TRI_MT, b = bary != nullptr;
@@ -461,7 +471,10 @@ int rq_launch_trace_radv(rq_ctx* ctx, const void* img, uint64_t bytes, const rq_
     uint32_t spread = 0;
     while (spread < kRadvSpread && (uint64_t(n) << (spread + 1)) <= uint64_t(ctx->num_sms) * kRadvFill) ++spread;
     dim3 g(uint32_t(((uint64_t(n) << spread) + kT - 1) / kT));
-#define RQ_RADV_CASE(A, M, B) k_trace_radv<A, M, B><<<g, kT, 0, st>>>(im, rays, n, spread, hits, bary, ctx->d_err)
+    const bool wide = bytes > kRadvNarrow;
+#define RQ_RADV_CASE(A, M, B)                                                                                 \
+    (wide ? k_trace_radv<A, M, B, true> : k_trace_radv<A, M, B, false>)<<<g, kT, 0, st>>>(im, rays, n, spread, \
+                                                                                          hits, bary, ctx->d_err)
     if (any && mt && b) RQ_RADV_CASE(true, true, true);
     else if (any && mt) RQ_RADV_CASE(true, true, false);
     else if (any && b) RQ_RADV_CASE(true, false, true);

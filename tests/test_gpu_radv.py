@@ -213,3 +213,64 @@ def test_trace_radv_ray_counts(ctx, flags):
         got, gb = rq.trace_radv(ctx, img, rays[:n].contiguous(), flags=flags, bary=True)
         assert torch.equal(got, want[:n]) and torch.equal(gb, wb[:n]), n
     ctx.sync_check()
+
+
+def chain_image(depth, far=0):
+    """A chain of `depth` two-child box nodes: the next node, which a ray along +z meets first, and a triangle behind
+    it; the last node has two triangles.  Every box is as wide as the scene, triangle k is at x in (k, k + 1).  The nodes
+    after the root start `far` units of 64 bytes on."""
+    img = np.zeros(192 + 64 * (2 * depth + depth + 1), np.uint8)
+    words = img[192:].view(np.uint32).reshape(-1, 16)
+    row = lambda k: 2 * k  # box k; the triangles come after the boxes
+    tri = lambda k: 2 * depth + k
+    unit = lambda r: r + (far if r else 0)
+    for k in range(depth):
+        last = k == depth - 1
+        first = (unit(tri(k + 1)) << 3) if last else (unit(row(k + 1)) << 3) | 5
+        box = np.full((4, 6), np.nan, np.float32)
+        box[0] = [-1, -1, 500 - depth, depth + 2, 1, 500 - k - 1]
+        box[1] = [-1, -1, 500 - k, depth + 2, 1, 500 - k]
+        flat = np.concatenate([np.array([first, unit(tri(k)) << 3, 0xffffffff, 0xffffffff], np.uint32),
+                               box.view(np.uint32).reshape(-1), np.zeros(4, np.uint32)])
+        words[row(k)], words[row(k) + 1] = flat[:16], flat[16:]
+    for k in range(depth + 1):
+        z = np.float32(500 - k)
+        v = np.array([k, -1, z, k + 1, -1, z, k + 0.5, 1, z], np.float32)
+        words[tri(k), :9] = v.view(np.uint32)
+        words[tri(k), 12] = 7000 + k
+    return img
+
+
+def chain_rays(depth):
+    o = np.zeros((depth + 2, 3), np.float32)
+    o[:, 0] = np.arange(depth + 2) + 0.5
+    return rays_plus_z(o, 0.0, 1000.0)
+
+
+@pytest.mark.parametrize("flags", [0, rq.RQ_TRACE_ANY, rq.RQ_TRI_MT])
+@pytest.mark.parametrize("depth", [31, 34, 60, 63])
+def test_narrow_deep_images(ctx, depth, flags):
+    """Nodes left behind with children to visit, up to the deepest chain a stack of 64 children held."""
+    img = chain_image(depth)
+    rays = chain_rays(depth)
+    hits, bary = rq.trace_radv(ctx, torch.from_numpy(img).cuda(), torch.from_numpy(rays).cuda(), flags=flags, bary=True)
+    ctx.sync_check()
+    want, wb = O.trace_radv(img, rays.view(O.RAY).reshape(-1), flags, want_bary=True)
+    assert rq.hits_numpy(hits).tobytes() == want.tobytes()
+    assert bary.cpu().numpy().reshape(-1).tobytes() == wb.tobytes()
+    assert want["primitive_id"].tolist() == [7000 + k for k in range(depth + 1)] + [0xffffffff]
+
+
+@pytest.mark.parametrize("flags", [0, rq.RQ_TRACE_ANY])
+def test_deep_image_past_the_narrow_entries(ctx, flags):
+    """The same chain at the end of a 600 MiB image: node offsets above 2^23 units of 64 bytes."""
+    depth, far = 63, 9 << 20
+    img = chain_image(depth, far)
+    big = torch.zeros(far * 64 + len(img), dtype=torch.uint8, device="cuda")
+    big[192:320] = torch.from_numpy(img[192:320]).cuda()
+    big[192 + 64 * far + 128:] = torch.from_numpy(img[320:]).cuda()
+    rays = chain_rays(depth)
+    hits, _ = rq.trace_radv(ctx, big, torch.from_numpy(rays).cuda(), flags=flags)
+    ctx.sync_check()
+    near = chain_image(depth)
+    assert rq.hits_numpy(hits).tobytes() == O.trace_radv(near, rays.view(O.RAY).reshape(-1), flags)[0].tobytes()
