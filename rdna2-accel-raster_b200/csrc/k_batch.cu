@@ -105,9 +105,9 @@ int rq_launch_batch_trace(rq_ctx* ctx, const rq_batch* b, const rq_ray* rays, co
     const uint32_t chunk = tuned ? b->tune.trace_chunk : 32u;
     const uint32_t regs = tuned ? b->tune.trace_reg_cap : 0u;
     int refill_min = int(tuned && b->tune.trace_refill_min ? b->tune.trace_refill_min : 1u);
-    // stack rows: an entry per open node of a path, for the deepest tree or
-    // for the tree the tuned entry count (3 per level) was chosen for
-    int rows = int((std::max(bound, b->tune.stack_entries) + 2u) / 3u) + 1;
+    // for the deepest tree, or for the tree the tuned entry count (3 per level)
+    // was chosen for
+    int rows = rq::rebuild_rows((std::max(bound, b->tune.stack_entries) + 2u) / 3u - 3u);
     const void* kern = mt ? (stats ? trace_kernel<true, true>(tt, chunk, regs) : trace_kernel<true, false>(tt, chunk, regs))
                           : (stats ? trace_kernel<false, true>(tt, chunk, regs) : trace_kernel<false, false>(tt, chunk, regs));
     if (wide)

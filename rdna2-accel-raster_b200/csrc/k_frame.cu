@@ -450,9 +450,7 @@ cudaError_t persistent_grid(rq_ctx* ctx, const void* k, int threads, size_t smem
     return e;
 }
 
-// Stack rows per lane: an entry per open node of a path, for the depth the
-// host knows and what an in-place rebuild may add before it is read back.
-int stack_rows(const rq_bvh* bvh) { return int(bvh->h_counts[2]) + 4; }
+int stack_rows(const rq_bvh* bvh) { return rq::rebuild_rows(bvh->h_counts[2]); }
 
 // Shadow/AO kernel of a launch shape (only the default shape has the counting
 // and reference-arithmetic variants).

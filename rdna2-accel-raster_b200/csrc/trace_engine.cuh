@@ -178,6 +178,18 @@ __device__ __forceinline__ void child_of(const rq_bvh4_node* __restrict__ nodes,
 // is short.
 constexpr int kFewSearch = 8, kLeafWait = 8;
 
+// Stack rows for trees of `depth` 4-wide levels, as the host knows them, whose
+// handle may be rebuilt in place before the host reads the new depth: d levels
+// leave at most d - 1 open nodes behind.  Four levels to spare, and otherwise
+// what the stack of children before held (3 * (depth + 2) + 1 entries) up to 24
+// rows, trees of 25 levels: a 2,000-triangle mesh 7 levels deep that contracts
+// toward a point is rebuilt to 20.  Up to 24 rows cost nothing, since the
+// shared memory they need comes in steps: camera rays on 8.3M triangles 2,245
+// us with 18 rows, 2,247 with 24, 2,266 with 28 and 2,306 with 46.
+inline int rebuild_rows(uint32_t depth) {
+    return int(depth + 4u > 24u ? depth + 4u : (3u * depth + 7u < 24u ? 3u * depth + 7u : 24u));
+}
+
 // A parked leaf holds RQ_MAX_LEAF primitives.  The host refuses trees with
 // larger leaves by its copy of the counts; after an in-place rebuild that it
 // has not read back the live count (counts[3]) tells.  One thread of a launch.

@@ -254,3 +254,38 @@ def test_batch_groups(ctx):
             assert g.tobytes() == w.tobytes(), m
     s.destroy()
     b.destroy()
+
+
+def test_batch_rebuilt_to_deeper_trees(ctx):
+    """The stack is sized by the first build's depths; meshes that contract and are rebuilt are traced as separate
+    builds of them, by rays along which the nested boxes pile up on the stack."""
+    from test_gpu_frame import contracting
+    n, m = 2000, 1 << 18
+    idx = np.arange(3 * n, dtype=np.uint32).reshape(-1, 3)
+    rng = np.random.default_rng(0)
+    c = np.concatenate([rng.uniform(-1, 1, (n, 2)), rng.uniform(-0.1, 0.1, (n, 1))], 1)
+    flat = (c[:, None] + rng.uniform(-0.02, 0.02, (n, 3, 3))).astype(np.float32).reshape(-1, 3)
+    deep = [contracting(n, 1.01), contracting(n, 1.008)]
+    p = torch.from_numpy(np.tile(flat, (2, 1))).cuda()
+    i = torch.from_numpy(np.tile(idx, (2, 1)).view(np.int32)).cuda()
+    b = rq.Batch(ctx, [(0, 3 * n, 0, n), (3 * n, 3 * n, n, n)], max_leaf=1)
+    b.build(p, i)
+    assert max(b.info(k)["depth4"] for k in (0, 1)) == 7
+    p.copy_(torch.from_numpy(np.concatenate(deep)))
+    b.build(p, i)
+    rays = np.zeros(m, rq.RAY)
+    rays["org"] = (-1.6, -1.5, -1.55)
+    rays["dir"] = rng.uniform(-1, 1, (m, 1)) + rng.uniform(-0.2, 0.2, (m, 3)) - rays["org"]
+    rays["tmax"] = 100
+    mesh = torch.arange(m, dtype=torch.int32, device="cuda") % 2
+    rt = torch.from_numpy(rays.view(np.float32).reshape(-1, 8)).cuda()
+    hits, _ = b.trace(rt, mesh)
+    ctx.sync_check()
+    for k in (0, 1):
+        s = rq.Bvh.build(ctx, torch.from_numpy(deep[k]).cuda(), max_leaf=1)
+        assert s.info()["depth4"] >= 18
+        want, _, _ = rq.trace(ctx, s, rt[k::2].contiguous())
+        assert torch.equal(hits[k::2], want)
+        assert 0.02 < (want[:, 0] != 0).float().mean() < 1
+        s.destroy()
+    b.destroy()

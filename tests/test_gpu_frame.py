@@ -240,3 +240,36 @@ def test_every_camera_schedule_gives_identical_gbuffers(ctx):
     with pytest.raises(rq.RqError):
         ctx.set_camera_tuning(2, 1, 1)
     b.destroy()
+
+
+def contracting(n, base):
+    """n triangles whose places and sizes shrink by `base` each toward (-1, -1, -1): a deep tree."""
+    s = np.float64(base) ** -np.arange(n)
+    e = np.random.default_rng(1).uniform(-0.3, 0.3, (n, 3, 3))
+    return (2 * s[:, None, None] - 1 + s[:, None, None] * e).astype(np.float32).reshape(-1, 3)
+
+
+@pytest.mark.parametrize("n,base,first,then", [(200, 1.05, 5, 14), (2000, 1.01, 7, 19)])
+def test_rebuild_in_place_to_a_deeper_tree(ctx, n, base, first, then):
+    """The host sizes the stack by the first build's depth; a mesh that contracts and is rebuilt in place is rendered as
+    a fresh build of it, from where the nested boxes pile up on the stack."""
+    rng = np.random.default_rng(0)
+    c = np.concatenate([rng.uniform(-1, 1, (n, 2)), rng.uniform(-0.1, 0.1, (n, 1))], 1)
+    flat = (c[:, None] + rng.uniform(-0.02, 0.02, (n, 3, 3))).astype(np.float32).reshape(-1, 3)
+    deep = torch.from_numpy(contracting(n, base)).cuda()
+    pos = torch.from_numpy(flat).cuda()
+    b = rq.Bvh.build(ctx, pos, max_leaf=1)
+    assert b.info()["depth4"] == first
+    fresh = rq.Bvh.build(ctx, deep, max_leaf=1)
+    assert fresh.info()["depth4"] == then
+    pos.copy_(deep)
+    rq.Bvh.build(ctx, pos, max_leaf=1, into=b)
+    cam = rq.camera_look_at((-1.6, -1.5, -1.55), (1, 1, 1), (0, 1, 0), 40.0, 640, 360)
+    got = rq.render_gbuffer(ctx, b, cam)
+    ctx.sync_check()
+    want = rq.render_gbuffer(ctx, fresh, cam)
+    ctx.sync_check()
+    assert torch.equal(got, want)
+    assert (got[:, 3] != 0).float().mean() > 0.01
+    b.destroy()
+    fresh.destroy()
