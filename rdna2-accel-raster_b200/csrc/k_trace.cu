@@ -23,7 +23,7 @@ constexpr int kT = 128;
 // triangles, incoherent).
 constexpr int kTraceRefill = 16;
 constexpr int kTraceBlocksPerSm = 8;
-constexpr uint32_t kSmallTree = 4096;  // 4-wide nodes
+constexpr uint32_t kSmallTree = 4096, kLargeTree = 1u << 17;  // 4-wide nodes
 
 __device__ __forceinline__ void store_miss(rq_hit* hits, uint32_t i) {
     reinterpret_cast<uint4*>(hits)[i] = make_uint4(0u, __float_as_uint(-1.0f), 0xffffffffu, 0xffffffffu);
@@ -382,12 +382,22 @@ cudaError_t launch4(rq_ctx* ctx, const rq_bvh* b, const rq_ray* rays, uint32_t n
     uint32_t blocks = uint32_t(ctx->num_sms) * uint32_t(wide && rows > 24 ? 4 : kTraceBlocksPerSm);
     // A batch of less than one ray per resident lane takes the time of its
     // slowest warp, whose length grows with the rays that share it: it is
-    // spread over all the warps there are, at 4, 8 or 16 rays each (999,698
-    // triangles, closest hit, us at 32 -> fewer: 8,192 rays 108 -> 74, 32,768
-    // 106 -> 94, 65,536 108 -> 100; 99,458 triangles 62 -> 45, 59 -> 53, 59 -> 61).
+    // spread over all the warps there are, at 4, 8 or 16 rays each, but not down
+    // to a ray for every lane that takes part: a warp that starts full has no
+    // slack, and the next step is as fast or faster from 3/4 on, on trees of more
+    // than kLargeTree nodes, whose walks differ more, from 7/8 on.  Closest hit,
+    // us at 4 / 8 / 16 / 32 rays (4 and 8 hold 18,944 and 37,888 rays):
+    //               99,458 triangles            999,698
+    //   12,000      44.8 / 44.7 / 46.5 / 48.6   48.8 / 48.8 / 50.6 / 53.5
+    //   18,000      50.8 / 48.8 / 48.7 / 51.0   53.5 / 51.7 / 50.9 / 55.2
+    //   37,000        -  / 55.0 / 55.1 / 54.6     -  / 61.0 / 57.2 / 57.7
+    //   65,536        -  /   -  / 61.2 / 59.3     -  /   -  / 65.2 / 65.3
+    // (any hit, 65,536 rays on 999,698: 58.1 at 16, 60.5 at 32; 8.3M triangles,
+    // closest hit 87.0 and 90.3; 968 triangles 42.9 and 40.5).
     const uint32_t warps = blocks * (kT / 32);
+    const uint32_t eighths = b->h_counts[1] > kLargeTree ? 7 : 6;
     uint32_t lanes = 4;
-    while (lanes < 32u && n > lanes * warps) lanes *= 2;
+    while (lanes < 32u && n > lanes * warps / 8u * eighths) lanes *= 2;
     // On small trees a node phase is a few steps, and leaving it early costs more
     // than the idle lanes do (2^20 rays, us with and without: 968 triangles
     // incoherent 166 / 156, coherent 101 / 98, 8,192 coherent 113 / 110; 99,458

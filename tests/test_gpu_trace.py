@@ -243,6 +243,12 @@ def test_small_batches_fill_few_lanes(ctx, n, any_hit):
     b.destroy()
 
 
+@pytest.mark.parametrize("n", [14208, 14209, 28416, 28417, 56832, 56833])
+def test_small_batches_at_three_quarters_of_the_lanes(ctx, n):
+    """The sizes where the lanes that take part double: three quarters of the resident warps' lanes hold a ray."""
+    test_small_batches_fill_few_lanes(ctx, n, False)
+
+
 @pytest.mark.parametrize("tmax", [np.float32(np.inf), np.finfo(np.float32).max])
 def test_boxes_at_infinity_and_rays_without_an_end(ctx, tmax):
     """Triangles parked at infinity: a child's entry distance is then infinite like a missed child's stand-in, and the
