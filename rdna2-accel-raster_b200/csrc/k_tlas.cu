@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kTT, kTlasBlocks)
                         set_err(err, RQ_DERR_STACK);
                 }
                 top.node = ci;
-                top.left = ANY ? hitm : child_sequence(hitm, tk, true);
+                top.left = ANY ? hitm : child_sequence<false>(hitm, tk, true);
             }
         }
         // ---- the lanes' other work

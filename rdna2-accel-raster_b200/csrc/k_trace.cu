@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kT) k_trace_radv(const uint8_t* __restrict__ i
                     ac[k] != RQ_RADV_INVALID_NODE)
                     hitm |= 1u << k;
             if (hitm) {
-                const uint32_t seq = rq::child_sequence(hitm, tk, !ANY), first = seq & 3u;
+                const uint32_t seq = rq::child_sequence<false>(hitm, tk, !ANY), first = seq & 3u;
                 if (seq >> 3) {
                     if (left) {
                         if (sp < kRadvRows) {

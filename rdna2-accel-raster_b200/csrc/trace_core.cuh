@@ -54,7 +54,7 @@ __device__ __forceinline__ void trace_ray(const rq_bvh4_node* __restrict__ nodes
                         set_err(err, RQ_DERR_STACK);  // deeper than the host knew
                 }
                 top.node = ci;
-                top.left = child_sequence(hitm, tk, true);
+                top.left = child_sequence<false>(hitm, tk, true);
             }
         } else {  // a leaf (or an empty slot whose point box the ray met)
             const uint32_t first = uint32_t(~ci);

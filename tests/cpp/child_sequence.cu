@@ -21,10 +21,11 @@ int main() {
                 if (sorted) std::stable_sort(order, order + n, [&](int a, int b) { return t[a] < t[b]; });
                 uint32_t want = 0;
                 for (int i = 0; i < n; ++i) want |= uint32_t(4 | order[i]) << (3 * i);
-                const uint32_t got = rq::child_sequence(hitm, t, sorted != 0);
-                if (got != want && bad++ < 5)
-                    std::printf("hits %x at %g %g %g %g, sorted %d: %o for %o\n", hitm, t[0], t[1], t[2], t[3], sorted,
-                                got, want);
+                const uint32_t got = rq::child_sequence<false>(hitm, t, sorted != 0),
+                               mixed = rq::child_sequence<true>(hitm, t, sorted != 0);
+                if ((got != want || mixed != want) && bad++ < 5)
+                    std::printf("hits %x at %g %g %g %g, sorted %d: %o, %o for %o\n", hitm, t[0], t[1], t[2], t[3], sorted,
+                                got, mixed, want);
             }
     std::printf("%d of 20000 wrong\n", bad);
     return bad != 0;
