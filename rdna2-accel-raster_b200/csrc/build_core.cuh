@@ -449,10 +449,9 @@ struct N2 {
     int32_t l, r;
 };
 
-template <bool NC>
 __device__ __forceinline__ N2 load_n2(const rq_bvh2_node* n2, int32_t i) {
     const float4* p = reinterpret_cast<const float4*>(n2 + i);
-    const float4 a = NC ? __ldg(p) : p[0], b = NC ? __ldg(p + 1) : p[1];
+    const float4 a = __ldg(p), b = __ldg(p + 1);
     N2 o;
     o.mn[0] = a.x;
     o.mn[1] = a.y;
@@ -476,7 +475,6 @@ __device__ __forceinline__ float node_area(const N2& nd) {
 // surface area (strict >, first wins) until four.  Returns the count;
 // inner[i]: candidate i is an inner binary node.  end, ce: in a pre-order tree,
 // the end of u's range and of each candidate's.
-template <bool NC>
 __device__ __forceinline__ int greedy_candidates(const rq_bvh2_node* n2, int32_t u, int32_t c[4], bool inner[4],
                                                  int32_t end, int32_t (&ce)[4]) {
     // each candidate's children and surface area, loaded once (slots are
@@ -489,9 +487,9 @@ __device__ __forceinline__ int greedy_candidates(const rq_bvh2_node* n2, int32_t
         cr[i] = nd.r;
         sa[i] = node_area(nd);
     };
-    const N2 nd = load_n2<NC>(n2, u);
+    const N2 nd = load_n2(n2, u);
     {
-        const N2 a = load_n2<NC>(n2, nd.l), b = load_n2<NC>(n2, nd.r);
+        const N2 a = load_n2(n2, nd.l), b = load_n2(n2, nd.r);
         set(0, nd.l, a);
         set(1, nd.r, b);
     }
@@ -526,7 +524,7 @@ __device__ __forceinline__ int greedy_candidates(const rq_bvh2_node* n2, int32_t
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (i == nc) ce[i] = e;
-        const N2 a = load_n2<NC>(n2, l), b = load_n2<NC>(n2, r);
+        const N2 a = load_n2(n2, l), b = load_n2(n2, r);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             if (i == best) set(i, l, a);
@@ -541,7 +539,6 @@ __device__ __forceinline__ int greedy_candidates(const rq_bvh2_node* n2, int32_t
 
 // Writes 4-wide node p from its candidates and the places of the inner ones
 // (-1: a leaf).
-template <bool NC>
 __device__ __forceinline__ void write_node4(const rq_bvh2_node* n2, const int32_t (&cand)[4], const int32_t (&at)[4],
                                             uint32_t p, rq_bvh4_node* out4, int32_t* map4) {
     float mnx[4], mxx[4], mny[4], mxy[4], mnz[4], mxz[4];
@@ -552,7 +549,7 @@ __device__ __forceinline__ void write_node4(const rq_bvh2_node* n2, const int32_
         ci[k] = 0;
         cc[k] = 0;
         if (cand[k] >= 0) {
-            const N2 nd = load_n2<NC>(n2, cand[k]);
+            const N2 nd = load_n2(n2, cand[k]);
             mnx[k] = nd.mn[0];
             mxx[k] = nd.mx[0];
             mny[k] = nd.mn[1];
@@ -614,15 +611,14 @@ __device__ __forceinline__ uint32_t inner_children(const CollapseIO& io, uint32_
 //      1 + the sizes of the earlier inner siblings (a walk up that stops at
 //      the first ancestor whose position a written parent already
 //      published), then the node write.
-// NARROW > 0 (grid-wide use):
-// block 0 alone expands the top levels while they hold at most NARROW
+// Block 0 alone expands the top levels while they hold at most NARROW
 // entries.  io.tail holds 16 control words.
 // Data written inside the collapse is read with ld.cg: other blocks wrote it.
-template <bool NC, uint32_t NARROW, class Sync>
+template <uint32_t NARROW, class Sync>
 __device__ __forceinline__ bool collapse_levels(const CollapseIO& io, uint32_t tid, uint32_t nthreads,
                                                 uint32_t max_levels, Sync sync, uint32_t* err,
                                                 uint32_t* total_out, uint32_t* depth_out) {
-    const bool root_leaf = load_n2<NC>(io.n2, 0).l < 0;
+    const bool root_leaf = load_n2(io.n2, 0).l < 0;
     // Entries of level L+1 are appended at end(L) + an atomic count of their
     // own, io.tail[4 + L % 3]: after the level's sync every thread reads that
     // count while the next level appends to another one, and the one after
@@ -639,7 +635,7 @@ __device__ __forceinline__ bool collapse_levels(const CollapseIO& io, uint32_t t
         if (root_leaf)
             c[0] = 0;
         else
-            greedy_candidates<NC>(io.n2, u, c, inner, 0, ce);
+            greedy_candidates(io.n2, u, c, inner, 0, ce);
         const uint32_t cnt = uint32_t(inner[0]) + uint32_t(inner[1]) + uint32_t(inner[2]) + uint32_t(inner[3]);
         const uint32_t act = __activemask();
         const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
@@ -672,30 +668,28 @@ __device__ __forceinline__ bool collapse_levels(const CollapseIO& io, uint32_t t
     }
     if (!sync()) return false;
     uint32_t start = 0, end = 1, depth = 0;
-    if (NARROW > 0) {
-        // the narrow top levels (at most NARROW entries each) by block 0
-        // alone, with block barriers; then one sync hands the frontier over
-        if (blockIdx.x == 0) {
-            while (start < end && end - start <= NARROW && depth + 1 < max_levels) {
-                if (threadIdx.x == 0) atomicExch(lvl_cnt + (depth + 1) % 3u, 0u);
-                for (uint32_t e = start + threadIdx.x; e < end; e += blockDim.x) expand(e, end, depth);
-                __syncthreads();
-                const uint32_t n = __ldcg(lvl_cnt + depth % 3u);
-                ++depth;
-                start = end;
-                end += n;
-            }
-            if (threadIdx.x == 0) {
-                __stcg(io.tail + 8, start);
-                __stcg(io.tail + 9, end);
-                __stcg(io.tail + 10, depth);
-            }
+    // the narrow top levels (at most NARROW entries each) by block 0
+    // alone, with block barriers; then one sync hands the frontier over
+    if (blockIdx.x == 0) {
+        while (start < end && end - start <= NARROW && depth + 1 < max_levels) {
+            if (threadIdx.x == 0) atomicExch(lvl_cnt + (depth + 1) % 3u, 0u);
+            for (uint32_t e = start + threadIdx.x; e < end; e += blockDim.x) expand(e, end, depth);
+            __syncthreads();
+            const uint32_t n = __ldcg(lvl_cnt + depth % 3u);
+            ++depth;
+            start = end;
+            end += n;
         }
-        if (!sync()) return false;
-        start = __ldcg(io.tail + 8);
-        end = __ldcg(io.tail + 9);
-        depth = __ldcg(io.tail + 10);
+        if (threadIdx.x == 0) {
+            __stcg(io.tail + 8, start);
+            __stcg(io.tail + 9, end);
+            __stcg(io.tail + 10, depth);
+        }
     }
+    if (!sync()) return false;
+    start = __ldcg(io.tail + 8);
+    end = __ldcg(io.tail + 9);
+    depth = __ldcg(io.tail + 10);
     while (start < end) {
         if (tid == 0) atomicExch(lvl_cnt + (depth + 1) % 3u, 0u);
         for (uint32_t e = start + tid; e < end; e += nthreads) expand(e, end, depth);
@@ -762,7 +756,7 @@ __device__ __forceinline__ bool collapse_levels(const CollapseIO& io, uint32_t t
             __stcg(io.acc + cq, (1ull << 63) | off);
             off += __ldcg(io.sz + cq);
         }
-        write_node4<NC>(io.n2, cand, at, pre, io.out4, io.map4);
+        write_node4(io.n2, cand, at, pre, io.out4, io.map4);
     }
     if (!sync()) return false;
     *total_out = end;

@@ -224,13 +224,11 @@ int rq_batch_create(rq_ctx* ctx, const rq_mesh_desc* meshes, uint32_t num_meshes
     if (!ctx || !meshes || !out || num_meshes == 0) return rq_set_error(ctx, RQ_ERR_INVALID_ARG, "bad batch");
     if (max_leaf < 1 || max_leaf > 16) return rq_set_error(ctx, RQ_ERR_INVALID_ARG, "max_leaf must be 1..16");
     uint64_t end = 0;
-    uint32_t maxt = 0;
     for (uint32_t m = 0; m < num_meshes; ++m) {
         const rq_mesh_desc& d = meshes[m];
         if (d.num_triangles == 0 || d.num_triangles > kMaxBatchMeshTris)
             return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "batch meshes need 1..2^20 triangles");
         end = std::max<uint64_t>(end, uint64_t(d.triangle_offset) + d.num_triangles);
-        maxt = std::max(maxt, d.num_triangles);
     }
     if (end >= RQ_MAX_TRIANGLES) return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "batch larger than 2^27 triangles");
     // triangle ranges must not overlap
@@ -250,7 +248,6 @@ int rq_batch_create(rq_ctx* ctx, const rq_mesh_desc* meshes, uint32_t num_meshes
     b->device = ctx->device;
     b->num_meshes = num_meshes;
     b->total_tris = uint32_t(end);
-    b->max_tris = maxt;
     b->max_leaf = max_leaf;
     b->meshes.assign(meshes, meshes + num_meshes);
     b->h_counts.assign(4ull * num_meshes, 0u);

@@ -92,7 +92,7 @@ __device__ __forceinline__ void collapse_top(const CollapseTree& t, uint32_t tre
         for (uint32_t e = start + threadIdx.x; e < end; e += kTopT) {
             int32_t c[4], ce[4];
             bool inner[4];
-            greedy_candidates<true>(t.n2, int32_t(t.q[e]), c, inner, int32_t(t.end[e]), ce);
+            greedy_candidates(t.n2, int32_t(t.q[e]), c, inner, int32_t(t.end[e]), ce);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 int32_t ch = -1;
@@ -134,7 +134,7 @@ __device__ __forceinline__ void collapse_treelet(TreeletShared& S, const Collaps
                                                  uint32_t k, uint4 rec) {
     const uint32_t u = rec.x, len = rec.y;
     for (uint32_t i = threadIdx.x; i < len; i += kCollapseT) {
-        const N2 nd = load_n2<true>(t.n2, int32_t(u + i));
+        const N2 nd = load_n2(t.n2, int32_t(u + i));
         S.link[i] = uint16_t(nd.l < 0 ? TreeletShared::kNone : uint32_t(nd.r) - u);
         S.area[i] = node_area(nd);
     }
@@ -375,7 +375,7 @@ __device__ __forceinline__ void collapse_write(const CollapseTree& t, const Tree
         }
         float lo[4] = {0.0f, 0.0f, 0.0f, 0.0f}, hi[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // rows 0..3, 4..7
         if (c >= 0) {
-            const N2 nd = load_n2<true>(t.n2, c);
+            const N2 nd = load_n2(t.n2, c);
             lo[0] = nd.mn[0];
             lo[1] = nd.mx[0];
             lo[2] = nd.mn[1];

@@ -54,17 +54,16 @@ struct BatchSrc {
 
 // Traversal blocks of TT threads, ray ids taken CHUNK at a time, and (REGS)
 // launch bounds that hold registers to REGS per thread: the tuned shapes.
-// The stack has `rows` entries per lane (from the batch's deepest tree); idle
-// lanes are refilled once `refill_min` of a warp's lanes are idle.  WIDE: a
-// mesh has room for more nodes than a 32-bit entry can name.
-template <bool MT, bool STATS, int TT, int CHUNK, int REGS, bool WIDE = false>
+// The stack has `rows` entries per lane (from the batch's deepest tree; 32 bits
+// name every node of a mesh of at most 2^20 triangles); idle lanes are refilled
+// once `refill_min` of a warp's lanes are idle.
+template <bool MT, bool STATS, int TT, int CHUNK, int REGS>
 __global__ void __launch_bounds__(TT, 65536 / (TT * (REGS ? REGS : 65536 / TT)))
     k_batch_trace(const __grid_constant__ BatchSrc<STATS> src, uint32_t* ctr, uint32_t* err, int rows,
                   int refill_min) {
-    extern __shared__ __align__(16) char s_stack[];
-    using Entry = typename rq::OpenNode<false, WIDE>::Entry;
-    rq::trace_persistent<rq::kAnyPerRay, MT, STATS, TT, const BatchSrc<STATS>, CHUNK, WIDE>(
-        nullptr, nullptr, src, ctr, reinterpret_cast<Entry*>(s_stack) + threadIdx.x, rows, err, refill_min);
+    extern __shared__ __align__(16) uint32_t s_entries[];
+    rq::trace_persistent<rq::kAnyPerRay, MT, STATS, TT, const BatchSrc<STATS>, CHUNK>(
+        nullptr, nullptr, src, ctr, s_entries + threadIdx.x, rows, err, refill_min);
 }
 
 // Kernel of a traversal shape (only the default shape has the counting and
@@ -98,9 +97,8 @@ int rq_launch_batch_trace(rq_ctx* ctx, const rq_batch* b, const rq_ray* rays, co
     const uint32_t bound = 3u * (b->max_depth + 2u) + 1u;
     if (bound > 128u) return rq_set_error(ctx, RQ_ERR_UNSUPPORTED, "4-wide tree deeper than 40 levels");
     const bool mt = flags & RQ_TRI_MT;
-    // the counting, reference-arithmetic and 64-bit entry variants run in the default shape
-    const bool wide = b->max_tris > RQ_NARROW_NODES;
-    const bool tuned = !mt && !stats && !wide;
+    // the counting and reference-arithmetic variants run in the default shape
+    const bool tuned = !mt && !stats;
     const uint32_t tt = tuned ? b->tune.trace_threads : 128u;
     const uint32_t chunk = tuned ? b->tune.trace_chunk : 32u;
     const uint32_t regs = tuned ? b->tune.trace_reg_cap : 0u;
@@ -110,13 +108,8 @@ int rq_launch_batch_trace(rq_ctx* ctx, const rq_batch* b, const rq_ray* rays, co
     int rows = rq::rebuild_rows((std::max(bound, b->tune.stack_entries) + 2u) / 3u - 3u);
     const void* kern = mt ? (stats ? trace_kernel<true, true>(tt, chunk, regs) : trace_kernel<true, false>(tt, chunk, regs))
                           : (stats ? trace_kernel<false, true>(tt, chunk, regs) : trace_kernel<false, false>(tt, chunk, regs));
-    if (wide)
-        kern = mt ? (stats ? reinterpret_cast<const void*>(k_batch_trace<true, true, 128, 32, 0, true>)
-                           : reinterpret_cast<const void*>(k_batch_trace<true, false, 128, 32, 0, true>))
-                  : (stats ? reinterpret_cast<const void*>(k_batch_trace<false, true, 128, 32, 0, true>)
-                           : reinterpret_cast<const void*>(k_batch_trace<false, false, 128, 32, 0, true>));
     if (!kern) return rq_set_error(ctx, RQ_ERR_INVALID_ARG, "no traversal kernel for this shape");
-    const size_t smem = size_t(rows) * tt * (wide ? 8 : 4);
+    const size_t smem = size_t(rows) * tt * sizeof(uint32_t);
     cudaError_t e = cudaMemsetAsync(ctr, 0, sizeof(uint32_t), st);
     if (e == cudaSuccess && smem > 48 * 1024)
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));

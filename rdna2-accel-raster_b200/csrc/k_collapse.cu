@@ -86,8 +86,8 @@ __global__ void __launch_bounds__(kT) k_collapse(CollapseArgs A) {
     uint32_t total = 0, depth = 0;
     auto sync = [&]() { return grid_sync(A.ctl, A.err); };
     // levels of at most 256 entries by block 0 alone (measured: a little faster than a grid barrier each)
-    if (!rq::collapse_levels<true, 256>(io, blockIdx.x * kT + threadIdx.x, gridDim.x * kT, kMaxLevels,
-                                               sync, A.err, &total, &depth))
+    if (!rq::collapse_levels<256>(io, blockIdx.x * kT + threadIdx.x, gridDim.x * kT, kMaxLevels, sync, A.err, &total,
+                                  &depth))
         return;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         A.counts[1] = total;
@@ -111,7 +111,6 @@ int rq_collapse_blocks(int device, int num_sms) {
 }
 
 int rq_launch_collapse(rq_ctx* ctx, rq_bvh* bvh, BuildScratch& s, cudaStream_t st) {
-    if (ctx->collapse_blocks <= 0) return rq_set_error(ctx, RQ_ERR_CUDA, "collapse kernel cannot be co-resident");
     cudaMemsetAsync(s.coll_ctl, 0, 256 * sizeof(uint32_t), st);
     if (!bvh->foreign) {
         // the node, leaf and centroid arrays of the build are free by now
@@ -123,6 +122,7 @@ int rq_launch_collapse(rq_ctx* ctx, rq_bvh* bvh, BuildScratch& s, cudaStream_t s
         rq::launch_collapse(t, T, 1, ctx->num_sms, st);
         return rq_cuda_status(ctx, cudaGetLastError(), "collapse launch");
     }
+    if (ctx->collapse_blocks <= 0) return rq_set_error(ctx, RQ_ERR_CUDA, "collapse kernel cannot be co-resident");
     CollapseArgs a;
     a.n2 = bvh->nodes2;
     a.counts = bvh->d_counts;

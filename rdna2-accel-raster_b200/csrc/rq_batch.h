@@ -43,7 +43,6 @@ struct rq_batch {
     int device = 0;
     uint32_t num_meshes = 0;
     uint32_t total_tris = 0;
-    uint32_t max_tris = 0;
     uint32_t max_leaf = 4;
     std::vector<rq_mesh_desc> meshes;  // host copy
     // arrays of all meshes: mesh m's binary nodes start at 2*triangle_offset,

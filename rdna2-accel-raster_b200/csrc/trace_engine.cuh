@@ -145,7 +145,6 @@ template <bool MIXED>
 __host__ __device__ __forceinline__ uint32_t child_sequence(uint32_t hitm, const float (&tk)[4], bool sorted) {
     float first[4], second[4];
     bool hit[4];
-#pragma unroll
     for (int k = 0; k < 4; ++k) {
         hit[k] = (hitm >> k) & 1u;
         const float t = sorted ? tk[k] : 0.0f;
@@ -158,7 +157,6 @@ __host__ __device__ __forceinline__ uint32_t child_sequence(uint32_t hitm, const
                    p23 = before(2, 3);
     const uint32_t r[4] = {3u - (p01 + p02 + p03), p01 + 2u - (p12 + p13), p02 + p12 + 1u - p23, p03 + p13 + p23};
     uint32_t s = 0;
-#pragma unroll
     for (uint32_t k = 0; k < 4; ++k) s |= hit[k] ? (4u | k) << (3u * r[k]) : 0u;
     return s;
 }
