@@ -2,9 +2,9 @@
 """Benchmark of the ray-query engine on one B200 (or N replicas).
 
 Default workload — the 1080p shadows + AO frame: a 2,499,848-triangle
-height-field grid (1118x1118 quads, seed 1), per step a full LBVH rebuild
-(Morton codes, onesweep radix sort, Karras hierarchy, refit, 4-wide
-collapse), 2,073,600 primary closest-hit rays into a G-buffer, then 16
+height-field grid (1118x1118 quads, seed 1), per step a full rebuild (Morton
+codes, radix sort, hierarchy with SAH-rebuilt subtrees, 4-wide collapse),
+2,073,600 primary closest-hit rays into a G-buffer, then 16
 any-hit shadow rays and 1 cosine AO ray per pixel generated and traced in one
 kernel.  value = rays traced per step / step time (Mrays/s); the per-frame
 build rate (Mtris/s) and the any-hit rate are reported beside it.

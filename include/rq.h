@@ -277,9 +277,9 @@ typedef struct rq_mesh_desc {
  * ranges must not overlap.  The batch owns its arrays and build scratch. */
 int rq_batch_create(rq_ctx* ctx, const rq_mesh_desc* meshes, uint32_t num_meshes, uint32_t max_leaf,
                     rq_batch** out);
-/* Build every mesh's binary and 4-wide BVH in ONE persistent launch: each
- * thread block builds one mesh at a time (largest first) with the same steps
- * as rq_build, so each mesh's bytes equal a separate rq_build of it.  Device
+/* Build every mesh's binary and 4-wide BVH together: each step of rq_build
+ * runs once over all meshes (over up to 16M triangles of whole meshes at a
+ * time), so each mesh's bytes equal a separate rq_build of it.  Device
  * pointers; stride as in rq_build.  The first build synchronises once to
  * read the depths; later builds stay asynchronous. */
 int rq_batch_build(rq_ctx* ctx, rq_batch* batch, const float* positions, uint32_t stride_bytes,
@@ -311,7 +311,8 @@ typedef struct rq_instance {
     float transform[12];  /* object -> world, row-major 3x4 (VkTransformMatrixKHR) */
     uint32_t instance_id; /* reported as rq_hit.instance_id (instanceCustomIndex) */
     uint32_t mask;        /* seen by rays whose cull mask shares a bit with it */
-    const rq_bvh* blas;   /* built with RQ_BUILD_BVH4; many instances may share one */
+    const rq_bvh* blas;   /* built with RQ_BUILD_BVH4, leaves of at most 16 triangles; many instances may
+                             share one */
 } rq_instance;
 
 /* Build the top level over `num_instances` instances (host array; copied).
@@ -327,7 +328,7 @@ int rq_tlas_trace(rq_ctx* ctx, const rq_tlas* tlas, const rq_ray* rays, uint32_t
                   uint32_t cull_mask, rq_hit* hits, rq_stream stream);
 int rq_tlas_destroy(rq_tlas* tlas);
 
-/* Launch shapes of a batch's two kernels.  Results do not depend on them. */
+/* Launch shape of a batch's traversal.  Results do not depend on it. */
 typedef struct rq_batch_tuning {
     uint32_t build_threads;       /* 256, 512 or 1024: accepted, without effect (all meshes' builds
                                      share their launches; so do the other build_* fields) */

@@ -16,7 +16,7 @@
 // With SAH subtrees (RQ_BUILD_SAH) step 4 is Karras 2012's search per node and
 // the steps further down.  The per-element steps live in build_core.cuh (shared
 // with k_forest.cu).
-// Also the refit of an existing handle (k_parents2, k_refit2, k_refit4).
+// Also the refit of an existing handle (k_refit2, k_refit2_top, k_refit4).
 #include <algorithm>
 
 #include "build_core.cuh"
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kT) k_sah_roots(uint32_t n, uint32_t K, const 
 
 // A finished SAH root's box where its Karras parent's union reads it, then the
 // walk up the Karras nodes above it (the second arrival at a node computes its
-// box, as refit_walk).  One thread.
+// box, as refit_walk_up).  One thread.
 __device__ void sah_refit_up(uint32_t rn, float4 rlo, float4 rhi, const int32_t* __restrict__ kl,
                              const int32_t* __restrict__ kr, const uint32_t* __restrict__ par_in,
                              const uint32_t* __restrict__ par_lf, float4* box_in, float4* box_lf,

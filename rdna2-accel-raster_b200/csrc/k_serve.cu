@@ -167,8 +167,8 @@ struct ServeSrc {
     }
 };
 
-// At most 72 registers per thread (7 blocks of 128 threads per SM), the
-// budget that measured fastest for the frame's any-hit traversal.  `rows`
+// At most 64 registers per thread (8 blocks of 128 threads per SM), as the
+// frame's any-hit traversal; the watertight variant spills 4 bytes.  `rows`
 // stack entries per lane (for the deepest tree); WIDE: a mesh has room for
 // more nodes than a 32-bit entry can name.
 template <bool MT, bool WIDE>

@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kT, 1) k_build_small(const __grid_constant__ S
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < 2 * kSmallMax / 32; i += kT) S.seen[i] = 0u;
 
-    // ---- emission counts (leaf_step)
+    // ---- emission counts: the nodes whose range starts at a position, down the left links
     uint32_t sum = 0;
     uint32_t cw[kItems];
 #pragma unroll
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kT, 1) k_build_small(const __grid_constant__ S
     }
     __syncthreads();
 
-    // ---- the emitted tree's links, by pre-order position (emit_step)
+    // ---- the emitted tree's links, by pre-order position
     const bool near = total <= kNodes;
     TreeArrays T = A.far;
     if (near) {

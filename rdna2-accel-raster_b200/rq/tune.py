@@ -5,12 +5,12 @@
     block size x refill chunk x register budget, then the refill threshold
     (median of 5 runs each);
   - the batched workload (512 deforming grids, 4,096 any-hit + 4,096
-    closest-hit rays per mesh) through rq_batch_autotune: every build block
-    size x blocks per SM, every traversal block size x chunk x register budget;
-and writes the chosen shapes and every measured candidate as JSON.  The
-committed copy (tuning_b200.json beside this file) is what the benchmark and
-callers load with `lookup` / `lookup_shadow`; a workload missing from it is
-tuned at run time.
+    closest-hit rays per mesh) through rq_batch_autotune: every traversal block
+    size x chunk x register budget, then the refill threshold;
+and writes the chosen shapes as JSON (with --trials, every measured candidate
+to a file of its own).  The committed copy (tuning_b200.json beside this file)
+is what the benchmark and callers load with `lookup` / `lookup_shadow`; a
+workload missing from it is tuned at run time.
 """
 import argparse
 import json
@@ -162,6 +162,7 @@ def main():
 
     ap = argparse.ArgumentParser()
     ap.add_argument("--out", required=True)
+    ap.add_argument("--trials", help="write every measured candidate here")
     ap.add_argument("--reps", type=int, default=5)
     ap.add_argument("--only", choices=["shadow", "batched"], help="tune one workload, keep the other's entry")
     ap.add_argument("--build", choices=["lbvh", "sah"], default="sah", help="the frame's build for the shadow tuning")
@@ -169,15 +170,19 @@ def main():
     ctx = rq.Context(0)
     table = load(args.out) if os.path.exists(args.out) else {}
     table.setdefault("device", torch.cuda.get_device_name(0))
+    measured = {}
     if args.only != "batched":
-        tune_frame(ctx, table, args)
+        tune_frame(ctx, table, measured, args)
     if args.only != "shadow":
-        tune_batch_entry(ctx, table, args)
+        tune_batch_entry(ctx, table, measured, args)
     with open(args.out, "w") as fo:
         json.dump(table, fo, indent=1)
+    if args.trials:
+        with open(args.trials, "w") as fo:
+            json.dump(measured, fo, indent=1)
 
 
-def tune_frame(ctx, table, args):
+def tune_frame(ctx, table, measured, args):
     import numpy as np
     import torch
     import rq
@@ -191,20 +196,23 @@ def tune_frame(ctx, table, args):
     params = W.shadow_params()
     gbuf = rq.render_gbuffer(ctx, bvh, W.shadow_camera())
     shape, trials = tune_shadow(ctx, bvh, gbuf, params, args.reps)
-    table.setdefault("shadow", {})[shadow_key(len(idx), params, sah)] = {
+    key = shadow_key(len(idx), params, sah)
+    measured[key] = trials
+    table.setdefault("shadow", {})[key] = {
         "workload": ("1080p shadows + AO frame (2.5M-triangle grid, seed 1, 16 lights, 1 AO ray)"
                      + (", LBVH with SAH-rebuilt subtrees" if sah else ", LBVH")),
-        "shape": shape, "ms": min(t["ms"] for t in trials), "trials": trials}
+        "shape": shape, "ms": min(t["ms"] for t in trials)}
     print(json.dumps({"shadow_shape": shape, "ms": min(t["ms"] for t in trials)}))
     cshape, ctrials = tune_camera(ctx, bvh, W.shadow_camera(), args.reps)
-    table.setdefault("camera", {})[shadow_key(len(idx), params, sah)] = {
+    measured["camera " + key] = ctrials
+    table.setdefault("camera", {})[key] = {
         "workload": "1080p frame's primary rays (the shadows + AO frame's camera)",
-        "shape": cshape, "ms": min(t["ms"] for t in ctrials), "trials": ctrials}
+        "shape": cshape, "ms": min(t["ms"] for t in ctrials)}
     print(json.dumps({"camera_schedule": cshape, "ms": min(t["ms"] for t in ctrials)}))
     bvh.destroy()
 
 
-def tune_batch_entry(ctx, table, args):
+def tune_batch_entry(ctx, table, measured, args):
     import numpy as np
     import torch
     import rq
@@ -223,8 +231,8 @@ def tune_batch_entry(ctx, table, args):
         "workload": "batched: 512 grids (seed 2), 4,096 any-hit + 4,096 closest-hit rays per mesh",
         "shape": {k: shape[k] for k in rq.Batch.TUNING_KEYS},
         "build_ms": shape["build_ms"], "trace_ms": shape["trace_ms"],
-        "trials": trials,
     }
+    measured[workload_key(descs, 8192)] = trials
     print(json.dumps({"shape": table["entries"][workload_key(descs, 8192)]["shape"],
                       "build_ms": shape["build_ms"], "trace_ms": shape["trace_ms"]}))
 
